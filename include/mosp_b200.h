@@ -130,7 +130,7 @@ void mosp_workspace_destroy(mosp_workspace *ws);
 int mosp_workspace_reserve(mosp_workspace *ws, int n, int K);
 
 /* mosp_workspace_reserve plus everything the near-far loops of graphs with
- * up to m edges need (near lists, the asynchronous near queue), so that
+ * up to m edges need (near lists, the asynchronous loop's spill queue and row records), so that
  * later calls on such graphs allocate nothing in the workspace (e.g. a
  * serving loop reserves before its first request). */
 int mosp_workspace_reserve_graph(mosp_workspace *ws, int n, long long m, int K);
@@ -172,13 +172,14 @@ int mosp_workspace_set_local_rounds(mosp_workspace *ws, int update_rounds,
 int mosp_workspace_set_narrow(mosp_workspace *ws, int max_items, int rounds);
 
 /* Near-far loop of the persistent launches: on = 1 (default) runs it
- * asynchronously - after each far-pile split every warp claims entries of
- * a sharded near queue, expands them and pushes what improves, with no grid
- * barrier until the phase has run dry - where the graph has no rows of more
- * than 2,048 edges; 0 runs the bulk-synchronous loop (one grid barrier per
- * iteration, the reference's schedule, src/sospUpdateGpu.cu:385-476) for
- * every graph. queue_slots bounds the near queue (8 bytes a slot; 0 = one
- * slot per vertex and objective plus n, at least 2^20) and the bulk loop's
+ * asynchronously - the warps of each CTA split a share of the far piles,
+ * expand what is near and go on with what improves, with no grid barrier
+ * until the phase has run dry; CTAs with much work feed dry ones through a
+ * spill queue - where the graph has no rows of more than 2,048 edges; 0 runs
+ * the bulk-synchronous loop (one grid barrier per iteration, the reference's
+ * schedule, src/sospUpdateGpu.cu:385-476) for every graph. queue_slots
+ * bounds the spill queue (8 bytes a slot; 0 = one slot per vertex and
+ * objective plus n, at least 2^20) and the bulk loop's
  * near lists (entries per objective; 0 = min(n + m, max(2n, 2^20))):
  * entries that find them full go to the far pile and are taken up in the
  * next phase or split. Results do not depend on either. */

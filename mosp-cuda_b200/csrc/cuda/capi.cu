@@ -67,10 +67,14 @@ struct mosp_workspace {
   u64 *nearD0 = nullptr, *nearD1 = nullptr;
   int *gen = nullptr;  // device stamp generation
   bool dirty = false;  // an aborted run may have left inFar/stamp set (or queue slots filled)
-  // asynchronous near queue: aqCap slots (all ~0 between launches) in
-  // kAsyncShards shards, two counter sets
+  // spill queue of the asynchronous loop: aqCap slots (all ~0 between
+  // launches) in kAsyncShards shards, three counter sets
   u64 *aqSlots = nullptr;
   long long aqCap = 0;
+  // row records of the asynchronous loop (two int4 per objective and vertex
+  // of the engine lists)
+  int4 *rec = nullptr;
+  long long recCap = 0;
   AsyncShard *aqCtr = nullptr;
   // near-far loop: 1 asynchronous where the graph allows it, 0 bulk
   // (mosp_workspace_set_async); results do not depend on it
@@ -176,6 +180,9 @@ void releaseAsync(mosp_workspace *ws) {
   ws->aqSlots = nullptr;
   ws->aqCtr = nullptr;
   ws->aqCap = 0;
+  if (ws->rec) cudaFree(ws->rec);
+  ws->rec = nullptr;
+  ws->recCap = 0;
 }
 
 void releaseLists(mosp_workspace *ws) {
@@ -249,7 +256,7 @@ int reserveNear(mosp_workspace *ws, long long n, long long m, int K) {
   return MOSP_OK;
 }
 
-/// Slots of the asynchronous near queue for K objectives of n vertices:
+/// Slots of the asynchronous loop's spill queue for K objectives of n vertices:
 /// one entry per vertex and objective plus n, at least 2^20 (or the size
 /// the caller set), in whole 32-slot claims per shard. A phase that pushes
 /// more moves the excess to the far piles, so this bounds memory, not
@@ -264,7 +271,7 @@ int reserveAsync(mosp_workspace *ws, long long n, int K) {
   if (ws->asyncMode == 0) return MOSP_OK;
   int st = MOSP_OK;
   if (ws->aqCtr == nullptr) {
-    if ((st = deviceAlloc(&ws->aqCtr, 2 * kAsyncShards)) != MOSP_OK) return st;
+    if ((st = deviceAlloc(&ws->aqCtr, 3 * kAsyncShards)) != MOSP_OK) return st;
   }
   const long long need = asyncSlotsFor(n, K, ws->asyncSlots);
   if (need == ws->aqCap && ws->aqSlots != nullptr) return MOSP_OK;
@@ -278,6 +285,15 @@ int reserveAsync(mosp_workspace *ws, long long n, int K) {
   return MOSP_OK;
 }
 
+/// Row records of K objectives (32 bytes per vertex each). They only make
+/// the loop faster: a launch without room for them runs without.
+void reserveRecords(mosp_workspace *ws, int K) {
+  const long long need = 2 * ws->nCap * K;
+  if (ws->asyncMode == 0 || need <= ws->recCap) return;
+  ws->recCap = 0;
+  if (deviceAlloc(&ws->rec, need) == MOSP_OK) ws->recCap = need;
+}
+
 int reserveLists(mosp_workspace *ws, long long n, int K) {
   if (n <= ws->nCap && K <= ws->kCap) return MOSP_OK;
   const long long newN = std::max(n, ws->nCap);
@@ -287,7 +303,8 @@ int reserveLists(mosp_workspace *ws, long long n, int K) {
   int st = MOSP_OK;
   if ((st = deviceAlloc(&ws->packed, total)) != MOSP_OK) return st;
   for (int **p : {&ws->val, &ws->stamp, &ws->inFar, &ws->cand, &ws->far0, &ws->far1}) {
-    if ((st = deviceAlloc(p, total)) != MOSP_OK) {
+    const bool pile = p == &ws->far0 || p == &ws->far1;
+    if ((st = deviceAlloc(p, pile ? kFarCopies * total : total)) != MOSP_OK) {
       releaseLists(ws);
       return st;
     }
@@ -413,6 +430,10 @@ void fillLists(EngineParams &p, mosp_workspace *ws, int block) {
     p.aqCtr = ws->aqCtr;
     p.aqShards = kAsyncShards;
     p.aqShardCap = static_cast<unsigned>(ws->aqCap / kAsyncShards);
+    // (the combined launch decides by its own edge count)
+    if ((p.mode == kModeCombined || recordsPay(p.n, p.m)) && 2 * ws->nCap * p.K <= ws->recCap) {
+      p.rec = ws->rec;
+    }
     p.stageEntries = std::min(kStageEntriesMax, std::max(kStageEntriesAsync, p.K * kThreads));
   } else {
     p.stageEntries = kStageEntriesMax;
@@ -432,6 +453,7 @@ void fillLists(EngineParams &p, mosp_workspace *ws, int block) {
   p.farL0 = ws->far0;
   p.farL1 = ws->far1;
   p.stride = ws->nCap;
+  p.strideFar = kFarCopies * ws->nCap;
   p.ctl = ws->ctl + block;
   p.blockSums = ws->blockSums;
 }
@@ -634,6 +656,7 @@ int prepareUpdate(mosp_workspace *ws, const UpdateArgs &a, EngineParams &p, int 
   if (st != MOSP_OK) return st;
   if ((st = reserveNear(ws, a.n, a.m, a.K)) != MOSP_OK) return st;
   if ((st = reserveAsync(ws, a.n, a.K)) != MOSP_OK) return st;
+  if (recordsPay(a.n, a.m)) reserveRecords(ws, a.K);
   std::memset(&p, 0, sizeof(p));
   p.n = a.n;
   p.m = a.m;
@@ -697,6 +720,7 @@ int prepareCombined(mosp_workspace *ws, int n, int K, const int *d_parents, cons
   if ((st = reserveCombined(ws, n, K)) != MOSP_OK) return st;
   if ((st = reserveNear(ws, n, static_cast<long long>(n) * K, 1)) != MOSP_OK) return st;
   if ((st = reserveAsync(ws, n, 1)) != MOSP_OK) return st;
+  reserveRecords(ws, 1);
   std::memset(&p, 0, sizeof(p));
   p.n = n;
   p.K = 1;
@@ -845,7 +869,10 @@ int mosp_workspace_reserve_graph(mosp_workspace *ws, int n, long long m, int K) 
   const long long nn = std::max(n, 1);
   // the update's near lists and queue, and those of the combined step
   if ((st = reserveNear(ws, nn, std::max(m, nn * K), K)) != MOSP_OK) return st;
-  return reserveAsync(ws, nn, K);
+  if ((st = reserveAsync(ws, nn, K)) != MOSP_OK) return st;
+  // (a batch may leave a graph with fewer edges)
+  reserveRecords(ws, recordsPay(nn, m - m / 8) ? K : 1);
+  return MOSP_OK;
 }
 
 int mosp_workspace_set_sources(mosp_workspace *ws, const int *h_sources, int count) {
@@ -1203,6 +1230,7 @@ int mosp_sosp_from_scratch(mosp_workspace *ws, int n, int m, const int *d_out_ro
   if ((st = reserveLists(ws, n, 1)) != MOSP_OK) return st;
   if ((st = reserveNear(ws, n, m, 1)) != MOSP_OK) return st;
   if ((st = reserveAsync(ws, n, 1)) != MOSP_OK) return st;
+  if (recordsPay(n, m)) reserveRecords(ws, 1);
   int bits = 0;
   u64 maxDist = 0;
   if ((st = choosePacking(n, max_weight, bits, maxDist)) != MOSP_OK) return st;

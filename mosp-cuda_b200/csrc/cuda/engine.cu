@@ -72,10 +72,6 @@ __device__ __forceinline__ int ldVolatile(const int *p) {
   return *reinterpret_cast<const volatile int *>(p);
 }
 
-__device__ __forceinline__ unsigned ldVolatileU(const unsigned *p) {
-  return *reinterpret_cast<const volatile unsigned *>(p);
-}
-
 __device__ __forceinline__ unsigned long long ldAcquire64(const unsigned long long *p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -88,10 +84,6 @@ __device__ __forceinline__ void stRelease64(unsigned long long *p, unsigned long
 
 __device__ __forceinline__ void stRelaxed64(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-__device__ __forceinline__ void redRelease(unsigned *p, unsigned v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 /// Word helpers for one objective.
@@ -284,8 +276,6 @@ struct StageHeader {
   int heavyDeg[kHeavyCap];
   u64 heavyD[kHeavyCap];       // push: the row's distance; pull: the word before the pass
   u64 heavyBest[kHeavyCap];    // pull: best word over the row, reduced by the CTA
-  int asyncFar[kThreads / 32]; // async loop: entries in each warp's far buffer
-  int asyncLocal[kThreads / 32]; // async loop: entries in each warp's local buffer (may overshoot)
 };
 
 struct StageEntry {
@@ -330,7 +320,7 @@ __device__ __forceinline__ Target listTarget(const EngineParams &P, const LoopSh
     return Target{&P.ctl->nearCount[l][wrSlot], nearWV + kn, nearWD + kn, nullptr};
   }
   const int k = l - K;
-  const long long ko = static_cast<long long>(k) * P.stride;
+  const long long ko = static_cast<long long>(k) * P.strideFar;
   if (L.mode[k] == kSplit) {
     const int s = (L.fs[k] + 1) % 3;
     return Target{&P.ctl->farCount[k][s], (L.fp[k] == 0 ? P.farL1 : P.farL0) + ko, nullptr,
@@ -435,162 +425,14 @@ __device__ void flushStage(const EngineParams &P, const LoopShared &L, int wrSlo
 #define MOSP_EDGE_SLOTS 2
 #endif
 constexpr int kSlots = MOSP_EDGE_SLOTS;
-// asynchronous rounds: three slots per lane cover the ~90 edges of 32 road
-// vertices in one pass (one chain of edge loads, atomicMin and reservation
-// instead of two)
-#ifndef MOSP_EDGE_SLOTS_ASYNC
-#define MOSP_EDGE_SLOTS_ASYNC 3
-#endif
-constexpr int kSlotsAsync = MOSP_EDGE_SLOTS_ASYNC;
-
-// ---------------------------------------------------------------------------
-// Asynchronous near queue
-//
-// In the asynchronous loop the near entries of all objectives go to one
-// queue of aqShards shards. An entry is one 64-bit word: the vertex and its
-// objective (v << 5 | k) in the low half and the distance it was pushed with
-// (saturated at kTagSat) in the high half; an empty slot holds all ones, so a
-// consumer that claimed a slot before its entry was written sees it arrive.
-// A warp reserves slots for the entries of one round with one atomic on the
-// target shard's tail (shards rotate per round, which spreads the work), and
-// claims 32 slots of its home shard with one atomic on the head; it settles
-// what it consumed with one release add on the shard's `done` after its own
-// reservations, so done == tail on every shard (read twice, identical) means
-// that no entry is left and none can be produced. A reservation past the
-// shard's capacity moves its vertex to the far pile instead (re-split in the
-// next phase), so the queue never needs more than its fixed size.
-// ---------------------------------------------------------------------------
-constexpr unsigned long long kEmptySlot = ~0ULL;
-constexpr unsigned kTagSat = 0xFFFFFFFEu;  // distances >= this are not carried in the entry
-constexpr int kFarBuf = 128;               // per-warp far buffer entries (async loop)
-constexpr int kLocalBuf = 32;              // per-warp local near entries (async loop)
-constexpr int kWarps = kThreads / 32;
-
-struct AsyncState {
-  AsyncShard *ctr;   // this phase's counter set
-  int target;        // shard that receives this warp round's near entries
-  unsigned spilled;  // this lane's reservations past the shard's capacity
-  bool local;        // near entries may stay in the warp's local buffer
-};
-
-/// Per-warp buffers of near entries the warp expands itself next (async
-/// loop), after the far buffers in the stage region.
-__device__ __forceinline__ u64 *asyncLocalBuffer(int warp) {
-  return reinterpret_cast<u64 *>(reinterpret_cast<int *>(stageEntries()) + kWarps * kFarBuf) +
-         warp * kLocalBuf;
-}
-
-/// Per-warp buffers of far-pile appends in the async loop (v << 5 | k), in
-/// the stage region of the dynamic shared memory.
-__device__ __forceinline__ int *asyncFarBuffer(int warp) {
-  return reinterpret_cast<int *>(stageEntries()) + warp * kFarBuf;
-}
-
-/// Far-pile append in the async loop: into the warp's buffer (flushed by
-/// flushAsyncFar before it can overflow), the CTA's far minimum in shared
-/// memory. An append that finds the buffer full goes to the pile directly.
-__device__ __forceinline__ void asyncFar(const EngineParams &P, const LoopShared &L, int k, int w,
-                                         u64 d) {
-  StageHeader &H = stageHeader();
-  const int warp = threadIdx.x >> 5;
-  atomicMin(&H.farMin[k], d);
-  const int slot = atomicAdd(&H.asyncFar[warp], 1);
-  if (slot < kFarBuf) {
-    asyncFarBuffer(warp)[slot] = (w << 5) | k;
-  } else {
-    const Target t = listTarget(P, L, P.K + k, 0, nullptr, nullptr);
-    const int idx = warpAppend(t.counter);
-    t.v[idx] = w;
-  }
-}
-
-/// The warp's buffered far appends to their piles (one reservation per
-/// objective group of lanes). All 32 lanes call it.
-__device__ void flushAsyncFar(const EngineParams &P, const LoopShared &L) {
-  StageHeader &H = stageHeader();
-  const int warp = threadIdx.x >> 5;
-  const unsigned lane = laneId();
-  __syncwarp();
-  int cnt = H.asyncFar[warp];
-  cnt = cnt < kFarBuf ? cnt : kFarBuf;
-  const int *buf = asyncFarBuffer(warp);
-  for (int i0 = 0; i0 < cnt; i0 += 32) {
-    const int i = i0 + static_cast<int>(lane);
-    if (i < cnt) {
-      const int e = buf[i];
-      const int k = e & 31;
-      const int v = static_cast<int>(static_cast<unsigned>(e) >> 5);
-      const Target t = listTarget(P, L, P.K + k, 0, nullptr, nullptr);
-      const int idx = warpAppend(t.counter);
-      t.v[idx] = v;
-    }
-  }
-  __syncwarp();
-  if (lane == 0) H.asyncFar[warp] = 0;
-  __syncwarp();
-}
-
-/// Whether the warp's far buffer has fewer than `margin` free entries; the
-/// same answer in every lane (all 32 lanes call it).
-__device__ __forceinline__ bool farBufferFull(int margin) {
-  __syncwarp();
-  const int cnt = __shfl_sync(kFull, stageHeader().asyncFar[threadIdx.x >> 5], 0);
-  return cnt > kFarBuf - margin;
-}
-
-/// Near-queue push of (w, d) for objective k into the round's target shard.
-/// The active lanes share one reservation.
-__device__ __forceinline__ void asyncNear(const EngineParams &P, const LoopShared &L, AsyncState &A,
-                                          int k, int w, u64 d) {
-  const unsigned lane = laneId();
-  const unsigned tag = d < kTagSat ? static_cast<unsigned>(d) : kTagSat;
-  if (A.local) {
-    // the warp keeps up to kLocalBuf of its own pushes and expands them
-    // next, without the queue's round trips
-    const int warp = threadIdx.x >> 5;
-    const int slot = atomicAdd(&stageHeader().asyncLocal[warp], 1);
-    if (slot < kLocalBuf) {
-      asyncLocalBuffer(warp)[slot] =
-          (static_cast<u64>(tag) << 32) | ((static_cast<unsigned>(w) << 5) | static_cast<unsigned>(k));
-      return;
-    }
-  }
-  const unsigned mask = __activemask();
-  const int leader = __ffs(mask) - 1;
-  unsigned base = 0;
-  if (static_cast<int>(lane) == leader) base = atomicAdd(&A.ctr[A.target].tail, __popc(mask));
-  base = __shfl_sync(mask, base, leader);
-  const unsigned idx = base + __popc(mask & ((1u << lane) - 1u));
-  if (idx < P.aqShardCap) {
-    const u64 e = (static_cast<u64>(tag) << 32) | ((static_cast<unsigned>(w) << 5) | static_cast<unsigned>(k));
-    u64 *slot = P.aqSlots + static_cast<long long>(A.target) * P.aqShardCap + idx;
-    // A consumer expands with min(tag, its read of the word), so only an
-    // entry without a usable tag needs the word ordered before it.
-    if (tag < kTagSat) stRelaxed64(slot, e); else stRelease64(slot, e);
-  } else {
-    ++A.spilled;
-    if (atomicExch(P.inFar + static_cast<long long>(k) * P.stride + w, 1) == 0) asyncFar(P, L, k, w, d);
-  }
-}
-
 /// A strict improvement of w's distance to d (objective k): to the next near
 /// list (d below the threshold) or, once, to the far pile.
-template <bool Async>
-__device__ __forceinline__ void pushImproved(const EngineParams &P, const LoopShared &L, AsyncState *A,
-                                             int k, int w, u64 d, int wrSlot, int *nearWV,
-                                             u64 *nearWD) {
+__device__ __forceinline__ void pushImproved(const EngineParams &P, const LoopShared &L, int k, int w,
+                                             u64 d, int wrSlot, int *nearWV, u64 *nearWD) {
   if (d < L.thr[k]) {
-    if constexpr (Async) {
-      asyncNear(P, L, *A, k, w, d);
-    } else {
-      stageAppend(P, L, k, w, d, wrSlot, nearWV, nearWD);
-    }
+    stageAppend(P, L, k, w, d, wrSlot, nearWV, nearWD);
   } else if (atomicExch(P.inFar + static_cast<long long>(k) * P.stride + w, 1) == 0) {
-    if constexpr (Async) {
-      asyncFar(P, L, k, w, d);
-    } else {
-      stageAppend(P, L, P.K + k, w, d, wrSlot, nearWV, nearWD);
-    }
+    stageAppend(P, L, P.K + k, w, d, wrSlot, nearWV, nearWD);
   }
 }
 
@@ -621,7 +463,7 @@ __device__ __forceinline__ void relaxEdge(const EngineParams &P, const LoopShare
   if (w == P.source || nd > O.maxDist) return;
   const u64 old = atomicMin(P.packed + ko + w, pk.pack(nd, u));
   if (nd >= pk.dist(old)) return;
-  pushImproved<false>(P, L, nullptr, k, w, nd, wrSlot, nearWV, nearWD);
+  pushImproved(P, L, k, w, nd, wrSlot, nearWV, nearWD);
 }
 
 /// The CTA's queued heavy rows, each expanded by all threads of the CTA.
@@ -655,12 +497,12 @@ __device__ void expandHeavy(const EngineParams &P, const LoopShared &L, const in
 /// with their loads and 64-bit atomicMin overlapped; every strict
 /// improvement is staged for the next near list or the far pile. All 32
 /// lanes call it.
-template <int Mode, bool Async = false>
+template <int Mode>
 __device__ __forceinline__ void expandWarp(const EngineParams &P, const LoopShared &L,
                                            const int *outRow, const int *outCol,
                                            const int *const *outWk, int k, int u, u64 du, int beg,
                                            int deg, int wrSlot, int *nearWV, u64 *nearWD,
-                                           bool heavyOn, AsyncState *A = nullptr) {
+                                           bool heavyOn) {
   StageHeader &H = stageHeader();
   const unsigned lane = laneId();
   {
@@ -707,7 +549,7 @@ __device__ __forceinline__ void expandWarp(const EngineParams &P, const LoopShar
       if (w == P.source || nd > O.maxDist) continue;
       const u64 old = atomicMin(P.packed + kob + w, pk.pack(nd, ub));
       if (nd >= pk.dist(old)) continue;
-      pushImproved<Async>(P, L, A, kb, w, nd, wrSlot, nearWV, nearWD);
+      pushImproved(P, L, kb, w, nd, wrSlot, nearWV, nearWD);
     }
   }
   if (deg > (1 << 20)) deg = 0;
@@ -719,12 +561,8 @@ __device__ __forceinline__ void expandWarp(const EngineParams &P, const LoopShar
   }
   const int edges = __shfl_sync(kFull, incl, 31);
   const int excl = incl - deg;
-  constexpr int SL = Async ? kSlotsAsync : kSlots;
+  constexpr int SL = kSlots;
   for (int s0 = 0; s0 < edges; s0 += 32 * SL) {
-    if constexpr (Async) {
-      // room for this round's far appends in the warp's buffer
-      if (farBufferFull(32 * SL)) flushAsyncFar(P, L);
-    }
     // SL edge slots per lane, their loads and atomics overlapped
     int sl[SL], kk[SL], uu[SL], ee[SL], ww[SL], wt[SL];
     u64 dd[SL], nd[SL], old[SL];
@@ -768,7 +606,7 @@ __device__ __forceinline__ void expandWarp(const EngineParams &P, const LoopShar
 #pragma unroll
     for (int h = 0; h < SL; ++h) {
       if (!act[h] || nd[h] >= pkOf(P.obj[kk[h]]).dist(old[h])) continue;
-      pushImproved<Async>(P, L, A, kk[h], ww[h], nd[h], wrSlot, nearWV, nearWD);
+      pushImproved(P, L, kk[h], ww[h], nd[h], wrSlot, nearWV, nearWD);
     }
   }
 }
@@ -924,7 +762,8 @@ __device__ bool nearFarLoop(const EngineParams &P, const int *outRow,
 
       if (mode == kSplit) {
         // far pile entry: to the near list below the new threshold
-        const int v = __ldcg((L.fp[k] == 0 ? P.farL0 : P.farL1) + ko + i);
+        const int v = __ldcg((L.fp[k] == 0 ? P.farL0 : P.farL1) +
+                             static_cast<long long>(k) * P.strideFar + i);
         const u64 word = __ldcg(P.packed + ko + v);
         const u64 d = word == kInfWord ? kInfWord : pkOf(P.obj[k]).dist(word);
         if (d < L.thr[k]) {
@@ -1050,229 +889,1172 @@ __device__ bool nearFarLoop(const EngineParams &P, const int *outRow,
 // ---------------------------------------------------------------------------
 // Asynchronous near-far loop
 //
-// The bulk loop above pays a grid barrier per iteration and, worse, waits in
-// every iteration for the slowest warp of the grid. Here a phase runs one
-// far-pile split and then expands the near entries asynchronously: every
-// warp claims slots of the near queue, expands what has arrived and pushes
-// what improves, with no barrier until the whole phase has run dry. Only the
-// split of the far piles (a new threshold per objective) needs the grid to
-// agree, so there is one grid barrier per phase (a few per launch) instead
-// of one per iteration (80-150). Relaxations are the same monotone 64-bit
-// atomicMin, so the fixed point, i.e. every word, is the one the bulk loop
-// reaches.
+// The bulk loop above pays a grid barrier per iteration and waits in every
+// iteration for the slowest warp of the grid. Here a phase splits the far
+// piles and expands the near entries with no barrier until the phase has run
+// dry; only a new threshold per objective needs the grid to agree.
+// Relaxations are the same monotone 64-bit atomicMin, so the fixed point,
+// i.e. every word, is the one the bulk loop reaches.
+//
+// What bounds the loop is the number of hops of the deepest path times the
+// latency of a hop, from the improvement of a vertex to the improvement of
+// its neighbours (thin wavefronts: about 2,000 hops of a few hundred entries
+// each on a grid road network of 500,000 vertices). So a hop stays inside
+// one warp, or at least inside one CTA:
+//
+//   * a CTA takes an equal, contiguous share of the far piles. An entry
+//     below the new threshold is expanded on the spot, the others go to the
+//     warp's far buffer;
+//   * a warp with few entries gives each a group of lanes and goes on with
+//     what they improve, hop after hop (chase, chaseRecords). What is more
+//     than it can hold goes by mail to a warp of the CTA that has nothing to
+//     do (slots and an mbarrier of its own, on which it waits without
+//     polling: 31 polling warps took half of the issue slots), or to the
+//     CTA's ring of near entries in shared memory;
+//   * with many entries, warps take up to 32 at a time from the ring and push
+//     what improves back to it;
+//   * a CTA whose ring holds more than kDonate entries while others have run
+//     dry, or more than kRingSpill in any case, sends its pushes to a global
+//     spill queue, from which dry CTAs claim up to 256 entries at a time. A
+//     push that finds its shard full goes to the far pile.
+//
+// Row records (one 32-byte sector with a vertex's first four edges) make the
+// loads of a hop one round trip to L2 that runs beside the atomicMin.
+//
+// Measured on a B200 against one grid-wide sharded queue with a claim, a slot
+// and two counters per hop: a hop of a bare chain 0.72 us; tree from scratch
+// of a 497,700-vertex road network 10.05 -> 2.59 ms, update of a million
+// vertices with local detours (K = 3) 28.7 -> 8.8 ms, combined graph of
+// 249,500 vertices (K = 6) 5.26 -> 1.38 ms, update of 2M vertices with
+// long-range insertions (wide phases) 2.49 -> 2.43 ms.
+//
+// A vertex enters the far pile when an atomicMin takes it from infinity (or,
+// in an update, from its tree distance) to a distance past the threshold;
+// while its word stays past the threshold it is in the pile already, so the
+// far append needs no flag.
+//
+// End of a phase: EngineControl::asyncPending counts the CTAs that still work
+// on their share and the spilled entries that are not settled. A warp adds
+// its finished entries to the CTA's `settled` count when it runs out of work,
+// after its far buffer is flushed; the warp that makes the counts meet
+// settles the CTA's share and its claimed entries with one atomic. The phase
+// is over when asyncPending is zero, which an idle warp of every CTA polls.
+// No grid barrier separates the phases: this counter and those of the far
+// piles and the spill queue rotate through three slots, so a CTA that enters
+// a phase early touches none that a late one reads.
 // ---------------------------------------------------------------------------
+constexpr unsigned long long kEmptySlot = ~0ULL;
+constexpr unsigned kTagSat = 0xFFFFFFFEu;  // distances >= this are not carried in the entry
+constexpr unsigned kOverflow = 0x80000000u;  // far-pile entry of an overflowed push
+constexpr int kWarps = kThreads / 32;
+constexpr unsigned kRingMask = kRing - 1;
+// a push finds the ring at most this full, plus 128 entries of each of the
+// other warps that passed the check at the same time, plus a claim
+constexpr unsigned kRingSpill = kRing / 4;
+constexpr unsigned kDonate = 512;    // ring entries above which a CTA feeds dry ones
+constexpr unsigned kSliceFirst = 1024;  // ring entries above which the share waits
+constexpr int kClaim = 256;          // entries claimed from the spill queue at a time
+constexpr int kOctBatch = 4;         // entries of a batch that is expanded by octets of lanes
+constexpr int kOctDeg = 32;          // longest row of such a batch
+constexpr int kQuadBatch = 8;        // the same with row records (four lanes each)
+constexpr int kChaseRing = 64;       // ring entries above which a warp keeps no entries of its own
+// What a batch of the loop reads: the CSR; row records for few entries and the
+// CSR for full batches; row records for all. Full batches read the records
+// while all of them fit L2; past that the CSR, which is half their size and
+// shares lines between neighbours, is the better source (near-far loop of an
+// update: 96 MB of records 6.06 ms against 6.85 ms, 123 MB 1.13 against 0.97,
+// 189 MB 1.42 against 1.20).
+enum : int { kCsrOnly = 0, kThinRecords = 1, kRecords = 2 };
+constexpr long long kRecordBytes = 100LL << 20;
+constexpr unsigned kThinShare = 64;  // far-pile entries per CTA up to which a phase is wider
+constexpr unsigned kSpinLimit = 1u << 24;
+#ifndef MOSP_EDGE_SLOTS_ASYNC
+#define MOSP_EDGE_SLOTS_ASYNC 3
+#endif
+// three slots per lane cover the ~90 edges of 32 road vertices in one pass
+constexpr int kSlotsAsync = MOSP_EDGE_SLOTS_ASYNC;
+static_assert(kRingSpill + kWarps * 128 + kClaim <= kRing, "ring reservations fit");
+static_assert(kMail == kQuadBatch, "a mail is a batch");
 
-/// Phase end detection (warp 0 of CTA 0 while it is idle): every CTA has
-/// finished its split and, in two successive reads of all shards' counters,
-/// done == tail everywhere with nothing changed in between (the counters
-/// only grow, so the second read shows the state of one moment).
-__device__ void detectPhaseEnd(const EngineParams &P, const AsyncShard *ctr, unsigned phase) {
-  EngineControl *c = P.ctl;
-  const unsigned lane = laneId();
-  const int S = P.aqShards;
-  unsigned split = 0;
-  if (lane == 0) split = ldAcquire(&c->asyncSplit);
-  split = __shfl_sync(kFull, split, 0);
-  if (split < (phase + 1) * gridDim.x) return;
-  unsigned d1 = 0, t1 = 0, d2 = 0, t2 = 0;
-  if (static_cast<int>(lane) < S) {
-    d1 = ldAcquire(&ctr[lane].done);
-    t1 = ldAcquire(&ctr[lane].tail);
-  }
-  if (!__all_sync(kFull, d1 == t1)) return;
-  if (static_cast<int>(lane) < S) {
-    d2 = ldAcquire(&ctr[lane].done);
-    t2 = ldAcquire(&ctr[lane].tail);
-  }
-  if (!__all_sync(kFull, d2 == d1 && t2 == t1)) return;
-  if (lane == 0) stRelease(&c->asyncPhase, phase + 1);
-}
-
-/// Settle one warp round: `consumed` entries of shard `from` and the lanes'
-/// reservations past the capacity of shard `to`, after the round's own
-/// reservations (release).
-__device__ __forceinline__ void settleRound(AsyncShard *ctr, int from, unsigned consumed, int to,
-                                            unsigned spilled) {
-  if (__any_sync(kFull, spilled != 0)) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) spilled += __shfl_xor_sync(kFull, spilled, off);
-  }
-  if (consumed == 0 && spilled == 0) return;  // the same in every lane
-  // the warp barrier orders the lanes' reservations before lane 0's
-  // release adds, which order them (cumulatively) before the new counts
-  __syncwarp();
-  if (laneId() == 0) {
-    if (consumed != 0) redRelease(&ctr[from].done, consumed);
-    if (spilled != 0) redRelease(&ctr[to].done, spilled);
-  }
-}
-
-/// Decode a near entry: objective k, vertex u (-1 if the entry is stale:
-/// a later, smaller distance has its own entry), the distance du to expand
-/// with and u's row. A word read older than the entry is covered by
-/// expanding with the entry's tag.
-template <int Mode>
-__device__ __forceinline__ void asyncEntry(const EngineParams &P, const int *outRow, u64 e, int &k,
-                                           int &u, u64 &du, int &beg, int &deg) {
-  const unsigned vk = static_cast<unsigned>(e);
-  const unsigned tag = static_cast<unsigned>(e >> 32);
-  k = static_cast<int>(vk & 31u);
-  const int v = static_cast<int>(vk >> 5);
-  const u64 word = __ldcg(P.packed + static_cast<long long>(k) * P.stride + v);
-  const int b0 = ldGraph<Mode>(outRow + v);
-  const int b1 = ldGraph<Mode>(outRow + v + 1);
-  const u64 d = word == kInfWord ? kInfWord : pkOf(P.obj[k]).dist(word);
-  u = -1;
-  if (tag < kTagSat) {
-    if (d >= tag) {
-      u = v;
-      du = tag;
-    }
-  } else if (d != kInfWord) {
-    u = v;
-    du = d;
-  }
-  if (u >= 0) {
-    beg = b0;
-    deg = b1 - b0;
-  }
-}
-
-/// The consumer side of one phase for one warp: expand its own local
-/// entries first, else claim slots and expand the entries that arrive,
-/// until the phase is over (true) or the launch is stopped (false).
-/// Per-warp counters of the asynchronous loop (lane 0): rounds and entries
-/// taken from the queue and from the warp's local buffer.
-struct AsyncCounts {
-  long long queueRounds, localRounds, queueItems, localItems;
+/// What an expansion needs of its objective.
+struct alignas(16) AsyncObj {
+  u64 *packed;
+  const int4 *rec;   // row records (two int4 per vertex) or null
+  u64 thrWord;       // words below it have a distance below the threshold
+  u64 mostWord;      // the largest word of a distance within the bound
+  unsigned scale;    // 1 << bits
+  unsigned mask;     // the word's parent field: the low `bits` bits
+  int bits;
+  int pad;
+  const int *outW;
+  const long long *dist;  // update: the distances of the input tree
+  u64 thr;
+  u64 prev;          // the last phase's threshold
 };
 
-template <int Mode>
-__device__ bool asyncConsume(const EngineParams &P, const LoopShared &L, const int *outRow,
-                             const int *outCol, const int *const *outWk, AsyncShard *ctr,
-                             unsigned phase, long long gwarp, const Sync &sync, AsyncCounts &cnt) {
-  EngineControl *c = P.ctl;
-  const unsigned lane = laneId();
-  const int S = P.aqShards;
-  const unsigned cap = P.aqShardCap;
-  int cs = static_cast<int>(gwarp % S);  // shard this warp claims from
-  int hops = 0;                          // shards found exhausted
-  int target = static_cast<int>((gwarp * 7 + 3) % S);
-  unsigned pend = 0, cb = 0, spins = 0, knownTail = 0;
-  // entries of shard cs consumed but not yet settled: a warp settles them
-  // only with its local buffer empty, so while it holds local work the
-  // shard's done stays below its tail and the phase cannot end
-  unsigned unsettled = 0;
-  StageHeader &H = stageHeader();
-  const int warp = threadIdx.x >> 5;
-  u64 *localBuf = asyncLocalBuffer(warp);
-  while (true) {
-    __syncwarp();
-    int nLocal = __shfl_sync(kFull, H.asyncLocal[warp], 0);
-    if (nLocal > 0) {
-      nLocal = nLocal < kLocalBuf ? nLocal : kLocalBuf;
-      const u64 le = static_cast<int>(lane) < nLocal ? localBuf[lane] : kEmptySlot;
-      __syncwarp();
-      if (lane == 0) {
-        H.asyncLocal[warp] = 0;
-        ++cnt.localRounds;
-        cnt.localItems += nLocal;
-      }
-      __syncwarp();
-      int k = 0, u = -1, beg = 0, deg = 0;
-      u64 du = 0;
-      if (le != kEmptySlot) asyncEntry<Mode>(P, outRow, le, k, u, du, beg, deg);
-      AsyncState A{ctr, target, 0u, (P.flags & kFlagLocal) != 0};
-      expandWarp<Mode, true>(P, L, outRow, outCol, outWk, k, u, du, beg, deg, 0, nullptr, nullptr,
-                             false, &A);
-      settleRound(ctr, cs, 0u, target, A.spilled);
-      target = target + 1 == S ? 0 : target + 1;
-      continue;
+/// An entry on its way from lane to lane: a head, the word it took and its
+/// row record.
+struct alignas(16) HopSlot {
+  u64 word;
+  int v, k;
+  int4 cols, wts;
+};
+
+/// A CTA's state of the asynchronous loop (shared memory). head and tail are
+/// the ring's positions, cur the entries taken of the CTA's share of the far
+/// piles, mailed the entries sent by mail, settled the finished entries of
+/// all three; dry when settled == tail + mailed + share. lock guards the
+/// change between busy and dry.
+struct AsyncCta {
+  unsigned head, tail, cur, settled;
+  unsigned share;    // entries of the CTA's share of this phase
+  unsigned owed;     // entries claimed from the spill queue (and the phase's own share: 1)
+  unsigned mailed;
+  unsigned idle;     // warps that wait for mail
+  int dry;
+  int lock;
+  int over;          // the phase is over
+  int abort;         // the launch stops
+  long long base;    // first far-pile index of the share
+  unsigned rounds, items, taken;  // statistics
+  unsigned expanded[kMaxK];
+  int mail[kWarps];  // entries in a warp's mail
+  u64 bar[kWarps];   // its mbarrier
+  int K;
+  unsigned phase;
+  unsigned long long deadline;
+  AsyncObj obj[kMaxK];
+  LoopShared L;
+  HopSlot hop[kWarps][kQuadBatch];   // a warp's entries of the next hop
+  HopSlot mailbox[kWarps][kMail];
+};
+static_assert(sizeof(AsyncCta) <= kAsyncCtaBytes, "kAsyncCtaBytes");
+
+__device__ __forceinline__ u64 *asyncRing() { return reinterpret_cast<u64 *>(stageEntries()); }
+
+/// The warp's buffer of far appends (distance << 32 | v << 5 | k).
+__device__ __forceinline__ u64 *asyncFarBuffer() {
+  return asyncRing() + kRing + (threadIdx.x >> 5) * kFarBuf;
+}
+
+/// The CTA's state, after the far buffers in the dynamic shared memory.
+__device__ __forceinline__ AsyncCta &asyncCta() {
+  return *reinterpret_cast<AsyncCta *>(asyncRing() + kRing + kWarps * kFarBuf);
+}
+
+__device__ __forceinline__ unsigned ldShared(const unsigned *p) {
+  return *reinterpret_cast<const volatile unsigned *>(p);
+}
+__device__ __forceinline__ int ldShared(const int *p) {
+  return *reinterpret_cast<const volatile int *>(p);
+}
+__device__ __forceinline__ u64 ldShared(const u64 *p) {
+  return *reinterpret_cast<const volatile u64 *>(p);
+}
+__device__ __forceinline__ void stShared(u64 *p, u64 v) { *reinterpret_cast<volatile u64 *>(p) = v; }
+__device__ __forceinline__ void stShared(int *p, int v) { *reinterpret_cast<volatile int *>(p) = v; }
+
+__device__ __forceinline__ void barInit(u64 *bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(bar)))
+               : "memory");
+}
+
+/// One arrival completes the phase the warp waits for (release: the mail).
+__device__ __forceinline__ void barArrive(u64 *bar) {
+  asm volatile("{ .reg .b64 s; mbarrier.arrive.release.cta.shared::cta.b64 s, [%0]; }" ::"r"(
+                   static_cast<unsigned>(__cvta_generic_to_shared(bar)))
+               : "memory");
+}
+
+/// Waits for the phase of parity `parity` for a few microseconds at most.
+__device__ __forceinline__ bool barTryWait(u64 *bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3; "
+      "selp.u32 %0, 1, 0, p; }"
+      : "=r"(done)
+      : "r"(static_cast<unsigned>(__cvta_generic_to_shared(bar))), "r"(parity), "r"(4000u)
+      : "memory");
+  return done != 0;
+}
+
+/// A bounded wait ran out (or the deadline passed): the launch stops.
+__device__ __noinline__ void asyncAbort(const EngineParams &P) {
+  AsyncCta &C = asyncCta();
+  atomicCAS(&P.ctl->status, 0, MOSP_ERR_TIMEOUT);
+  stShared(&C.abort, 1);
+}
+
+/// Whether the launch has to stop (a warp with work looks now and then, so
+/// that a run ends by its deadline whether it stalls or keeps iterating).
+/// All lanes call it.
+__device__ __noinline__ bool asyncStop(const EngineParams &P) {
+  AsyncCta &C = asyncCta();
+  int stop = 0;
+  if (laneId() == 0) {
+    stop = ldShared(&C.abort);
+    if (stop == 0 && (ldVolatile(&P.ctl->status) != 0 || globalNs() > C.deadline)) {
+      asyncAbort(P);
+      stop = 1;
     }
-    if (unsettled != 0) {
-      settleRound(ctr, cs, unsettled, 0, 0u);
-      unsettled = 0;
-    }
-    if (pend == 0 && hops < S) {
-      unsigned b = 0;
-      if (lane == 0) b = atomicAdd(&ctr[cs].head, 32u);
-      b = __shfl_sync(kFull, b, 0);
-      if (b >= cap) {
-        cs = (cs + 1) % S;
-        ++hops;
-        knownTail = 0;
-        continue;
-      }
-      cb = b;
-      const unsigned room = cap - b;
-      pend = room >= 32u ? kFull : ((1u << room) - 1u);
-    }
-    u64 *slot = P.aqSlots + static_cast<long long>(cs) * cap + cb + lane;
-    u64 e = kEmptySlot;
-    // only slots below the shard's tail are reserved; the tail only grows,
-    // so the last value read is reloaded only when a pending slot lies past
-    // it (one load per warp, and none while the shard is ahead of the warp)
-    const bool mine = (pend >> lane) & 1u;
-    if (__any_sync(kFull, mine && cb + lane >= knownTail)) {
-      unsigned t = 0;
-      if (lane == 0) t = ldVolatileU(&ctr[cs].tail);
-      knownTail = __shfl_sync(kFull, t, 0);
-    }
-    if (mine && cb + lane < knownTail) e = ldAcquire64(slot);
-    const unsigned ready = __ballot_sync(kFull, e != kEmptySlot);
-    if (ready == 0) {
-      unsigned ph = 0;
-      if (lane == 0) ph = ldAcquire(&c->asyncPhase);
-      ph = __shfl_sync(kFull, ph, 0);
-      if (ph > phase) return true;
-      if (gwarp == 0) detectPhaseEnd(P, ctr, phase);
-      if ((++spins & 63u) == 0) {
-        int stop = 0;
-        if (lane == 0) {
-          stop = ldVolatile(&c->status) != 0;
-          if (!stop && globalNs() > sync.deadline) {
-            atomicCAS(&c->status, 0, MOSP_ERR_TIMEOUT);
-            stop = 1;
-          }
-        }
-        if (__shfl_sync(kFull, stop, 0)) return false;
-      }
-      __nanosleep(spins < 32 ? 32 : 256);
-      continue;
-    }
-    spins = 0;
-    pend &= ~ready;
-    if (lane == 0) {
-      ++cnt.queueRounds;
-      cnt.queueItems += __popc(ready);
-    }
-    int k = 0, u = -1, beg = 0, deg = 0;
-    u64 du = 0;
-    if (e != kEmptySlot) {
-      stRelaxed64(slot, kEmptySlot);
-      asyncEntry<Mode>(P, outRow, e, k, u, du, beg, deg);
-    }
-    AsyncState A{ctr, target, 0u, (P.flags & kFlagLocal) != 0};
-    expandWarp<Mode, true>(P, L, outRow, outCol, outWk, k, u, du, beg, deg, 0, nullptr, nullptr,
-                           false, &A);
-    unsettled += __popc(ready);
-    settleRound(ctr, cs, 0u, target, A.spilled);
-    target = target + 1 == S ? 0 : target + 1;
+  }
+  return __shfl_sync(kFull, stop, 0) != 0;
+}
+
+/// Takes an idle warp out of the idle set (lane 0): its number or -1.
+__device__ __forceinline__ int takeIdle() {
+  AsyncCta &C = asyncCta();
+  unsigned m = ldShared(&C.idle);
+  while (m != 0) {
+    const int w = __ffs(m) - 1;
+    m = atomicAnd(&C.idle, ~(1u << w));
+    if ((m >> w) & 1u) return w;
+  }
+  return -1;
+}
+
+/// Sends up to `count` idle warps to the ring (lane 0).
+__device__ __noinline__ void wakeIdle(int count) {
+  AsyncCta &C = asyncCta();
+  while (count-- > 0) {
+    const int w = takeIdle();
+    if (w < 0) return;
+    C.mail[w] = 0;
+    barArrive(&C.bar[w]);
   }
 }
 
+/// Wakes every idle warp, a lane per warp. All lanes call it.
+__device__ __forceinline__ void wakeAll() {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  unsigned m = 0;
+  if (lane == 0) m = atomicExch(&C.idle, 0u);
+  m = __shfl_sync(kFull, m, 0);
+  if ((m >> lane) & 1u) {
+    C.mail[lane] = 0;
+    barArrive(&C.bar[lane]);
+  }
+  __syncwarp();
+}
+
+/// The warp's far buffer to the piles: one reservation per objective and 32
+/// entries, the pile minimum into the CTA's. All lanes call it.
+__device__ __noinline__ void flushFarEntries(const EngineParams &P, int count) {
+  const LoopShared &L = asyncCta().L;
+  StageHeader &H = stageHeader();
+  const int lane = static_cast<int>(laneId());
+  const u64 *buf = asyncFarBuffer();
+  __syncwarp();
+#pragma unroll 1
+  for (int i0 = 0; i0 < count; i0 += 32) {
+    const bool have = i0 + lane < count;
+    const u64 e = have ? buf[i0 + lane] : 0;
+    const int k = have ? static_cast<int>(e & 31u) : -1;
+    const unsigned peers = __match_any_sync(kFull, k);
+    const unsigned least = __reduce_min_sync(peers, static_cast<unsigned>(e >> 32));
+    const int leader = __ffs(peers) - 1;
+    const Target t = listTarget(P, L, P.K + (k < 0 ? 0 : k), 0, nullptr, nullptr);
+    int at = 0;
+    if (have && lane == leader) {
+      // (a distance that does not fit the tag went to the minimum on its own)
+      if (least < kTagSat) atomicMin(&H.farMin[k], static_cast<u64>(least));
+      at = atomicAdd(t.counter, __popc(peers));
+    }
+    at = __shfl_sync(kFull, at, leader);
+    if (have) t.v[at + __popc(peers & ((1u << lane) - 1u))] = static_cast<int>(static_cast<unsigned>(e) >> 5);
+  }
+  __syncwarp();
+}
+
+/// Append (w, d) of objective k to the warp's far buffer in the lanes with
+/// `want`; flushes first when the buffer could overflow. All lanes call it.
+__device__ __forceinline__ void farAppend(const EngineParams &P, int &farCount, bool want, int k, int w,
+                                          u64 d) {
+  const unsigned mask = __ballot_sync(kFull, want);
+  if (mask == 0) return;
+  if (farCount > kFarBuf - 32) {
+    flushFarEntries(P, farCount);
+    farCount = 0;
+  }
+  if (want) {
+    const unsigned tag = d < kTagSat ? static_cast<unsigned>(d) : kTagSat;
+    if (tag == kTagSat) atomicMin(&stageHeader().farMin[k], d);
+    asyncFarBuffer()[farCount + __popc(mask & ((1u << laneId()) - 1u))] =
+        (static_cast<u64>(tag) << 32) | ((static_cast<unsigned>(w) << 5) | static_cast<unsigned>(k));
+  }
+  farCount += __popc(mask);
+}
+
+/// Whether a vertex x whose word went from `old` to a distance past the
+/// threshold is not in the far pile yet: it comes from infinity or, in an
+/// update, from the distance of its input tree.
 template <int Mode>
-__device__ bool asyncNearFar(const EngineParams &P, const int *outRow, const int *outCol,
-                             const int *const *outWk, Sync &epoch, u64 *deltaOverride, int genBase) {
-  __shared__ LoopShared L;
+__device__ __forceinline__ bool newInFar(const AsyncObj &O, u64 old, int x) {
+  if (old == kInfWord) return true;
+  if constexpr (Mode == kModeUpdate) {
+    return __ldcg(O.dist + x) == static_cast<long long>(old >> O.bits);
+  } else {
+    return false;
+  }
+}
+
+/// Near entries of the lanes with `want` to the spill queue: counted in
+/// asyncPending before their slots can be claimed (the reservation releases
+/// the count). Past the shard's capacity a vertex goes to the far pile, once
+/// (by its flag), marked so that the split expands it. All lanes call it.
+__device__ __noinline__ void spillNear(const EngineParams &P, unsigned mask, u64 entry) {
+  AsyncCta &C = asyncCta();
+  const LoopShared &L = C.L;
+  const int lane = static_cast<int>(laneId());
+  const int count = __popc(mask);
+  // the shards take turns, a different one for each CTA
+  const int s = static_cast<int>((blockIdx.x * 5u + (threadIdx.x >> 5) + (ldShared(&C.settled) >> 5)) %
+                                 static_cast<unsigned>(P.aqShards));
+  const int target = __shfl_sync(kFull, s, 0);
+  unsigned base = 0;
+  if (lane == 0) {
+    atomicAdd(&P.ctl->asyncPending[C.phase % 3], static_cast<unsigned>(count));
+    u64 old;
+    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
+                 : "=l"(old)
+                 : "l"(&P.aqCtr[C.phase % 3 * P.aqShards + target].claimed), "l"(static_cast<u64>(count) << 32)
+                 : "memory");
+    base = static_cast<unsigned>(old >> 32);
+    // the ones past the capacity are not queued
+    const unsigned end = base + static_cast<unsigned>(count);
+    if (end > P.aqShardCap) {
+      atomicSub(&P.ctl->asyncPending[C.phase % 3], end - (base > P.aqShardCap ? base : P.aqShardCap));
+    }
+  }
+  base = __shfl_sync(kFull, base, 0);
+  if (!((mask >> lane) & 1u)) return;
+  const unsigned idx = base + __popc(mask & ((1u << lane) - 1u));
+  if (idx < P.aqShardCap) {
+    // release: an entry without a usable tag needs its word before it
+    stRelease64(P.aqSlots + static_cast<long long>(target) * P.aqShardCap + idx, entry);
+    return;
+  }
+  const int k = static_cast<int>(entry & 31u);
+  const int v = static_cast<int>(static_cast<unsigned>(entry) >> 5);
+  __threadfence();  // the word before the flag
+  if (atomicExch(P.inFar + static_cast<long long>(k) * P.stride + v, 1) == 0) {
+    const Target t = listTarget(P, L, P.K + k, 0, nullptr, nullptr);
+    t.v[atomicAdd(t.counter, 1)] = static_cast<int>(static_cast<unsigned>(v) | kOverflow);
+  }
+}
+
+/// Write an entry to a reserved ring slot. The slot is empty unless the warp
+/// that claimed its last entry has not read it yet.
+__device__ __forceinline__ void ringWrite(const EngineParams &P, unsigned pos, u64 entry) {
+  AsyncCta &C = asyncCta();
+  u64 *slot = asyncRing() + (pos & kRingMask);
+  unsigned spin = 0;
+  while (ldShared(slot) != kEmptySlot) {
+    if (++spin > kSpinLimit || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
+      asyncAbort(P);
+      break;
+    }
+  }
+  if (static_cast<unsigned>(entry >> 32) == kTagSat) __threadfence();  // the word before the entry
+  stShared(slot, entry);
+}
+
+/// Room in the ring for `count` entries (lane 0): reserved at `at`, or false
+/// when the CTA spills.
+__device__ __forceinline__ bool ringReserve(bool donate, int count, unsigned &at) {
+  AsyncCta &C = asyncCta();
+  const unsigned held = ldShared(&C.tail) - ldShared(&C.head);
+  if (held > kRingSpill || (donate && held > kDonate)) return false;
+  at = atomicAdd(&C.tail, static_cast<unsigned>(count));
+  __threadfence_block();  // the entries before the look at the idle warps
+  if (ldShared(&C.idle) != 0) wakeIdle(1 + (count >> 3));
+  return true;
+}
+
+/// Near entries of the lanes in `mask` to the CTA's ring, one reservation
+/// for the warp, or to the spill queue. All lanes call it.
+__device__ __noinline__ void ringPush(const EngineParams &P, unsigned mask, bool donate, u64 entry) {
+  const unsigned lane = laneId();
+  unsigned at = 0;
+  int room = 0;
+  if (lane == 0) room = ringReserve(donate, __popc(mask), at);
+  room = __shfl_sync(kFull, room, 0);
+  at = __shfl_sync(kFull, at, 0);
+  if (!room) {
+    spillNear(P, mask, entry);
+  } else if ((mask >> lane) & 1u) {
+    ringWrite(P, at + __popc(mask & ((1u << lane) - 1u)), entry);
+  }
+}
+
+__device__ __forceinline__ u64 nearEntry(int k, int w, u64 d) {
+  const unsigned tag = d < kTagSat ? static_cast<unsigned>(d) : kTagSat;
+  return (static_cast<u64>(tag) << 32) | ((static_cast<unsigned>(w) << 5) | static_cast<unsigned>(k));
+}
+
+/// The offer of edge weight w by v at distance d is offerBase + w * scale,
+/// with v in the parent field (runNearFar sees to it that a distance within
+/// the bound plus any weight fits the word).
+__device__ __forceinline__ u64 offerBase(const AsyncObj &O, u64 d, int v) {
+  return O.bits == 0 ? d : (d << O.bits) | static_cast<u64>(static_cast<unsigned>(v));
+}
+
+/// The offer base of a head x that took word `word`.
+__device__ __forceinline__ u64 nextBase(u64 word, int x, unsigned mask) {
+  const unsigned lo = (static_cast<unsigned>(word) & ~mask) | (static_cast<unsigned>(x) & mask);
+  return (word & 0xffffffff00000000ULL) | lo;
+}
+
+/// Improvements of one edge per lane (x of objective k from word `old` to
+/// cw): near ones to the ring, new far ones to the far buffer. All lanes.
+template <int Mode>
+__device__ __forceinline__ void pushEdges(const EngineParams &P, const AsyncObj &O, bool donate,
+                                          int &farCount, int k, int x, u64 cw, u64 old) {
+  const bool imp = old > (cw | O.mask);
+  const bool near = imp && cw < O.thrWord;
+  const unsigned mask = __ballot_sync(kFull, near);
+  if (mask != 0) ringPush(P, mask, donate, nearEntry(k, x, cw >> O.bits));
+  const bool far = imp && !near && newInFar<Mode>(O, old, x);
+  farAppend(P, farCount, far, k, x, cw >> O.bits);
+}
+
+/// Lane 0 of the warp that settled the CTA's last entry: if the CTA is still
+/// dry under the lock (the fetching warp may have brought new entries),
+/// settle its share and claimed entries.
+__device__ __noinline__ void asyncDry(const EngineParams &P, unsigned phase) {
+  AsyncCta &C = asyncCta();
+  const LoopShared &L = C.L;
+  EngineControl *c = P.ctl;
+  StageHeader &H = stageHeader();
+  unsigned spin = 0;
+  while (atomicCAS(&C.lock, 0, 1) != 0) {
+    if (++spin > kSpinLimit || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
+      asyncAbort(P);
+      return;
+    }
+  }
+  __threadfence_block();
+  if (C.dry == 0 && ldShared(&C.settled) == ldShared(&C.tail) + ldShared(&C.mailed) + C.share) {
+#pragma unroll 1
+    for (int k = 0; k < P.K; ++k) {
+      if (H.farMin[k] != kInfWord) {
+        atomicMax(listTarget(P, L, P.K + k, 0, nullptr, nullptr).minC, ~H.farMin[k]);
+        H.farMin[k] = kInfWord;
+      }
+    }
+    C.dry = 1;
+    const unsigned done = C.owed;
+    C.owed = 0;
+    atomicAdd(&c->asyncHungry[phase % 3], 1);
+    // release: what the CTA's warps wrote; acquire-free, the others poll
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&c->asyncPending[phase % 3]),
+                 "r"(0u - done)
+                 : "memory");
+  }
+  __threadfence_block();
+  atomicExch(&C.lock, 0);
+}
+
+/// The idle turn of warp 0: the end of the phase, or entries of the spill
+/// queue for the CTA's ring. All lanes call it.
+__device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
+  AsyncCta &C = asyncCta();
+  EngineControl *c = P.ctl;
+  const int lane = static_cast<int>(laneId());
+  const int S = P.aqShards;
+  unsigned left = 1;
+  u64 q = 0;
+  AsyncShard *shards = P.aqCtr + phase % 3 * S;
+  // (relaxed polls: an acquire would empty L1 at every turn)
+  if (lane < S) q = *reinterpret_cast<volatile u64 *>(&shards[lane].claimed);
+  if (lane == 31) left = *reinterpret_cast<volatile unsigned *>(&c->asyncPending[phase % 3]);
+  if (__shfl_sync(kFull, left, 31) == 0) {
+    if (lane == 0) {
+      __threadfence();
+      stShared(&C.over, 1);
+    }
+    __syncwarp();
+    wakeAll();
+    return;
+  }
+  const unsigned cap = P.aqShardCap;
+  unsigned head = static_cast<unsigned>(q), tail = static_cast<unsigned>(q >> 32);
+  if (tail > cap) tail = cap;
+  const unsigned have = __ballot_sync(kFull, lane < S && tail > head);
+  if (have == 0) return;
+  // the first shard with entries from this CTA's own on
+  const unsigned own = blockIdx.x % S;
+  const unsigned later = have >> own << own;
+  const int s = __ffs(later != 0 ? later : have) - 1;
+  q = __shfl_sync(kFull, q, s);
+  head = static_cast<unsigned>(q);
+  tail = static_cast<unsigned>(q >> 32);
+  if (tail > cap) tail = cap;
+  const unsigned n = tail - head < kClaim ? tail - head : kClaim;
+  unsigned r0 = 0;
+  int got = 0;
+  if (lane == 0 && atomicCAS(&C.lock, 0, 1) == 0) {
+    __threadfence_block();
+    if (ldShared(&C.tail) - ldShared(&C.head) <= kDonate &&
+        atomicCAS(&shards[s].claimed, q, q + n) == q) {
+      __threadfence();  // acquire: the producers' counts and slots
+      C.owed += n;
+      C.taken += n;
+      r0 = atomicAdd(&C.tail, n);
+      if (C.dry != 0) {
+        C.dry = 0;
+        atomicSub(&c->asyncHungry[phase % 3], 1);
+      }
+      got = 1;
+    }
+    __threadfence_block();
+    atomicExch(&C.lock, 0);
+  }
+  if (__shfl_sync(kFull, got, 0) == 0) return;
+  r0 = __shfl_sync(kFull, r0, 0);
+  u64 *slots = P.aqSlots + static_cast<long long>(s) * cap + head;
+  u64 e[kClaim / 32];
+#pragma unroll
+  for (int i = 0; i < kClaim / 32; ++i) {
+    const unsigned j = static_cast<unsigned>(i * 32 + lane);
+    e[i] = j < n ? ldAcquire64(slots + j) : 0;
+  }
+#pragma unroll
+  for (int i = 0; i < kClaim / 32; ++i) {
+    const unsigned j = static_cast<unsigned>(i * 32 + lane);
+    if (j >= n) continue;
+    // the producer reserved the slot and is about to write it
+    for (unsigned spin = 0; e[i] == kEmptySlot; e[i] = ldAcquire64(slots + j)) {
+      if (++spin > (kSpinLimit >> 4) || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
+        asyncAbort(P);
+        break;
+      }
+    }
+    stRelaxed64(slots + j, kEmptySlot);
+    ringWrite(P, r0 + j, e[i]);
+  }
+  __syncwarp();
+  if (lane == 0) wakeIdle(static_cast<int>(n >> 3));
+}
+
+/// Graph loads of the asynchronous loop. The combined mode's graph was
+/// written earlier in the same launch and is read-only since the last grid
+/// barrier, so plain loads may keep it in L1.
+template <int Mode>
+__device__ __forceinline__ int ldLoop(const int *p) {
+  if constexpr (Mode == kModeCombined) {
+    return *p;
+  } else {
+    return __ldg(p);
+  }
+}
+
+/// Graphs without row records, thin wavefronts: up to four entries (one per
+/// octet of lanes; rows of at most kOctDeg edges, beg == end for none),
+/// expanded hop after hop by the same warp for as long as they improve
+/// something below the threshold. The row pointers of the heads are loaded
+/// while the atomicMin is on its way.
+template <int Mode>
+__device__ __forceinline__ void chase(const EngineParams &P, const int *outRow, const int *outCol,
+                                      bool donate, int &farCount, int k, int v, u64 du, int beg, int end) {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  u64 base = offerBase(C.obj[k], du, v);
+  for (unsigned hops = 1;; ++hops) {
+    if ((hops & 4095u) == 0 && asyncStop(P)) return;
+    const AsyncObj &O = C.obj[k];
+    int e = beg + static_cast<int>(lane & 7u);
+    int x, rb = 0, re = 0;
+    u64 cw, old;
+    while (true) {
+      const bool in = e < end;
+      x = in ? ldLoop<Mode>(outCol + e) : P.source;
+      cw = base + static_cast<u64>(static_cast<unsigned>(in ? ldLoop<Mode>(O.outW + e) : 0)) * O.scale;
+      old = 0;
+      if (x != P.source && cw <= O.mostWord) {
+        old = atomicMin(O.packed + x, cw);
+        rb = ldLoop<Mode>(outRow + x);
+        re = ldLoop<Mode>(outRow + x + 1);
+      }
+      e += 8;
+      if (!__any_sync(kFull, e < end)) break;
+      pushEdges<Mode>(P, O, donate, farCount, k, x, cw, old);
+    }
+    const bool imp = old > (cw | O.mask);
+    const bool near = imp && cw < O.thrWord;
+    const unsigned nearMask = __ballot_sync(kFull, near);
+    farAppend(P, farCount, imp && !near && newInFar<Mode>(O, old, x), k, x, cw >> O.bits);
+    if (nearMask == 0) return;
+    unsigned keep = __ballot_sync(kFull, near && re - rb <= kOctDeg);
+    if (keep != nearMask || __popc(keep) > kOctBatch) {
+      // a CTA with work for all its warps keeps the breadth-first order
+      const int busy =
+          __shfl_sync(kFull, static_cast<int>(ldShared(&C.tail) - ldShared(&C.head)), 0) > kChaseRing;
+      const bool mine = (keep >> lane) & 1u;
+      const bool give = near && (busy || !mine || __popc(keep & ((1u << lane) - 1u)) >= kOctBatch);
+      const unsigned mask = __ballot_sync(kFull, give);
+      if (mask != 0) ringPush(P, mask, donate, nearEntry(k, x, cw >> O.bits));
+      if (busy) return;
+    }
+    // octet q goes on with the q-th of them
+    HopSlot *slots = C.hop[threadIdx.x >> 5];
+    const int rank = __popc(keep & ((1u << lane) - 1u));
+    const int count = __popc(keep);
+    if (((keep >> lane) & 1u) && rank < kOctBatch) {
+      slots[rank].word = cw;
+      slots[rank].v = x;
+      slots[rank].k = k;
+    }
+    const int src = rank < kOctBatch && ((keep >> lane) & 1u) ? rank : -1;
+    __syncwarp();
+    const int q = static_cast<int>(lane >> 3);
+    const bool on = q < count;
+    // the row of the q-th comes from the lane that loaded it
+    int from = 0;
+#pragma unroll
+    for (int i = 0; i < kOctBatch; ++i) {
+      const unsigned who = __ballot_sync(kFull, src == i);
+      if (i == q && who != 0) from = __ffs(who) - 1;
+    }
+    beg = __shfl_sync(kFull, rb, from);
+    end = __shfl_sync(kFull, re, from);
+    if (on) {
+      v = slots[q].v;
+      k = slots[q].k;
+      base = nextBase(slots[q].word, v, C.obj[k].mask);
+      if ((lane & 7u) == 0) atomicAdd(&C.expanded[k], 1u);
+    } else {
+      end = beg;
+    }
+    __syncwarp();
+  }
+}
+
+/// The edges from the fourth on of the rows longer than a record (this
+/// lane's entry v with offer base `base` has one where `more`), one lane per
+/// row. All lanes call it.
+template <int Mode>
+__device__ __noinline__ int restOfRows(const EngineParams &P, bool donate, int farCount, bool more, int k,
+                                       int v, u64 base) {
+  AsyncCta &C = asyncCta();
+  const AsyncObj &O = C.obj[k];
+  const int *outRow = Mode == kModeCombined ? P.combRow : P.outRow;
+  const int *outCol = Mode == kModeCombined ? P.combCol : P.outCol;
+  int e = 0, end = 0;
+  if (more) {
+    e = ldLoop<Mode>(outRow + v) + kRecordEdges;
+    end = ldLoop<Mode>(outRow + v + 1);
+  }
+  while (__any_sync(kFull, e < end)) {
+    const bool in = e < end;
+    const int x = in ? ldLoop<Mode>(outCol + e) : P.source;
+    const u64 cw =
+        base + static_cast<u64>(in ? static_cast<unsigned>(ldLoop<Mode>(O.outW + e)) : 0u) * O.scale;
+    u64 old = 0;
+    if (in && x != P.source && cw <= O.mostWord) old = atomicMin(O.packed + x, cw);
+    pushEdges<Mode>(P, O, donate, farCount, k, x, cw, old);
+    ++e;
+  }
+  return farCount;
+}
+
+/// Thin wavefronts of a graph with row records: up to eight entries, four
+/// lanes each (lane sub of the quad takes the record's edge sub), expanded
+/// hop after hop by the same warp for as long as they improve something
+/// below the threshold. The record of a head is requested before its
+/// atomicMin, so a hop is one round trip to L2 and a short run of
+/// instructions (a lone warp issues them one after another, so they count
+/// as much as the round trip): words are compared without unpacking them,
+/// and the next hop's entries pass through slots in shared memory. More than
+/// eight go to an idle warp by mail, or to the ring.
+template <int Mode>
+__device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int farCount, int k, int v,
+                                         u64 base, int x, int t) {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  const int sub = static_cast<int>(lane & 3u);
+  const int q = static_cast<int>(lane >> 2);
+  HopSlot *slots = C.hop[threadIdx.x >> 5];
+  const AsyncObj *O = &C.obj[k];
+  u64 *packed = O->packed;
+  const int4 *rec = O->rec;
+  u64 thrWord = O->thrWord, mostWord = O->mostWord;
+  unsigned scale = O->scale, mask = O->mask;
+  const bool oneK = C.K == 1;
+  for (unsigned hops = 1;; ++hops) {
+    if ((hops & 4095u) == 0 && (ldShared(&C.abort) != 0 || globalNs() > C.deadline)) {
+      atomicCAS(&P.ctl->status, 0, MOSP_ERR_TIMEOUT);
+      stShared(&C.abort, 1);
+      return farCount;
+    }
+    const u64 cw = static_cast<u64>(static_cast<unsigned>(t)) * scale + base;
+    u64 old = 0;
+    int4 cols, wts;
+    if (x >= 0 && cw <= mostWord) {
+      // (volatile, so that they are requested before the atomicMin)
+      asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(cols.x), "=r"(cols.y), "=r"(cols.z), "=r"(cols.w)
+                   : "l"(rec + 2LL * x));
+      asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(wts.x), "=r"(wts.y), "=r"(wts.z), "=r"(wts.w)
+                   : "l"(rec + 2LL * x + 1));
+      old = atomicMin(packed + x, cw);
+    }
+    if (__any_sync(kFull, x == kMoreEdges)) {
+      farCount = restOfRows<Mode>(P, donate, farCount, x == kMoreEdges, k, v, base);
+    }
+    const bool imp = old > (cw | mask);
+    const bool near = imp && cw < thrWord;
+    const unsigned keep = __ballot_sync(kFull, near);
+    farAppend(P, farCount, imp && !near && newInFar<Mode>(*O, old, x), k, x, cw >> O->bits);
+    if (keep == 0) return farCount;
+    const int count = __popc(keep);
+    const int rank = __popc(keep & ((1u << lane) - 1u));
+    if (count > kQuadBatch) {
+      // the next eight by mail to an idle warp
+      int w = -1, busy = 0;
+      if (lane == 0) {
+        w = takeIdle();
+        busy = w < 0 && ldShared(&C.tail) - ldShared(&C.head) > kChaseRing;
+      }
+      w = __shfl_sync(kFull, w, 0);
+      busy = __shfl_sync(kFull, busy, 0);
+      int kept = kQuadBatch;
+      if (w >= 0) {
+        if (near && rank >= kQuadBatch && rank < 2 * kQuadBatch) {
+          C.mailbox[w][rank - kQuadBatch] = HopSlot{cw, x, k, cols, wts};
+        }
+        __syncwarp();
+        if (lane == 0) {
+          const int sent = count - kQuadBatch < kMail ? count - kQuadBatch : kMail;
+          atomicAdd(&C.mailed, static_cast<unsigned>(sent));
+          C.mail[w] = sent;
+          barArrive(&C.bar[w]);
+        }
+        kept = 2 * kQuadBatch;
+      }
+      // a CTA with work for all its warps keeps the breadth-first order
+      const unsigned give = __ballot_sync(kFull, near && (busy || rank >= kept));
+      if (give != 0) ringPush(P, give, donate, nearEntry(k, x, cw >> O->bits));
+      if (busy) return farCount;
+    }
+    // quad q goes on with the q-th of them
+    if (near && rank < kQuadBatch) slots[rank] = HopSlot{cw, x, k, cols, wts};
+    __syncwarp();
+    x = -1;
+    if (q < count) {
+      const HopSlot &h = slots[q];
+      v = h.v;
+      if (!oneK) {
+        k = h.k;
+        O = &C.obj[k];
+        packed = O->packed;
+        rec = O->rec;
+        thrWord = O->thrWord;
+        mostWord = O->mostWord;
+        scale = O->scale;
+        mask = O->mask;
+      }
+      x = reinterpret_cast<const int *>(&h.cols)[sub];
+      t = reinterpret_cast<const int *>(&h.wts)[sub];
+      base = nextBase(h.word, v, mask);
+      if (sub == 0) atomicAdd(&C.expanded[k], 1u);
+    }
+    __syncwarp();
+  }
+}
+
+/// One entry per lane of a graph with row records: its word and its record
+/// arrive together, its edges' atomicMin go out together, the improvements
+/// of the warp take one reservation of the ring.
+template <int Mode>
+__device__ __noinline__ int expandRecords(const EngineParams &P, bool donate, int farCount, int k, int v,
+                                          u64 base, bool live, int4 cols, int4 wts) {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  const AsyncObj &O = C.obj[k];
+  const unsigned scale = O.scale;
+  const u64 most = live ? O.mostWord : 0;  // 0: nothing passes
+  const u64 thrWord = O.thrWord;
+  const int x[4] = {cols.x, cols.y, cols.z, cols.w};
+  const u64 cw[4] = {static_cast<u64>(static_cast<unsigned>(wts.x)) * scale + base,
+                     static_cast<u64>(static_cast<unsigned>(wts.y)) * scale + base,
+                     static_cast<u64>(static_cast<unsigned>(wts.z)) * scale + base,
+                     static_cast<u64>(static_cast<unsigned>(wts.w)) * scale + base};
+  u64 old[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    old[h] = 0;
+    if (x[h] >= 0 && cw[h] <= most) old[h] = atomicMin(O.packed + x[h], cw[h]);
+  }
+  if (__any_sync(kFull, live && x[3] == kMoreEdges)) {
+    farCount = restOfRows<Mode>(P, donate, farCount, live && x[3] == kMoreEdges, k, v, base);
+  }
+  unsigned near = 0, far = 0;  // bit h: this lane's edge h
+  unsigned ballot[4];
+  int count = 0;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const bool imp = old[h] > (cw[h] | O.mask);
+    const bool nr = imp && cw[h] < thrWord;
+    near |= static_cast<unsigned>(nr) << h;
+    far |= static_cast<unsigned>(imp && !nr && newInFar<Mode>(O, old[h], x[h])) << h;
+    ballot[h] = __ballot_sync(kFull, nr);
+    count += __popc(ballot[h]);
+  }
+  if (count > 0) {
+    unsigned at = 0;
+    int room = 0;
+    if (lane == 0) room = ringReserve(donate, count, at);
+    room = __shfl_sync(kFull, room, 0);
+    at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      if (ballot[h] == 0) continue;
+      const u64 e = nearEntry(k, x[h], cw[h] >> O.bits);
+      if (!room) {
+        spillNear(P, ballot[h], e);
+      } else {
+        if ((near >> h) & 1u) ringWrite(P, at + __popc(ballot[h] & ((1u << lane) - 1u)), e);
+        at += __popc(ballot[h]);
+      }
+    }
+  }
+  if (__any_sync(kFull, far != 0)) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) farAppend(P, farCount, (far >> h) & 1u, k, x[h], cw[h] >> O.bits);
+  }
+  return farCount;
+}
+
+/// The rows of the lanes' entries (this lane's: edges [beg, end) of v at
+/// distance du in objective k; beg == end for none) as one flat range of
+/// edges, three per lane and turn. All lanes call it.
+template <int Mode>
+__device__ __forceinline__ void expandRows(const EngineParams &P, const int *outCol, bool donate,
+                                           int &farCount, int k, int v, u64 du, int beg, int end) {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  const u64 base = offerBase(C.obj[k], du, v);
+  int deg = end - beg;
+  // a row of more than 2^20 edges goes to the whole warp by itself
+  unsigned huge = __ballot_sync(kFull, deg > (1 << 20));
+  while (huge != 0) {
+    const int src = __ffs(huge) - 1;
+    huge &= huge - 1;
+    const int kb = __shfl_sync(kFull, k, src);
+    const u64 ob = __shfl_sync(kFull, base, src);
+    const int bb = __shfl_sync(kFull, beg, src);
+    const int eb = __shfl_sync(kFull, end, src);
+    const AsyncObj &O = C.obj[kb];
+    for (int e0 = bb; e0 < eb; e0 += 32) {
+      const int e = e0 + static_cast<int>(lane);
+      const int x = e < eb ? ldLoop<Mode>(outCol + e) : P.source;
+      const u64 cw =
+          ob + static_cast<u64>(static_cast<unsigned>(e < eb ? ldLoop<Mode>(O.outW + e) : 0)) * O.scale;
+      const u64 old = x != P.source && cw <= O.mostWord ? atomicMin(O.packed + x, cw) : 0;
+      pushEdges<Mode>(P, O, donate, farCount, kb, x, cw, old);
+    }
+  }
+  if (deg > (1 << 20)) deg = 0;
+  int incl = deg;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(kFull, incl, off);
+    if (static_cast<int>(lane) >= off) incl += o;
+  }
+  const int edges = __shfl_sync(kFull, incl, 31);
+  const int first = beg - (incl - deg);
+  constexpr int SL = kSlotsAsync;
+  for (int s0 = 0; s0 < edges; s0 += 32 * SL) {
+    int kk[SL], ww[SL];
+    u64 cw[SL], old[SL];
+#pragma unroll
+    for (int h = 0; h < SL; ++h) {
+      const int sl = s0 + 32 * h + static_cast<int>(lane);
+      const int o = slotOwner(incl, sl);
+      kk[h] = __shfl_sync(kFull, k, o);
+      cw[h] = __shfl_sync(kFull, base, o);
+      const int e = __shfl_sync(kFull, first, o) + sl;
+      ww[h] = P.source;
+      if (sl < edges) {
+        const AsyncObj &O = C.obj[kk[h]];
+        ww[h] = ldLoop<Mode>(outCol + e);
+        cw[h] += static_cast<u64>(static_cast<unsigned>(ldLoop<Mode>(O.outW + e))) * O.scale;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < SL; ++h) {
+      const AsyncObj &O = C.obj[kk[h]];
+      old[h] = ww[h] != P.source && cw[h] <= O.mostWord ? atomicMin(O.packed + ww[h], cw[h]) : 0;
+    }
+#pragma unroll
+    for (int h = 0; h < SL; ++h) pushEdges<Mode>(P, C.obj[kk[h]], donate, farCount, kk[h], ww[h], cw[h], old[h]);
+  }
+}
+
+/// An idle warp's wait (warps other than 0): the entries that came by mail,
+/// 0 when it has to look around again. All lanes call it.
+__device__ __forceinline__ int asyncWait(const EngineParams &P, const Sync &sync, unsigned &parity) {
+  AsyncCta &C = asyncCta();
+  const int warp = static_cast<int>(threadIdx.x >> 5);
+  int mail = 0;
+  if (laneId() == 0) {
+    atomicOr(&C.idle, 1u << warp);
+    __threadfence_block();
+    // what came between the last look and the idle bit
+    bool wait = true;
+    if (ldShared(&C.over) != 0 || ldShared(&C.abort) != 0 || ldShared(&C.tail) != ldShared(&C.head)) {
+      // (a cleared bit means that a signal is on its way)
+      wait = ((atomicAnd(&C.idle, ~(1u << warp)) >> warp) & 1u) == 0;
+    }
+    if (wait) {
+      unsigned turns = 0;
+      while (!barTryWait(&C.bar[warp], parity)) {
+        ++turns;
+        if (ldShared(&C.abort) != 0) break;
+        if ((turns & 255u) == 0 && globalNs() > sync.deadline + 1000000000ULL) {
+          asyncAbort(P);
+          break;
+        }
+      }
+      parity ^= 1u;
+      mail = ldShared(&C.mail[warp]);
+    }
+  }
+  parity = __shfl_sync(kFull, parity, 0);
+  return __shfl_sync(kFull, mail, 0);
+}
+
+/// One phase for one warp: entries of the CTA's share and ring until the
+/// phase is over (true) or the launch stops (false).
+template <int Mode, int Kind>
+__device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *outRow, const int *outCol,
+                                             unsigned phase, const Sync &sync, unsigned &parity) {
+  AsyncCta &C = asyncCta();
+  const LoopShared &L = C.L;
+  EngineControl *c = P.ctl;
+  unsigned owed = 0;    // finished entries not yet added to the CTA's count
+  int farCount = 0;     // entries in the warp's far buffer
+  bool donate = false;  // other CTAs have run dry
+  constexpr bool Rec = Kind != kCsrOnly;
+  constexpr bool wideRecords = Kind == kRecords;
+  const unsigned lane = laneId();
+  const int warp = threadIdx.x >> 5;
+  unsigned spins = 0, rounds = 0;
+  while (true) {
+    // ---- a batch of the ring, or of the share while the ring is short ----
+    unsigned what = 0, at = 0;  // what: source << 8 | entries, donate in bit 16
+    if (lane == 0) {
+      while (true) {
+        const unsigned h = ldShared(&C.head);
+        const unsigned held = ldShared(&C.tail) - h;
+        const unsigned cur = ldShared(&C.cur);
+        if (cur < C.share && held <= kSliceFirst) {
+          const unsigned left = C.share - cur;
+          const unsigned n = left >= 1024 ? 32u : (left + 31u) >> 5;
+          at = atomicAdd(&C.cur, n);
+          if (at >= C.share) continue;
+          what = (2u << 8) | (C.share - at < n ? C.share - at : n);
+          break;
+        }
+        if (held == 0) break;
+        const unsigned n = held >= 128 ? 32u : (held + 3u) >> 2;
+        if (atomicCAS(&C.head, h, h + n) != h) continue;
+        at = h;
+        what = (1u << 8) | n;
+        if (held > kDonate) what |= 1u << 16;
+        break;
+      }
+    }
+    what = __shfl_sync(kFull, what, 0);
+    int k = 0, v = 0;
+    if (what == 0) {
+      // ---- idle: settle what is done, then wait ---------------------------
+      if (owed != 0) {
+        if (farCount > 0) flushFarEntries(P, farCount);
+        farCount = 0;
+        if (lane == 0) {
+          __threadfence_block();
+          const unsigned now = atomicAdd(&C.settled, owed) + owed;
+          __threadfence_block();
+          if (now == ldShared(&C.tail) + ldShared(&C.mailed) + C.share) asyncDry(P, phase);
+        }
+        owed = 0;
+        __syncwarp();
+        continue;
+      }
+      int stop = 0;
+      if (lane == 0) stop = ldShared(&C.abort) != 0 ? 2 : ldShared(&C.over);
+      stop = __shfl_sync(kFull, stop, 0);
+      if (stop == 2) return false;
+      if (stop == 1) return true;
+      if (warp == 0) {
+        asyncFetch(P, phase);
+        if ((++spins & 63u) == 0 && lane == 0 &&
+            (ldVolatile(&c->status) != 0 || globalNs() > sync.deadline)) {
+          asyncAbort(P);
+        }
+        __nanosleep(40);
+        __syncwarp();
+        continue;
+      }
+      const int mail = asyncWait(P, sync, parity);
+      if constexpr (Rec) {
+        if (mail > 0) {
+          owed += mail;
+          const int q = static_cast<int>(lane >> 2);
+          u64 base = 0;
+          int x = -1, t = 0;
+          if (q < mail) {
+            const HopSlot &h = C.mailbox[warp][q];
+            k = h.k;
+            v = h.v;
+            base = nextBase(h.word, v, C.obj[k].mask);
+            x = reinterpret_cast<const int *>(&h.cols)[lane & 3u];
+            t = reinterpret_cast<const int *>(&h.wts)[lane & 3u];
+            if ((lane & 3u) == 0) atomicAdd(&C.expanded[k], 1u);
+          }
+          __syncwarp();
+          farCount = chaseRecords<Mode>(P, donate, farCount, k, v, base, x, t);
+        }
+      }
+      continue;
+    }
+    at = __shfl_sync(kFull, at, 0);
+    spins = 0;
+    if ((++rounds & 1023u) == 0 && asyncStop(P)) return false;
+    const bool fromRing = ((what >> 8) & 3u) == 1u;
+    const unsigned n = what & 63u;
+    // other CTAs have run dry (read with the entries' loads)
+    int hungry = 0;
+    if (lane == 0) {
+      if ((what >> 16) != 0) hungry = ldVolatile(&c->asyncHungry[phase % 3]);
+      atomicAdd(&C.rounds, 1u);
+      atomicAdd(&C.items, n);
+    }
+    owed += n;
+    // few entries: a group of lanes each, expanded hop after hop
+    constexpr unsigned kGroup = Rec ? 4 : 8;
+    const bool thin = n <= 32 / kGroup;
+    const unsigned mine = thin ? lane / kGroup : lane;
+    const bool lead = !thin || lane % kGroup == 0;
+    const bool have = mine < n;
+    unsigned tag = kTagSat;
+    bool marked = false;
+    if (fromRing) {
+      u64 *slot = asyncRing() + ((at + mine) & kRingMask);
+      u64 e = kEmptySlot;
+      if (have) {
+        unsigned spin = 0;
+        while ((e = ldShared(slot)) == kEmptySlot) {  // reserved, about to be written
+          if (++spin > kSpinLimit || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
+            asyncAbort(P);
+            e = 0;
+            break;
+          }
+        }
+        k = static_cast<int>(e & 31u);
+        v = static_cast<int>(static_cast<unsigned>(e) >> 5);
+        tag = static_cast<unsigned>(e >> 32);
+      }
+      __syncwarp();
+      if (have && lead) stShared(slot, kEmptySlot);
+    } else if (have) {
+      const long long j = C.base + at + mine;
+      while (k + 1 < P.K && L.off[k + 1] <= j) ++k;
+      const unsigned raw = static_cast<unsigned>(
+          __ldcg((L.fp[k] == 0 ? P.farL0 : P.farL1) + static_cast<long long>(k) * P.strideFar +
+                 (j - L.off[k])));
+      v = static_cast<int>(raw & ~kOverflow);
+      marked = (raw & kOverflow) != 0;
+      if (marked || phase == 0) {
+        // the flag is cleared before the word is read, so a push that still
+        // finds it set is covered by the distance read here
+        if (lead) atomicExch(P.inFar + static_cast<long long>(k) * P.stride + v, 0);
+        __threadfence();
+      }
+    }
+    if (!fromRing) __syncwarp();
+    u64 word = kInfWord;
+    int beg = 0, end = 0;
+    // the entry's row record (thin: the lane's edge of it)
+    const bool records = Rec && (thin || wideRecords);
+    int4 cols = make_int4(-1, -1, -1, -1), wts = make_int4(0, 0, 0, 0);
+    if (have) {
+      word = __ldcg(C.obj[k].packed + v);
+      if (records) {
+        const int4 *r = C.obj[k].rec + 2LL * v;
+        if (thin) {
+          cols.x = reinterpret_cast<const int *>(r)[lane & 3u];
+          wts.x = reinterpret_cast<const int *>(r)[4 + (lane & 3u)];
+        } else {
+          cols = r[0];
+          wts = r[1];
+        }
+      } else {
+        beg = ldLoop<Mode>(outRow + v);
+        end = ldLoop<Mode>(outRow + v + 1);
+      }
+    }
+    // A ring entry is stale when its vertex has improved since (the newer
+    // distance has its own entry); else it is expanded with its tag, which
+    // also covers a word read that is older than the entry. A pile entry
+    // below the last phase's threshold was expanded when it got there.
+    const AsyncObj &O = C.obj[k];
+    const u64 d = word == kInfWord ? kInfWord : word >> O.bits;
+    bool live = false;
+    u64 du = d;
+    if (fromRing) {
+      if (tag < kTagSat) {
+        live = have && d >= tag;
+        du = tag;
+      } else {
+        live = have && d != kInfWord;
+      }
+    } else {
+      const bool near = d < O.thr;
+      live = have && near && (marked || d >= O.prev);
+      farAppend(P, farCount, have && !near && lead, k, v, d);
+    }
+    if (live && lead) atomicAdd(&C.expanded[k], 1u);
+    donate = __shfl_sync(kFull, hungry, 0) > 0;
+    if constexpr (Rec) {
+      const u64 base = offerBase(O, du, v);
+      if (thin) {
+        farCount = chaseRecords<Mode>(P, donate, farCount, k, v, base, live ? cols.x : -1, wts.x);
+        continue;
+      }
+      if (wideRecords) {
+        farCount = expandRecords<Mode>(P, donate, farCount, k, v, base, live, cols, wts);
+        continue;
+      }
+    }
+    if (!live) end = beg;
+    if constexpr (!Rec) {
+      if (thin && !__any_sync(kFull, end - beg > kOctDeg)) {
+        chase<Mode>(P, outRow, outCol, donate, farCount, k, v, du, beg, end);
+        continue;
+      }
+    }
+    expandRows<Mode>(P, outCol, donate, farCount, k, v, du, beg, lead ? end : beg);
+  }
+}
+
+template <int Mode, int Kind>
+__device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outRow, const int *outCol,
+                                          const int *const *outWk, Sync &epoch, u64 *deltaOverride,
+                                          int genBase) {
+  AsyncCta &C = asyncCta();
+  LoopShared &L = C.L;
   StageHeader &H = stageHeader();
   EngineControl *c = P.ctl;
   const int K = P.K;
-  const int S = P.aqShards;
   const unsigned lane = laneId();
   const int warp = threadIdx.x >> 5;
-  const long long gwarp = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + warp;
-  const long long nwarps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  const Sync sync = epoch;
 
   // per-objective state, held by lane k of warp 0 (the same in every CTA)
   u64 thr = 0;
@@ -1281,15 +2063,32 @@ __device__ bool asyncNearFar(const EngineParams &P, const int *outRow, const int
   if (warp == 0 && static_cast<int>(lane) < K) {
     delta = P.obj[lane].delta;
     if (deltaOverride != nullptr && lane == 0) delta = *deltaOverride;
+    const ObjectiveArgs &O = P.obj[lane];
+    AsyncObj &A = C.obj[lane];
+    A.packed = P.packed + lane * P.stride;
+    A.rec = P.rec == nullptr ? nullptr : P.rec + 2 * lane * P.stride;
+    A.outW = outWk[lane];
+    A.dist = O.dist;
+    A.bits = O.parentBits;
+    A.scale = 1u << O.parentBits;
+    A.mask = A.scale - 1u;
+    A.mostWord = (O.maxDist << O.parentBits) | A.mask;
+    A.thr = 0;
   }
-  if (threadIdx.x < kMaxK) H.expanded[threadIdx.x] = 0;
-  if (threadIdx.x < kWarps) {
-    H.asyncFar[threadIdx.x] = 0;
-    H.asyncLocal[threadIdx.x] = 0;
+  if (threadIdx.x < kMaxK) C.expanded[threadIdx.x] = 0;
+  if (threadIdx.x < kWarps) barInit(&C.bar[threadIdx.x]);
+  if (threadIdx.x == 0) {
+    C.lock = 0;
+    C.abort = 0;
+    C.idle = 0;
+    C.rounds = C.items = C.taken = 0;
+    C.K = K;
+    C.deadline = sync.deadline;
   }
+  for (int i = threadIdx.x; i < kRing; i += blockDim.x) asyncRing()[i] = kEmptySlot;
+  unsigned parity = 0;
   const unsigned long long t0 = globalNs();
   unsigned long long tPhase = t0;
-  AsyncCounts cnt{0, 0, 0, 0};
   unsigned phase = 0;
   for (;; ++phase) {
     if (threadIdx.x < kMaxK) H.farMin[threadIdx.x] = kInfWord;
@@ -1298,37 +2097,74 @@ __device__ bool asyncNearFar(const EngineParams &P, const int *outRow, const int
       const bool act = k < K;
       int mode = kDone;
       long long items = 0;
+      u64 least = 0;
       if (act) {
         const int fc = __ldcg(&c->farCount[k][fs]);
+        const u64 mnC = __ldcg(&c->farMinC[k][fs]);
+        C.obj[k].prev = thr;
         if (fc > 0) {
           mode = kSplit;
           items = fc;
-          const u64 mnC = __ldcg(&c->farMinC[k][fs]);
-          u64 lo = thr;
-          if (mnC != 0) {
-            const u64 mn = ~mnC;
-            lo = mn > thr ? mn : thr;
-          }
-          thr = (lo > kInfWord - delta) ? kInfWord - 1 : lo + delta;
+          if (mnC != 0) least = ~mnC;
         }
       }
       long long incl = items;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
+      for (int off = 1; off < K; off <<= 1) {
         const long long o = __shfl_up_sync(kFull, incl, off);
         if (static_cast<int>(lane) >= off) incl += o;
+      }
+      const long long total = __shfl_sync(kFull, incl, K - 1);
+      if (mode == kSplit) {
+        // Thin phases (few entries per CTA) are twice as wide: they pay for
+        // their start and end more than for entries expanded again. Twice
+        // the width everywhere: loop from scratch of a 497,700-vertex road
+        // network 2.90 -> 2.50 ms (1,500 entries per phase), combined graph
+        // of 249,500 vertices 1.47 -> 1.29 ms, but the update of 2M vertices
+        // with 1.2M entries per phase 1.20 -> 1.30 ms; four times: 2.71,
+        // 1.38 and 1.25 ms.
+        const u64 width = total <= static_cast<long long>(kThinShare) * gridDim.x ? 2 * delta : delta;
+        const u64 lo = least > thr ? least : thr;
+        thr = lo > kInfWord - width ? kInfWord - 1 : lo + width;
       }
       if (act) {
         L.off[k] = incl - items;
         L.thr[k] = thr;
+        AsyncObj &A = C.obj[k];
+        A.thr = thr;
+        A.thrWord = thr > (kInfWord >> A.bits) ? kInfWord : thr << A.bits;
         L.mode[k] = mode;
         L.fp[k] = fp;
         L.fs[k] = fs;
       }
-      const long long total = __shfl_sync(kFull, incl, 31);
-      if (lane == 0) L.total = total;
+      if (lane == 0) {
+        // this CTA's share: an equal, contiguous range of the piles
+        const long long per = (total + gridDim.x - 1) / gridDim.x;
+        const long long lo = per * blockIdx.x < total ? per * blockIdx.x : total;
+        const long long hi = lo + per < total ? lo + per : total;
+        L.total = total;
+        C.base = lo;
+        C.share = static_cast<unsigned>(hi - lo);
+        C.head = C.tail = C.cur = C.settled = C.mailed = 0;
+        C.owed = 1;
+        C.dry = 0;
+        C.over = 0;
+        C.phase = phase;
+        if (blockIdx.x == 0) {
+          // the counters of the next phase (last looked at before this one)
+          c->asyncPending[(phase + 1) % 3] = gridDim.x;
+          c->asyncHungry[(phase + 1) % 3] = 0;
+        }
+        if (globalNs() > sync.deadline) {
+          atomicCAS(&c->status, 0, MOSP_ERR_TIMEOUT);
+          L.total = -1;  // the launch stops
+        }
+      }
+      if (blockIdx.x == 0 && static_cast<int>(lane) < P.aqShards) {
+        P.aqCtr[(phase + 1) % 3 * P.aqShards + lane].claimed = 0;
+      }
       if (act && mode == kSplit) {
         if (blockIdx.x == 0) {
+          // the slot the next phase appends to (last read a phase ago)
           c->farCount[k][(fs + 2) % 3] = 0;
           c->farMinC[k][(fs + 2) % 3] = 0;
         }
@@ -1337,60 +2173,12 @@ __device__ bool asyncNearFar(const EngineParams &P, const int *outRow, const int
         fs = (fs + 1) % 3;
       }
     }
-    // the counter set of the next phase (last used two phases ago)
-    if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < S) {
-      AsyncShard &nx = P.aqCtr[((phase + 1) & 1u) * S + threadIdx.x];
-      nx.head = 0;
-      nx.tail = 0;
-      nx.done = 0;
-    }
     __syncthreads();
-    const long long total = L.total;
-    if (total == 0) break;
-    AsyncShard *ctr = P.aqCtr + (phase & 1u) * S;
-
-    // ---- split: this warp's share of the far piles, below the new
-    // threshold to the near queue, the rest to the other pile
-    {
-      // (split pushes all go to the queue: a warp settles nothing in the
-      // split, so it must not hold local work past it)
-      AsyncState A{ctr, static_cast<int>(gwarp % S), 0u, false};
-      for (long long base = gwarp * 32; base < total; base += nwarps * 32) {
-        if (farBufferFull(32)) flushAsyncFar(P, L);
-        const long long j = base + lane;
-        if (j < total) {
-          int k = 0;
-          while (k + 1 < K && L.off[k + 1] <= j) ++k;
-          const long long ko = static_cast<long long>(k) * P.stride;
-          const int v = __ldcg((L.fp[k] == 0 ? P.farL0 : P.farL1) + ko + (j - L.off[k]));
-          const u64 word = __ldcg(P.packed + ko + v);
-          const u64 d = word == kInfWord ? kInfWord : pkOf(P.obj[k]).dist(word);
-          if (d < L.thr[k]) {
-            P.inFar[ko + v] = 0;
-            asyncNear(P, L, A, k, v, d);
-          } else {
-            asyncFar(P, L, k, v, d);
-          }
-        }
-        settleRound(ctr, 0, 0u, A.target, A.spilled);
-        A.spilled = 0;
-        A.target = A.target + 1 == S ? 0 : A.target + 1;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      redRelease(&c->asyncSplit, 1u);
-    }
-
-    // ---- expand until the phase runs dry
-    if (!asyncConsume<Mode>(P, L, outRow, outCol, outWk, ctr, phase, gwarp, epoch, cnt)) return false;
-    flushAsyncFar(P, L);
-    __syncthreads();
-    if (threadIdx.x < K && H.farMin[threadIdx.x] != kInfWord) {
-      atomicMax(listTarget(P, L, K + threadIdx.x, 0, nullptr, nullptr).minC, ~H.farMin[threadIdx.x]);
-    }
-    if (!gridSync(c, epoch)) return false;
+    if (L.total < 0) return false;
+    if (L.total == 0) break;
+    if (threadIdx.x == 0 && C.share == 0) asyncDry(P, phase);
+    const bool ok = asyncConsume<Mode, Kind>(P, outRow, outCol, phase, sync, parity);
+    if (__syncthreads_or(!ok)) return false;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       // phase durations (the first four, then the rest summed)
       const unsigned long long now = globalNs();
@@ -1398,20 +2186,19 @@ __device__ bool asyncNearFar(const EngineParams &P, const int *outRow, const int
       tPhase = now;
     }
   }
-  if (lane == 0 && (cnt.queueRounds | cnt.localRounds) != 0) {
+  if (threadIdx.x == 0 && C.rounds != 0) {
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopIters[1]),
-              static_cast<unsigned long long>(cnt.queueRounds + cnt.localRounds));
-    atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopItems[0]),
-              static_cast<unsigned long long>(cnt.queueItems));
-    atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopItems[1]),
-              static_cast<unsigned long long>(cnt.localItems));
+              static_cast<unsigned long long>(C.rounds));
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopNs[1]),
-              static_cast<unsigned long long>(cnt.localRounds));
+              static_cast<unsigned long long>(C.rounds));
+    atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopItems[0]),
+              static_cast<unsigned long long>(C.taken));
+    atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopItems[1]),
+              static_cast<unsigned long long>(C.items));
   }
-
-  if (threadIdx.x < K && H.expanded[threadIdx.x] != 0) {
+  if (threadIdx.x < K && C.expanded[threadIdx.x] != 0) {
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->pushes[threadIdx.x]),
-              static_cast<unsigned long long>(H.expanded[threadIdx.x]));
+              static_cast<unsigned long long>(C.expanded[threadIdx.x]));
   }
   if (blockIdx.x == 0 && warp == 0 && static_cast<int>(lane) < K) {
     c->iterations[lane] = phasesK;
@@ -1701,18 +2488,58 @@ template <int Mode>
 __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBase,
                                   const int **sOutWk);
 
+/// Row records for the asynchronous loop, one 32-byte sector per objective
+/// and vertex: the heads of its first four edges (-1: none, or the source,
+/// which nothing improves) and their weights. A row of more than four edges
+/// holds kMoreEdges in place of the fourth; the rest stays in the CSR.
+/// Thread tid of T.
+template <int Mode>
+__device__ void buildRecords(const EngineParams &P, const int *outRow, const int *outCol,
+                             const int *const *outWk, long long tid, long long T) {
+  for (long long v = tid; v < P.n; v += T) {
+    const int b = ldLoop<Mode>(outRow + v);
+    const int deg = ldLoop<Mode>(outRow + v + 1) - b;
+    int c[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] = q < deg ? ldLoop<Mode>(outCol + b + q) : -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] = c[q] == P.source ? -1 : c[q];
+    if (deg > 4) c[3] = kMoreEdges;
+    for (int k = 0; k < P.K; ++k) {
+      int w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[q] = q < deg ? ldLoop<Mode>(outWk[k] + b + q) : 0;
+      int4 *r = P.rec + 2 * (static_cast<long long>(k) * P.stride + v);
+      r[0] = make_int4(c[0], c[1], c[2], c[3]);
+      r[1] = make_int4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
 /// The near-far loop of a launch: asynchronous when the launch asks for it
 /// and the graph has no hub rows (which the bulk loop hands to whole CTAs);
 /// the same decision in every CTA (the hub flag is set before a barrier).
 template <int Mode>
 __device__ bool runNearFar(const EngineParams &P, const int *outRow, const int *outCol,
-                           const int *const *outWk, Sync &epoch, u64 *deltaOverride, int genBase) {
-  const bool async = (P.flags & kFlagAsync) != 0 && P.aqSlots != nullptr && P.aqShards > 0 &&
+                           const int *const *outWk, Sync &epoch, u64 *deltaOverride, int genBase,
+                           bool rec) {
+  // the asynchronous loop adds a weight to a packed word without a check: a
+  // bound within 2^31 of what the word holds goes to the bulk loop
+  bool fits = true;
+  for (int k = 0; k < P.K; ++k) {
+    fits = fits && P.obj[k].maxDist + (1ULL << 31) <= (kInfWord >> P.obj[k].parentBits);
+  }
+  const bool async = fits && (P.flags & kFlagAsync) != 0 && P.aqSlots != nullptr && P.aqShards > 0 &&
                      P.aqShards <= kAsyncShards && P.n <= (1 << 27) &&
-                     P.stageEntries * sizeof(StageEntry) >=
-                         kWarps * (kFarBuf * sizeof(int) + kLocalBuf * sizeof(u64)) &&
+                     P.stageEntries >= kStageEntriesAsync &&
                      __ldcg(&P.ctl->heavy) == 0;
-  if (async) return asyncNearFar<Mode>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
+  if (async && rec && 32LL * P.n * P.K <= kRecordBytes) {
+    return asyncNearFar<Mode, kRecords>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
+  }
+  if (async && rec) {
+    return asyncNearFar<Mode, kThinRecords>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
+  }
+  if (async) return asyncNearFar<Mode, kCsrOnly>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
   return nearFarLoop<Mode>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
 }
 
@@ -1771,7 +2598,7 @@ __device__ void pushFromValid(const EngineParams &P, int k, const int *w, long l
     if (nd >= pk.dist(old)) return;
     if (atomicExch(P.inFar + ko + x, 1) == 0) {
       const int idx = warpAppend(&c->farCount[k][0]);
-      P.farL0[ko + idx] = x;
+      P.farL0[static_cast<long long>(k) * P.strideFar + idx] = x;
       warpMinInto(&c->farMinC[k][0], nd);
     }
   };
@@ -1825,14 +2652,12 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
   const int *outCol = P.outCol;
 
   markPhase(c, kPhaseStart);
-  // both counter sets of the asynchronous near queue start at zero (every
-  // mode passes a grid barrier before its near-far loop)
+  // the asynchronous loop's spill queue starts empty and every CTA owes its
+  // share of the first phase (every mode passes a grid barrier before its
+  // near-far loop)
   if ((P.flags & kFlagAsync) != 0 && P.aqCtr != nullptr) {
-    for (long long i = tid; i < 2LL * P.aqShards; i += T) {
-      P.aqCtr[i].head = 0;
-      P.aqCtr[i].tail = 0;
-      P.aqCtr[i].done = 0;
-    }
+    for (long long i = tid; i < P.aqShards; i += T) P.aqCtr[i].claimed = 0;
+    if (tid == 0) c->asyncPending[0] = gridDim.x;
   }
   if constexpr (Mode == kModeUpdate) {
     // ---- Heavy rows: does the graph have rows for whole-CTA handling? -----
@@ -1884,6 +2709,8 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
     }
     if (badParent) c->invalid = 1;
     if (badDist) c->overflow = 1;
+    __syncthreads();  // sOutWk
+    if (P.rec != nullptr) buildRecords<Mode>(P, outRow, outCol, sOutWk, tid, T);
     if (!gridSync(c, epoch)) return;
     markPhase(c, kPhasePacked);
 
@@ -2077,7 +2904,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
         __syncthreads();
         for (int k = 0; k < K; ++k) {
           const int cnt = H.count[k];
-          const long long ko = static_cast<long long>(k) * P.stride;
+          const long long ko = static_cast<long long>(k) * P.strideFar;
           for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
             P.farL0[ko + H.base[k] + q] = E[k * H.cap + q].v;
           }
@@ -2145,7 +2972,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
             P.inFar[ko + v] = 1;
             if (!staged) {
               const int idx = warpAppend(&c->farCount[k][0]);
-              P.farL0[ko + idx] = v;
+              P.farL0[static_cast<long long>(k) * P.strideFar + idx] = v;
               warpMinInto(&c->farMinC[k][0], pk.dist(best));
             } else {
               const unsigned peers = __match_any_sync(__activemask(), k);
@@ -2199,7 +3026,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
                 if (ph.dist(besth) < (curh == kInfWord ? kInfWord : ph.dist(curh))) {
                   P.inFar[koh + vh] = 1;
                   const int idx = atomicAdd(&c->farCount[kh][0], 1);
-                  P.farL0[koh + idx] = vh;
+                  P.farL0[static_cast<long long>(kh) * P.strideFar + idx] = vh;
                   atomicMax(&c->farMinC[kh][0], ~ph.dist(besth));
                 }
               }
@@ -2225,7 +3052,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
     }
     if (!gridSync(c, epoch)) return;
     markPhase(c, kPhasePulled);
-    if (!runNearFar<Mode>(P, outRow, outCol, sOutWk, epoch, nullptr, genBase)) return;
+    if (!runNearFar<Mode>(P, outRow, outCol, sOutWk, epoch, nullptr, genBase, P.rec != nullptr)) return;
     markPhase(c, kPhaseLoop);
     unpackResults<Mode>(P, outRow, outCol, sOutWk, epoch);
     if (!gridSync(c, epoch)) return;
@@ -2410,6 +3237,14 @@ __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBas
     heavyRow |= ldGraph<Mode>(outRow + v + 1) - ldGraph<Mode>(outRow + v) > heavyDegOf(P);
   }
   if (heavyRow) c->heavy = 1;
+  __syncthreads();  // sOutWk
+  // (of the combined graph only the kernel knows the edge count)
+  bool rec = P.rec != nullptr;
+  if constexpr (Mode == kModeCombined) {
+    rec = rec && recordsPay(n, static_cast<long long>(__ldcg(&c->sums[0])));
+    if (rec && !gridSync(c, epoch)) return;  // the rows are filled
+  }
+  if (rec) buildRecords<Mode>(P, outRow, outCol, sOutWk, tid, T);
   for (int k = 0; k < K; ++k) {
     const Pk pk = pkOf(P.obj[k]);
     const long long ko = static_cast<long long>(k) * P.stride;
@@ -2421,7 +3256,7 @@ __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBas
     for (long long i = tid; i < roots; i += T) {
       const int r = P.nSources > 1 ? P.sources[i] : P.source;
       P.inFar[ko + r] = 1;
-      P.farL0[ko + i] = r;
+      P.farL0[static_cast<long long>(k) * P.strideFar + i] = r;
     }
     if (tid == 0) {
       c->farCount[k][0] = roots;
@@ -2432,7 +3267,7 @@ __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBas
   markPhase(c, kPhasePulled);
   u64 *deltaOverride = nullptr;
   if constexpr (Mode == kModeCombined) deltaOverride = &sCombDelta;
-  if (!runNearFar<Mode>(P, outRow, outCol, sOutWk, epoch, deltaOverride, genBase)) return;
+  if (!runNearFar<Mode>(P, outRow, outCol, sOutWk, epoch, deltaOverride, genBase, rec)) return;
   markPhase(c, kPhaseLoop);
   unpackResults<Mode>(P, outRow, outCol, sOutWk, epoch);
   if (!gridSync(c, epoch)) return;

@@ -31,7 +31,14 @@ constexpr int kLaneRowMax = 32;               // rows above: warp-cooperative
 // entries of the per-CTA append stage of a bulk near-far launch (16 bytes
 // each, dynamic shared memory); asynchronous launches take fewer
 constexpr int kStageEntriesMax = MOSP_STAGE_ENTRIES;
-constexpr int kStageEntriesAsync = 1536;     // far buffers + local buffers of 32 warps
+// entries of an asynchronous launch: the CTA's ring of near entries (8 bytes
+// each), the far buffers of its 32 warps (128 entries of 8 bytes) and its
+// state (AsyncCta in engine.cu)
+constexpr int kRing = 8192;
+constexpr int kFarBuf = 128;
+constexpr int kMail = 8;
+constexpr int kAsyncCtaBytes = 30 * 1024;
+constexpr int kStageEntriesAsync = (kRing + kThreads / 32 * kFarBuf) / 2 + kAsyncCtaBytes / 16;
 
 enum EngineMode : int { kModeUpdate = 0, kModeScratch = 1, kModeCombined = 2 };
 
@@ -59,10 +66,13 @@ struct alignas(128) EngineControl {
   unsigned pad0[31];
   unsigned release;      // barrier epoch released by the last arrival
   unsigned pad1[31];
-  unsigned asyncPhase;   // asynchronous near-far: phases completed (monotone)
-  unsigned pad3[31];
-  unsigned asyncSplit;   // asynchronous near-far: CTAs past their phase's split (monotone)
-  unsigned pad4[31];
+  // asynchronous near-far, one slot per phase modulo three: CTAs that still
+  // work on their share of the phase plus entries of the spill queue that are
+  // not settled; CTAs that have run dry
+  unsigned asyncPending[3];
+  unsigned pad3[29];
+  int asyncHungry[3];
+  unsigned pad4[29];
   int status;            // 0 or MOSP_ERR_TIMEOUT (run aborted)
   int overflow;          // an input distance does not fit the packing
   int invalid;           // malformed input (ids out of range, cycles)
@@ -85,8 +95,9 @@ struct alignas(128) EngineControl {
   // near-far loop profile. Bulk loop (written by CTA 0): time and items of
   // iterations that split a far pile ([0]) and of pure push iterations
   // ([1]). Asynchronous loop: loopNs[0] its time, loopIters[0] its phases,
-  // loopIters[1] warp rounds, loopNs[1] of which local rounds, loopItems
-  // entries taken from the queue ([0]) and from local buffers ([1])
+  // loopIters[1] warp rounds, loopNs[1] of which on the CTA's own work, loopItems
+  // entries taken from the spill queue ([0]) and from the CTAs' own rings
+  // and far-pile shares ([1])
   unsigned long long loopNs[2];
   long long loopIters[2];
   long long loopItems[2];
@@ -112,9 +123,7 @@ enum : int {
                          // no hub rows
   kFlagPullOnly = 8,     // always pull into the candidates (never push from the
                          // valid vertices)
-  kFlagLocal = 16,       // asynchronous loop with warp-local continuation (a warp
-                         // expands up to 32 of its own pushes next); measured
-                         // slower on the road workload (more re-expansions)
+                         // 16: not used (was: per-warp continuation)
   kFlagCanonical = 32    // the input trees follow the lowest-id tie rule: with
                          // kFlagHostRecovery, distance-only objectives recover
                          // parents only where the batch can change them
@@ -128,21 +137,29 @@ enum : int {
 // whose in-row is scanned again.
 enum : unsigned char { kRecChanged = 1, kRecScan = 2 };
 
-/// Counters of one shard of the asynchronous near queue, each on its own
-/// 128-byte line: `head` is advanced by the warps that claim slots, `tail`
-/// by the warps that reserve slots for new entries, `done` counts the
-/// reserved entries that are settled (expanded, skipped as stale, or moved to
-/// the far pile because the shard was full). A phase is over when every
-/// shard has done == tail.
+/// Positions of one shard of the asynchronous loop's spill queue: entries
+/// reserved by producers (high half) and claimed by consumers (low half), in
+/// one word, so that one load sees both and one compare-and-swap claims.
 struct alignas(128) AsyncShard {
-  unsigned head;
-  unsigned pad0[31];
-  unsigned tail;
-  unsigned pad1[31];
-  unsigned done;
-  unsigned pad2[31];
+  u64 claimed;  // reserved << 32 | claimed
+  unsigned pad[30];
 };
-constexpr int kAsyncShards = 32;  // shards of the near queue (one counter set)
+constexpr int kAsyncShards = 16;  // shards of the spill queue
+
+// Row records of the asynchronous loop: the first edges of a row, side by
+// side with their weights, in one 32-byte sector per objective and vertex.
+constexpr int kRecordEdges = 3;  // edges in the record of a row of more than four
+constexpr int kMoreEdges = -2;   // fourth head of such a record
+
+/// A far pile of the asynchronous loop holds a vertex at most this often:
+/// once as it leaves infinity or its valid tree distance, once more when an
+/// invalidated vertex passes its old distance, and once by overflow of the
+/// spill queue (flagged).
+constexpr int kFarCopies = 3;
+
+/// Whether a launch makes row records: graphs of at most 3.5 edges per
+/// vertex.
+__host__ __device__ inline bool recordsPay(long long n, long long m) { return 2 * m <= 7 * n; }
 
 // Phase boundaries recorded in EngineControl::phaseNs.
 enum : int {
@@ -180,13 +197,15 @@ struct EngineParams {
   int *nearV0, *nearV1;        // near lists: vertices
   u64 *nearD0, *nearD1;        // near lists: distance when appended
   long long stride, strideNear;
-  // asynchronous near queue (kFlagAsync): aqShards shards of aqShardCap
-  // slots, every slot ~0 (empty) between launches; two counter sets of
-  // aqShards shards (phase parity)
+  long long strideFar;         // far piles: objective k from k * strideFar
+  // spill queue of the asynchronous loop (kFlagAsync): aqShards shards of
+  // aqShardCap slots, every slot ~0 (empty) between launches
   u64 *aqSlots;
   AsyncShard *aqCtr;
   unsigned aqShardCap;
   int aqShards;
+  int4 *rec;                   // row records (two int4 per vertex; objective k from
+                               // 2 * k * stride) or null: the launch uses none
   int stageEntries;            // entries of the per-CTA append stage (dynamic shared memory)
   int heavyDeg;                // rows above this many edges: whole-CTA handling (0: 2,048)
   EngineControl *ctl;

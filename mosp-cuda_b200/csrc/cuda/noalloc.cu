@@ -166,6 +166,7 @@ extern "C" int mosp_sosp_from_scratch_static(int n, int m, const int *d_out_row,
   p.farL0 = ints + 4 * intStride;
   p.farL1 = ints + 5 * intStride;
   p.stride = kMaxVertices;
+  p.strideFar = kMaxVertices;  // (the bulk loop lists a vertex once)
   p.nearV0 = reinterpret_cast<int *>(b + kOffNearV0);
   p.nearV1 = reinterpret_cast<int *>(b + kOffNearV1);
   p.nearD0 = reinterpret_cast<u64 *>(b + kOffNearD0);

@@ -446,8 +446,8 @@ class Workspace:
         """Near-far loop of the last launch. Bulk loop: {split|push: (ms,
         iterations, items)} and the parts of a push iteration; asynchronous
         loop: its time and phases, the durations of the first four phases
-        (the rest summed), warp rounds and the entries taken from the queue
-        and from the warps' local buffers."""
+        (the rest summed), warp rounds and the entries taken from the spill
+        queue and from the CTAs' own rings and far-pile shares."""
         ns = (C.c_ulonglong * 7)()
         it = (C.c_longlong * 2)()
         items = (C.c_longlong * 2)()
@@ -533,7 +533,7 @@ class Workspace:
 
     def set_async(self, on=True, queue_slots=0):
         """Asynchronous near-far loop (default) or the bulk-synchronous one;
-        queue_slots bounds the asynchronous near queue (0: default size)."""
+        queue_slots bounds the asynchronous loop's spill queue (0: default size)."""
         check(lib().mosp_workspace_set_async(self._h, 1 if on else 0, int(queue_slots)))
 
     def set_canonical_trees(self, on=True):
