@@ -98,7 +98,7 @@ struct mosp_workspace {
   // combined graph
   long long combN = 0, combEdgesCap = 0;
   int *combDeg = nullptr, *combRow = nullptr, *combCol = nullptr, *combW = nullptr;
-  // reverse-CSR build cursor
+  // reverse-CSR build: in-degrees and edge ranks
   long long cursorCap = 0;
   int *cursor = nullptr;
   // path costs
@@ -138,6 +138,8 @@ struct mosp_workspace {
   long long recMarkCap = 0;
   u64 *recChunks = nullptr;  // two chunk lists of recChunkCap entries
   long long recChunkCap = 0;
+  int4 *recDist = nullptr;   // full recovery: interleaved 32-bit distances
+  long long recDistCap = 0;
   // CUDA graph of mosp_update_device's launch sequence (mosp_workspace_use_graphs)
   bool useGraphs = false;
   cudaStream_t captureStream = nullptr;
@@ -697,6 +699,15 @@ int prepareUpdate(mosp_workspace *ws, const UpdateArgs &a, EngineParams &p, int 
     p.recScanList = ws->recVerts + ws->recMarkCap;
     p.recChunkList = ws->recChunks;
     p.recChunkCap = static_cast<int>(ws->recChunkCap);
+  } else if (const long long fall = std::count(bitsOut, bitsOut + a.K, 0)) {
+    // the full recovery's distances side by side; without room for them it
+    // reads the objectives' own arrays
+    const long long need = static_cast<long long>(a.n) * (fall <= 4 ? 1 : (fall + 7) / 8 * 2);
+    if (need > ws->recDistCap) {
+      ws->recDistCap = 0;
+      if (deviceAlloc(&ws->recDist, need) == MOSP_OK) ws->recDistCap = need;
+    }
+    if (need <= ws->recDistCap) p.recDist = ws->recDist;
   }
   return MOSP_OK;
 }
@@ -836,7 +847,8 @@ void mosp_workspace_destroy(mosp_workspace *ws) {
                   static_cast<void *>(ws->edgeOf), static_cast<void *>(ws->anc0),
                   static_cast<void *>(ws->anc1), static_cast<void *>(ws->acc0),
                   static_cast<void *>(ws->acc1), static_cast<void *>(ws->recMark),
-                  static_cast<void *>(ws->recVerts), static_cast<void *>(ws->recChunks)}) {
+                  static_cast<void *>(ws->recVerts), static_cast<void *>(ws->recChunks),
+                  static_cast<void *>(ws->recDist)}) {
     if (p) cudaFree(p);
   }
   for (void *p : ws->user) {
@@ -1061,9 +1073,11 @@ int mosp_build_device_graph(mosp_workspace *ws, int n, int m, int K, const int *
                  d_in_col == nullptr || d_in_w == nullptr))) {
     return fail(MOSP_ERR_INVALID, "Error: invalid device graph arguments.");
   }
-  if (n + 1 > ws->cursorCap) {
-    if ((st = deviceAlloc(&ws->cursor, static_cast<size_t>(n) + 1)) != MOSP_OK) return st;
-    ws->cursorCap = static_cast<long long>(n) + 1;
+  if (static_cast<long long>(n) + 1 + m > ws->cursorCap) {
+    const long long need = static_cast<long long>(n) + 1 + m;
+    ws->cursorCap = 0;
+    if ((st = deviceAlloc(&ws->cursor, need)) != MOSP_OK) return st;
+    ws->cursorCap = need;
   }
   cudaStream_t s = asStream(stream);
   BuildParams b{};
@@ -1079,6 +1093,7 @@ int mosp_build_device_graph(mosp_workspace *ws, int n, int m, int K, const int *
   b.inCol = d_in_col;
   b.inW = d_in_w;
   b.cursor = ws->cursor;
+  b.rank = ws->cursor + n + 1;
   b.blockSums = ws->blockSums;
   b.ctl = ws->ctl + 2;
   MOSP_CUDA(cudaMemsetAsync(ws->ctl + 2, 0, sizeof(EngineControl), s));

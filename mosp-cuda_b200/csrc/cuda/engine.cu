@@ -2213,6 +2213,74 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
   return true;
 }
 
+// ---------------------------------------------------------------------------
+// Passes over all edges with their rows (device-graph fill, tree edges of the
+// path costs, parent recovery): warps take chunks of the edge array on
+// demand, find the row of a chunk's first edge by binary search and the rows
+// of 32 edges at a time by a shuffle search over row ends. Equal slices
+// per warp would leave half of the grid idle on power-law graphs: where rows
+// are short a slice takes several times as long.
+// ---------------------------------------------------------------------------
+struct EdgeChunks {
+  long long size, m, nwarps;
+  long long mine;  // the warp's first chunk; the others come off the counter
+  unsigned *next;  // zero at the start of the pass
+
+  /// About eight chunks per warp, of at least 256 edges (a chunk pays for a
+  /// binary search); fewer edges than that: one chunk per warp.
+  __device__ __forceinline__ EdgeChunks(long long edges, long long gwarp, long long warps, unsigned *counter)
+      : m(edges), nwarps(warps), mine(gwarp), next(counter) {
+    size = (m / (8 * nwarps) + 31) / 32 * 32;
+    if (size < 256) size = 256;
+    if (size > 4096) size = 4096;
+    if (size * nwarps > m) size = (m + 32 * nwarps - 1) / (32 * nwarps) * 32;
+  }
+  /// The warp's next chunk [wb, we) and the row of its first edge: false
+  /// when there is none. All lanes call it.
+  __device__ __forceinline__ bool take(const int *outRow, int n, long long &wb, long long &we, int &row) {
+    long long i = mine;
+    mine = -1;
+    if (i < 0) {
+      if (size * nwarps >= m) return false;
+      unsigned a = 0;
+      if (laneId() == 0) a = atomicAdd(next, 1u);
+      i = nwarps + __shfl_sync(kFull, a, 0);
+    }
+    wb = size * i;
+    we = wb + size < m ? wb + size : m;
+    if (wb >= we) return false;
+    row = 0;  // the last row that starts at or before wb
+    for (int hi = n; hi - row > 1;) {
+      const int mid = row + ((hi - row) >> 1);
+      if (__ldg(outRow + mid) <= wb) row = mid; else hi = mid;
+    }
+    return true;
+  }
+};
+
+/// The row of this lane's edge (`in`: it has one) of 32 consecutive edges, none
+/// of which lies in a row before r0; r0 moves on to the last one's. The
+/// window holding row n - 1 ends the search: rows past n count as ending at
+/// INT_MAX. All lanes call it.
+__device__ __forceinline__ int edgeRow(const int *outRow, int n, long long e, bool in, int &r0) {
+  int row = in ? -1 : r0;
+  for (int base = r0; base < n; base += 32) {
+    const int rr = base + static_cast<int>(laneId());
+    const int end = rr < n ? __ldg(outRow + rr + 1) : INT_MAX;
+    int at = 0;  // rows of the window that end at or before the edge
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+      if (__shfl_sync(kFull, end, at + step - 1) <= e) at += step;
+    }
+    // every lane takes part in the shuffles, found or not
+    const int lastEnd = __shfl_sync(kFull, end, 31);
+    if (row < 0 && e < lastEnd) row = base + at;
+    if (__all_sync(kFull, row >= 0)) break;
+  }
+  r0 = __shfl_sync(kFull, row, 31);  // the largest; past the chunk the caller ends
+  return row;
+}
+
 /// Lowest-id tight parent of every vertex of the distance-only objectives
 /// (parent INT_MAX after the unpack, -1 for roots and unreached vertices);
 /// thread tid of T.
@@ -2298,6 +2366,15 @@ __device__ void recoverTightParents(const EngineParams &P, const int *outRow, co
   }
 }
 
+/// The distance-only objectives of a launch, in order: their number.
+__device__ int fallbackObjectives(const EngineParams &P, int *which) {
+  int count = 0;
+  for (int k = 0; k < P.K; ++k) {
+    if (P.obj[k].parentBits == 0) which[count++] = k;
+  }
+  return count;
+}
+
 // ---------------------------------------------------------------------------
 // Unpack words into (distance, parent); distance-only objectives recover
 // the lowest-id tight parent (reference src/sospUpdateGpu.cu:478-512).
@@ -2368,6 +2445,8 @@ __device__ bool unpackResults(const EngineParams &P, const int *outRow,
           if (chg) changed[at + __popc(bal & ((1u << lane) - 1))] = static_cast<int>(v);
         }
       }
+    } else if (Mode == kModeUpdate && P.recDist != nullptr) {
+      anyFallback = true;  // below, all of them together
     } else {
       anyFallback = true;
       for (long long v = tid; v < n; v += T) {
@@ -2378,6 +2457,40 @@ __device__ bool unpackResults(const EngineParams &P, const int *outRow,
                           : INT_MAX;
       }
     }
+  }
+  if (Mode == kModeUpdate && anyFallback && !restricted && P.recDist != nullptr) {
+    // a vertex's distances side by side for recoverParents32
+    __shared__ int sFall[kMaxK];
+    __shared__ int sCount;
+    if (threadIdx.x == 0) sCount = fallbackObjectives(P, sFall);
+    __syncthreads();
+    const int count = sCount;
+    const int vec = count <= 4 ? 1 : 2;
+    bool wide = false;
+    for (int g0 = 0; g0 < count; g0 += 8) {
+      int4 *out = P.recDist + static_cast<long long>(g0 / 8) * 2 * n;
+      for (long long v = tid; v < n; v += T) {
+        const bool root = isRoot(P.source, P.sources, P.nSources, static_cast<int>(v));
+        unsigned d32[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          d32[j] = ~0u;
+          if (g0 + j >= count) continue;
+          const int k = sFall[g0 + j];
+          const ObjectiveArgs &O = P.obj[k];
+          const u64 word = __ldcg(P.packed + static_cast<long long>(k) * P.stride + v);
+          O.dist[v] = word == kInfWord ? kDistInf : static_cast<long long>(word);
+          O.parent[v] = word == kInfWord || root ? -1 : INT_MAX;
+          if (word != kInfWord) {
+            wide |= word >= (1ULL << 31);
+            d32[j] = static_cast<unsigned>(word);
+          }
+        }
+        out[vec * v] = make_int4(d32[0], d32[1], d32[2], d32[3]);
+        if (vec == 2) out[2 * v + 1] = make_int4(d32[4], d32[5], d32[6], d32[7]);
+      }
+    }
+    if (wide) P.ctl->recWide = 1;
   }
   if (!anyFallback || (P.flags & kFlagHostRecovery) != 0) return true;
   if (!gridSync(P.ctl, epoch)) return false;
@@ -3277,6 +3390,14 @@ __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBas
 // ---------------------------------------------------------------------------
 // Device graph: objective-major weights and the reverse CSR (reference
 // src/deviceGraph.cu:28-63, 87-135), one cooperative launch.
+//
+// Bound by the scattered traffic of the transposition: one returning atomic
+// per edge (its rank among the edges into its head, kept, so that the fill
+// needs no second atomic) and K + 1 scattered stores. Both passes are
+// balanced over edges. (With rows dealt to warps, the
+// one that held the low ids of an R-MAT graph walked most of its hubs: 3.9M
+// edges, K = 4: 4.13 -> 0.36 ms; 16.1M, K = 3: 11.2 -> 1.8 ms; road network
+// of 5.6M edges, K = 3: 0.24 -> 0.22 ms.)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant__ BuildParams B) {
   EngineControl *c = B.ctl;
@@ -3284,64 +3405,80 @@ __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant_
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long T = static_cast<long long>(gridDim.x) * blockDim.x;
   const unsigned lane = laneId();
-  const long long gwarp = tid >> 5, nwarps = T >> 5;
+  const long long nwarps = T >> 5;
   Sync epoch = startSync(B.timeoutNs);
 
-  // validate the CSR; split the weights; clear the degree counts
-  if (tid == 0 && (__ldg(B.outRow) != 0 || __ldg(B.outRow + n) != m)) c->invalid = 1;
-  for (long long v = tid; v < n; v += T) {
-    if (__ldg(B.outRow + v + 1) < __ldg(B.outRow + v)) c->invalid = 1;
+  // validate the row offsets; clear the degree counts
+  bool bad = tid == 0 && (__ldg(B.outRow) != 0 || __ldg(B.outRow + n) != m);
+  for (long long v = tid; v <= n; v += T) {
+    bad |= v < n && __ldg(B.outRow + v + 1) < __ldg(B.outRow + v);
+    B.cursor[v] = 0;
   }
-  for (long long e = tid; e < m; e += T) {
-    const int x = __ldg(B.outCol + e);
-    if (x < 0 || x >= n) c->invalid = 1;
+  if (bad) c->invalid = 1;
+  if (!gridSync(c, epoch)) return;
+
+  // validate the heads; count them, keeping each edge's rank; split the
+  // weights. Four edges per thread, so their atomics are in flight together.
+  bad = false;
+  for (long long e0 = tid; e0 < m; e0 += 4 * T) {
+    int x[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long e = e0 + q * T;
+      x[q] = e < m ? __ldg(B.outCol + e) : -1;
+      if (e < m && (x[q] < 0 || x[q] >= n)) {
+        bad = true;
+        x[q] = -1;
+      }
+    }
+    int r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) r[q] = x[q] >= 0 ? atomicAdd(B.cursor + x[q], 1) : 0;
+    for (int k = 0; k < K; ++k) {
+      int w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long e = e0 + q * T;
+        w[q] = e < m ? __ldg(B.edgeMajorW + e * K + k) : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long e = e0 + q * T;
+        if (e < m) B.outW[static_cast<long long>(k) * m + e] = w[q];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long e = e0 + q * T;
+      if (e < m) B.rank[e] = r[q];
+    }
   }
-  for (long long i = tid; i < static_cast<long long>(m) * K; i += T) {
-    const long long e = i / K;
-    const int k = static_cast<int>(i - e * K);
-    B.outW[static_cast<long long>(k) * m + e] = __ldg(B.edgeMajorW + i);
-  }
-  for (long long v = tid; v <= n; v += T) B.cursor[v] = 0;
+  if (bad) c->invalid = 1;
   if (!gridSync(c, epoch)) return;
   if (__ldcg(&c->invalid) != 0) return;
-
-  for (long long e = tid; e < m; e += T) atomicAdd(B.cursor + __ldg(B.outCol + e), 1);
-  if (!gridSync(c, epoch)) return;
   long long total = 0;
-  if (!gridExclusiveScan(B.cursor, B.inRow, B.cursor, static_cast<long long>(n) + 1,
-                         B.blockSums, c, epoch, &total)) {
+  if (!gridExclusiveScan(B.cursor, B.inRow, nullptr, static_cast<long long>(n) + 1, B.blockSums, c, epoch,
+                         &total)) {
     return;
   }
   if (!gridSync(c, epoch)) return;
 
-  // fill: one lane per short row, one warp per long row
-  for (long long base = gwarp * 32; base < n; base += nwarps * 32) {
-    const long long u = base + lane;
-    int beg = 0, end = 0;
-    if (u < n) {
-      beg = __ldg(B.outRow + u);
-      end = __ldg(B.outRow + u + 1);
-    }
-    const int deg = end - beg;
-    unsigned big = __ballot_sync(kFull, deg > kLaneRowMax);
-    auto place = [&](int uu, int e) {
-      const int pos = atomicAdd(B.cursor + __ldg(B.outCol + e), 1);
-      B.inCol[pos] = uu;
+  // fill: edge e of row u goes to position rank[e] of its head's row
+  EdgeChunks chunks(m, tid >> 5, nwarps, &c->chunkNext);
+  long long wb, we;
+  int r0;
+  while (chunks.take(B.outRow, n, wb, we, r0)) {
+    for (long long e0 = wb; e0 < we; e0 += 32) {
+      const long long e = e0 + lane;
+      const bool in = e < we;
+      const int x = in ? __ldg(B.outCol + e) : 0;
+      const int pos = in ? __ldcg(B.inRow + x) + __ldcg(B.rank + e) : 0;
+      const int row = edgeRow(B.outRow, n, e, in, r0);
+      if (!in) continue;
+      B.inCol[pos] = row;
       for (int k = 0; k < K; ++k) {
-        B.inW[static_cast<long long>(k) * m + pos] =
-            __ldg(B.edgeMajorW + static_cast<long long>(e) * K + k);
+        B.inW[static_cast<long long>(k) * m + pos] = __ldg(B.edgeMajorW + e * K + k);
       }
-    };
-    if (deg <= kLaneRowMax) {
-      for (int e = beg; e < end; ++e) place(static_cast<int>(u), e);
-    }
-    while (big != 0) {
-      const int src = __ffs(big) - 1;
-      big &= big - 1;
-      const int ub = static_cast<int>(__shfl_sync(kFull, u, src));
-      const int bb = __shfl_sync(kFull, beg, src);
-      const int eb = __shfl_sync(kFull, end, src);
-      for (int e = bb + static_cast<int>(lane); e < eb; e += 32) place(ub, e);
     }
   }
 }
@@ -3364,47 +3501,26 @@ __global__ void __launch_bounds__(kThreads, 1) pathCosts(const __grid_constant__
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long T = static_cast<long long>(gridDim.x) * blockDim.x;
   const unsigned lane = laneId();
-  const long long gwarp = tid >> 5, nwarps = T >> 5;
+  const long long nwarps = T >> 5;
   Sync epoch = startSync(C.timeoutNs);
 
   for (long long v = tid; v < n; v += T) C.edgeOf[v] = INT_MAX;
   if (!gridSync(c, epoch)) return;
-  // first occurrence of the tree edge (parent[v], v): lowest e in row p.
-  // Edge-balanced: warp w takes the w-th equal slice of the edge array and
-  // finds the row of each of its 32 edges from the ends of the next 32 rows
-  // (one coalesced load, a 5-step shuffle search), so hub rows are shared
-  // by many warps instead of walked by one.
+  // first occurrence of the tree edge (parent[v], v): lowest e in row p
   {
     const long long m = __ldg(C.outRow + n);
-    const long long wb = m * gwarp / nwarps, we = m * (gwarp + 1) / nwarps;
-    if (wb < we) {  // the same for the whole warp
-      int lo = 0, hi = n;  // the row of the slice's first edge: last r with row[r] <= wb
-      while (hi - lo > 1) {
-        const int mid = lo + ((hi - lo) >> 1);
-        if (__ldg(C.outRow + mid) <= wb) lo = mid; else hi = mid;
-      }
-      int r0 = lo;
+    EdgeChunks chunks(m, tid >> 5, nwarps, &c->chunkNext);
+    long long wb, we;
+    int r0;
+    while (chunks.take(C.outRow, n, wb, we, r0)) {
       for (long long e0 = wb; e0 < we; e0 += 32) {
         const bool valid = e0 + lane < we;
         const int e = static_cast<int>(e0 + lane);
         const int x = valid ? __ldg(C.outCol + e) : 0;
-        int row = valid ? -1 : 0;
-        for (int base = r0; base < n; base += 32) {
-          const int rr = base + static_cast<int>(lane);
-          const int end = rr < n ? __ldg(C.outRow + rr + 1) : INT_MAX;
-          int pos = 0;  // rows of the window that end at or before e
-#pragma unroll
-          for (int step = 16; step >= 1; step >>= 1) {
-            if (__shfl_sync(kFull, end, pos + step - 1) <= e) pos += step;
-          }
-          // every lane takes part in the shuffle, found or not
-          const int lastEnd = __shfl_sync(kFull, end, 31);
-          if (row < 0 && e < lastEnd) row = base + pos;
-          if (__all_sync(kFull, row >= 0)) break;
-        }
-        r0 = __shfl_sync(kFull, row, 31);  // the largest row; past the slice the loop ends
-        if (valid && row >= 0 && row < n && static_cast<unsigned>(x) < static_cast<unsigned>(n) &&
-            !isRoot(C.source, C.sources, C.nSources, x) && __ldg(C.parent + x) == row) {
+        const bool known = valid && static_cast<unsigned>(x) < static_cast<unsigned>(n);
+        const int p = known ? __ldg(C.parent + x) : -1;
+        const int row = edgeRow(C.outRow, n, e, valid, r0);
+        if (known && p == row && row >= 0 && !isRoot(C.source, C.sources, C.nSources, x)) {
           atomicMin(C.edgeOf + x, e);
         }
       }
@@ -3501,6 +3617,7 @@ __global__ void barrierCost(EngineControl *c, int rounds, int reads, long long t
 /// size for the graph reads.
 __global__ void __launch_bounds__(256) recoverParents(const __grid_constant__ EngineParams P) {
   __shared__ const int *sOutWk[kMaxK];
+  if (P.recDist != nullptr && __ldcg(&P.ctl->recWide) == 0) return;  // recoverParents32 did it
   if (threadIdx.x < kMaxK) {
     sOutWk[threadIdx.x] =
         static_cast<int>(threadIdx.x) < P.K ? P.obj[threadIdx.x].outW : nullptr;
@@ -3509,6 +3626,68 @@ __global__ void __launch_bounds__(256) recoverParents(const __grid_constant__ En
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long T = static_cast<long long>(gridDim.x) * blockDim.x;
   recoverTightParents<kModeUpdate>(P, P.outRow, P.outCol, sOutWk, tid, T);
+}
+
+/// The same recovery with the distances of up to 4 V objectives side by side
+/// in 32 bits (every finite one is below 2^31, so a sum with a weight is
+/// exact): edge (u, x) gathers one sector for x where the objectives' own
+/// arrays take one each, and warps take chunks on demand. Bound by the
+/// gathers (a wavefront of L1 per edge) and the streams of heads and weights,
+/// which are read past L2's lasting part to leave it to the distances: 65M
+/// edges of an R-MAT graph of scale 22, K = 5: 2.89 -> 1.07 ms (2.05 with
+/// equal slices).
+template <int V>
+__global__ void __launch_bounds__(256) recoverParents32(const __grid_constant__ EngineParams P) {
+  __shared__ int sFall[kMaxK];
+  __shared__ int sCount;
+  if (__ldcg(&P.ctl->recWide) != 0) return;
+  if (threadIdx.x == 0) sCount = fallbackObjectives(P, sFall);
+  __syncthreads();
+  const int n = P.n;
+  const unsigned lane = laneId();
+  const long long m = __ldg(P.outRow + n);
+  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  EdgeChunks chunks(m, tid >> 5, (static_cast<long long>(gridDim.x) * blockDim.x) >> 5, &P.ctl->chunkNext);
+  long long wb, we;
+  int first;
+  while (chunks.take(P.outRow, n, wb, we, first)) {
+    for (int g0 = 0; g0 < sCount; g0 += 4 * V) {
+      const int4 *dist = P.recDist + static_cast<long long>(g0 / 8) * 2 * n;
+      const int count = sCount - g0 < 4 * V ? sCount - g0 : 4 * V;
+      int r0 = first;
+      for (long long e0 = wb; e0 < we; e0 += 32) {
+        const long long e = e0 + lane;
+        const bool in = e < we;
+        const int x = in ? __ldcs(P.outCol + e) : 0;
+        int4 dx[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) dx[i] = __ldg(dist + static_cast<long long>(V) * x + i);
+        int w[4 * V];
+#pragma unroll
+        for (int j = 0; j < 4 * V; ++j) {
+          w[j] = in && j < count ? __ldcs(P.obj[sFall[g0 + j]].outW + e) : 0;
+        }
+        const int row = edgeRow(P.outRow, n, e, in, r0);
+        if (!in || row < 0) continue;
+        int4 du[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) du[i] = __ldg(dist + static_cast<long long>(V) * row + i);
+#pragma unroll
+        for (int j = 0; j < 4 * V; ++j) {
+          if (j >= count) break;
+          const int4 a = du[j / 4], b = dx[j / 4];
+          const unsigned from =
+              static_cast<unsigned>(j % 4 == 0 ? a.x : j % 4 == 1 ? a.y : j % 4 == 2 ? a.z : a.w);
+          const unsigned to =
+              static_cast<unsigned>(j % 4 == 0 ? b.x : j % 4 == 1 ? b.y : j % 4 == 2 ? b.z : b.w);
+          // (roots hold parent -1, which no id lowers; ~0 is no sum)
+          if (from != ~0u && from + static_cast<unsigned>(w[j]) == to) {
+            atomicMin(P.obj[sFall[g0 + j]].parent + x, row);
+          }
+        }
+      }
+    }
+  }
 }
 
 template <typename Kernel>
@@ -3576,6 +3755,16 @@ cudaError_t launchRecovery(const EngineParams &p, cudaStream_t s) {
   if (err != cudaSuccess) return err;
   if ((p.flags & kFlagCanonical) != 0 && p.recMark != nullptr) {
     return launchRestrictedRecovery(p, sms, s);
+  }
+  if (p.recDist != nullptr) {
+    int count = 0;
+    for (int k = 0; k < p.K; ++k) count += p.obj[k].parentBits == 0;
+    if (count <= 4) {
+      recoverParents32<1><<<sms * 8, 256, 0, s>>>(p);
+    } else {
+      recoverParents32<2><<<sms * 8, 256, 0, s>>>(p);
+    }
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
   }
   recoverParents<<<sms * 8, 256, 0, s>>>(p);
   return cudaGetLastError();

@@ -111,6 +111,8 @@ struct alignas(128) EngineControl {
   int recChanged[kMaxK];
   int recScan[kMaxK];
   int recChunks[2];
+  int recWide;        // full parent recovery: a distance of 2^31 or more (recDist is not used)
+  unsigned chunkNext; // next chunk of a pass over all edges (at most one per launch)
 };
 
 // EngineParams::flags (tuning switches; results do not depend on them)
@@ -227,6 +229,11 @@ struct EngineParams {
   int *recScanList;
   u64 *recChunkList;
   int recChunkCap;
+  // full parent recovery: the distances of the distance-only objectives side
+  // by side in 32 bits (~0: unreached), written by the unpack, or null. Up to
+  // four of them: one int4 per vertex; else groups of eight, two int4 per
+  // vertex and group, group g from g * 2 * n
+  int4 *recDist;
   ObjectiveArgs obj[kMaxK];
 };
 static_assert(sizeof(EngineParams) <= 4096, "kernel parameter block limit");
@@ -244,7 +251,8 @@ struct BuildParams {
   long long timeoutNs;
   const int *outRow, *outCol, *edgeMajorW;
   int *outW, *inRow, *inCol, *inW;
-  int *cursor;
+  int *cursor;  // in-degrees [n + 1]
+  int *rank;    // edge e among the edges into its head [m]
   long long *blockSums;
   EngineControl *ctl;
 };
