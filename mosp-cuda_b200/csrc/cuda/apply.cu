@@ -583,7 +583,10 @@ Layout layoutFor(unsigned char *base, long long n, long long m, long long B) {
   L.flags = carve<int>(p, B + 1);
   L.pos = carve<int>(p, B + 1);
   L.hist = carve<int>(p, 256 * tiles + 1);
-  const long long longest = 256 * tiles + 1 > n + 1 ? 256 * tiles + 1 : n + 1;
+  // one entry per chunk of the longest scan: a radix histogram, the rows or
+  // the batch
+  long long longest = 256 * tiles + 1 > n + 1 ? 256 * tiles + 1 : n + 1;
+  if (B + 1 > longest) longest = B + 1;
   L.aux = carve<int>(p, (longest + kScanChunk - 1) / kScanChunk + 1);
   L.rowHead = carve<int>(p, B + 1);
   L.rowPos = carve<int>(p, B + 1);
