@@ -1,5 +1,6 @@
 // apply.cu - Step 1 on the GPU: apply a change batch to a device CSR graph
 // (the semantics of applyChangeBatch, reference src/csrGraph.cu:727-894).
+// Batches of up to kFusedBatch changes take applyFused.cu instead.
 //
 // Semantics, per source row u (the host restatement is applyBatchView in
 // csrc/host/csrGraph.cpp):

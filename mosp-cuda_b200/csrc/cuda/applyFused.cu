@@ -1,0 +1,601 @@
+// applyFused.cu - Step 1 on the GPU in one cooperative launch, for batches of
+// up to kFusedBatch changes (larger ones: the sorted form in apply.cu, which
+// states the semantics both follow).
+//
+// The sorted form pays for its launches: two radix sorts and half a dozen
+// scans are some 75 launches and four read-backs. Here the changes of a (u,v)
+// group meet in a hash table instead of a sort, and every per-group quantity
+// of the rules does not depend on the order in which they arrive:
+//   deletions and insertions of the group: counts;
+//   its first and last insertion: minimum and maximum of file positions;
+//   occurrences of v in row u and the first one: count and minimum over the
+//   row's edges.
+// Order matters in two places. The place of a live edge is its old one less
+// the removed edges of its row before it: a ballot over the 32 edges a warp
+// copies, carried along the row. The place of an appended edge is the number
+// of appended groups of its row with an earlier first insertion, counted over
+// the row's own list, which costs the square of the insertions into one row:
+// with all of a batch of 65,536 in one row 1.9 ms (sorted form 10.6), of
+// 262,144 14 ms (24). That sets kFusedBatch.
+//
+// The copy is one pass over all edges in chunks on demand: a warp takes 32
+// edges, finds their rows by a shuffle search and moves their heads and their
+// 32 K weights as one consecutive range each, so loads and stores coalesce
+// whatever K is; the weight statistics are taken from the same loads. Bound
+// by HBM: the graph read and written once.
+//
+// Measured on a B200, sorted form and this one: 50,000 changes on a road
+// network of 5.56M edges, K = 3 (178 MB read and written): 578 -> 223 us;
+// 24 changes on 4,200 edges: 307 -> 78 us; 20,000 on an R-MAT graph of 3.9M
+// edges, K = 4: 2112 -> 235 us; 60,000 on one of 65M, K = 5: 12.8 -> 2.2 ms.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "device.h"
+
+namespace mospb200 {
+namespace {
+
+constexpr u64 kNoKey = ~0ULL;
+constexpr int kLaneRow = 16;  // touched rows of at most so many edges are searched by one lane,
+constexpr int kPiece = 64;    // longer ones in pieces of so many by a warp each
+constexpr int kCopyThreads = 256;
+constexpr int kEarly = 4;     // turns of the copy whose weights are loaded ahead
+
+struct FusedScratch {
+  // groups: a hash table of `slots` (a power of two, at least twice the batch)
+  u64 *key;  // u << 32 | v
+  int *cD, *cI, *firstIns, *lastIns, *occ, *first;
+  unsigned *bits;
+  unsigned slots;
+  unsigned *filter;  // filterBits bits, 16 or more per group, set where a group hashes
+  unsigned filterBits;
+  int *entrySlot;  // slot of batch entry j (deletions first)
+  // touched rows, in no order
+  int *rows, *nApp, *nDead, *segApp, *segDead, *curApp, *curDead;
+  u64 *pieces;     // of the longer touched rows: vertex << 32 | piece
+  unsigned *hit;   // one bit per edge: it belongs to a group
+  int *app;        // insertions that append, by row segment
+  int *dead;       // removed edges, by row segment
+  // per vertex: touched row + 1 (0: none), and its change of degree
+  int *rowSlot, *delta;
+  int *counts;     // touched rows, pieces, appended, removed
+  long long *blockSums;
+  FusedResult *result;
+};
+
+__device__ __forceinline__ unsigned hashOf(u64 key) {
+  key ^= key >> 33;
+  key *= 0xff51afd7ed558ccdULL;
+  key ^= key >> 33;
+  key *= 0xc4ceb9fe1a85ec53ULL;
+  key ^= key >> 33;
+  return static_cast<unsigned>(key);
+}
+
+/// The filter bit of a key with this hash.
+__device__ __forceinline__ unsigned filterBit(const FusedScratch &S, unsigned hash) {
+  return (hash >> 9) & (S.filterBits - 1);
+}
+
+/// The group of edge (u, v), or -1. (At most half of the slots are taken, so
+/// the probe ends.)
+__device__ __forceinline__ int findGroup(const FusedScratch &S, int u, int v) {
+  const u64 key = (static_cast<u64>(static_cast<unsigned>(u)) << 32) | static_cast<unsigned>(v);
+  unsigned s = hashOf(key) & (S.slots - 1);
+  while (true) {
+    const u64 at = __ldcg(S.key + s);
+    if (at == key) return static_cast<int>(s);
+    if (at == kNoKey) return -1;
+    s = (s + 1) & (S.slots - 1);
+  }
+}
+
+/// Edges b, b + step, ... (< end) of touched row u: occurrences of their
+/// groups. Four at a time, their loads and probes in flight together.
+__device__ __forceinline__ void countOccurrences(const ApplyParams &P, const FusedScratch &S, int u, int b,
+                                                 int end, int step) {
+  for (int e0 = b; e0 < end; e0 += 4 * step) {
+    u64 key[4], at[4];
+    unsigned s[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = e0 + q * step;
+      key[q] = (static_cast<u64>(static_cast<unsigned>(u)) << 32) |
+               static_cast<unsigned>(e < end ? __ldg(P.col + e) : -1);
+      s[q] = hashOf(key[q]);
+    }
+    // most edges of a touched row are in no group: the filter says so from L1
+    // (a plain load: nothing writes it after the barrier before this phase)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned f = filterBit(S, s[q]);
+      at[q] = e0 + q * step < end && ((S.filter[f >> 5] >> (f & 31u)) & 1u) ? 0 : kNoKey;
+      s[q] &= S.slots - 1;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (at[q] == 0) at[q] = __ldcg(S.key + s[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      while (at[q] != key[q] && at[q] != kNoKey) {
+        s[q] = (s[q] + 1) & (S.slots - 1);
+        at[q] = __ldcg(S.key + s[q]);
+      }
+      if (at[q] == kNoKey) continue;
+      const int e = e0 + q * step;
+      atomicAdd(S.occ + s[q], 1);
+      atomicMin(S.first + s[q], e);
+      atomicOr(S.hit + (e >> 5), 1u << (e & 31));
+    }
+  }
+}
+
+/// Sum of x over the lanes before this one; the warp's sum in `total`.
+__device__ __forceinline__ int warpExclusive(int x, int &total) {
+  int incl = x;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(kFull, incl, off);
+    if (static_cast<int>(laneId()) >= off) incl += o;
+  }
+  total = __shfl_sync(kFull, incl, 31);
+  return incl - x;
+}
+
+/// Room for x entries per lane behind one counter, one atomic for the warp.
+/// All lanes call it.
+__device__ __forceinline__ int warpReserve(int *counter, int x) {
+  int total;
+  const int before = warpExclusive(x, total);
+  int base = 0;
+  if (laneId() == 0 && total > 0) base = atomicAdd(counter, total);
+  return __shfl_sync(kFull, base, 0) + before;
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedScratch S, EngineControl *c,
+           long long timeoutNs) {
+  const int n = static_cast<int>(P.n), m = static_cast<int>(P.m), K = P.K;
+  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const long long T = static_cast<long long>(gridDim.x) * blockDim.x;
+  const unsigned lane = laneId();
+  const int B = P.nDel + P.nIns;
+  Sync epoch = startSync(timeoutNs);
+
+  // ---- clear ---------------------------------------------------------------
+  for (long long v = tid; v < n + 4; v += T) {
+    S.rowSlot[v] = 0;
+    S.delta[v] = 0;
+  }
+  for (long long s = tid; s < S.slots; s += T) {
+    S.key[s] = kNoKey;
+    S.cD[s] = S.cI[s] = S.occ[s] = 0;
+    S.firstIns[s] = S.first[s] = INT_MAX;
+    S.lastIns[s] = -1;
+    S.bits[s] = 0;
+  }
+  for (long long i = tid; i < (m + 31LL) / 32; i += T) S.hit[i] = 0;
+  for (long long i = tid; i < S.filterBits / 32; i += T) S.filter[i] = 0;
+  for (long long r = tid; r < B; r += T) S.nApp[r] = S.nDead[r] = S.curApp[r] = S.curDead[r] = 0;
+  if (tid < 4) S.counts[tid] = 0;
+  if (tid < kMaxK) {
+    S.result->maxWeight[tid] = 1;
+    S.result->weightSum[tid] = 0;
+  }
+  if (!gridSync(c, epoch)) return;
+
+  // ---- groups and touched rows ---------------------------------------------
+  for (long long j0 = tid - lane; j0 < B; j0 += T) {  // the same j0 in the whole warp
+    const long long j = j0 + lane;
+    const bool del = j < P.nDel;
+    const int i = static_cast<int>(del ? j : j - P.nDel);
+    int u = -1, v = -1;
+    if (j < B) {
+      u = del ? P.delFrom[i] : P.insFrom[i];
+      v = del ? P.delTo[i] : P.insTo[i];
+      if (u < 0 || u >= n || v < 0 || v >= n) {
+        c->invalid = 1;
+        u = -1;
+      }
+    }
+    bool newRow = false;
+    if (u >= 0) {
+      const u64 key = (static_cast<u64>(static_cast<unsigned>(u)) << 32) | static_cast<unsigned>(v);
+      const unsigned hash = hashOf(key), f = filterBit(S, hash);
+      atomicOr(S.filter + (f >> 5), 1u << (f & 31u));
+      unsigned s = hash & (S.slots - 1);
+      while (true) {
+        const u64 old = atomicCAS(S.key + s, kNoKey, key);
+        if (old == kNoKey || old == key) break;
+        s = (s + 1) & (S.slots - 1);
+      }
+      S.entrySlot[j] = static_cast<int>(s);
+      if (del) {
+        atomicAdd(S.cD + s, 1);
+      } else {
+        atomicAdd(S.cI + s, 1);
+        atomicMin(S.firstIns + s, i);
+        atomicMax(S.lastIns + s, i);
+      }
+      newRow = atomicCAS(S.rowSlot + u, 0, -1) == 0;
+    }
+    const int r = warpReserve(S.counts + 0, newRow ? 1 : 0);
+    const int deg = newRow ? __ldg(P.row + u + 1) - __ldg(P.row + u) : 0;
+    const int mine = deg > kLaneRow ? (deg + kPiece - 1) / kPiece : 0;
+    const int at = warpReserve(S.counts + 1, mine);
+    if (newRow) {
+      S.rows[r] = u;
+      S.rowSlot[u] = r + 1;
+      for (int p = 0; p < mine; ++p) S.pieces[at + p] = (static_cast<u64>(u) << 32) | static_cast<unsigned>(p);
+    }
+  }
+  if (!gridSync(c, epoch)) return;
+  if (__ldcg(&c->invalid) != 0) return;
+
+  // ---- occurrences: a lane per short touched row (a lane of every warp
+  // before a second one of any), a warp per piece of a longer one
+  const int R = __ldcg(S.counts + 0);
+  const long long warps = T >> 5;
+  for (long long r = (tid >> 5) + lane * warps; r < R; r += T) {
+    const int u = __ldcg(S.rows + r);
+    const int b = __ldg(P.row + u), end = __ldg(P.row + u + 1);
+    if (end - b <= kLaneRow) countOccurrences(P, S, u, b, end, 1);
+  }
+  const int pieces = __ldcg(S.counts + 1);
+  for (long long i = tid >> 5; i < pieces; i += warps) {
+    const u64 piece = __ldcg(S.pieces + i);
+    const int u = static_cast<int>(piece >> 32);
+    const int b = __ldg(P.row + u) + static_cast<int>(piece) * kPiece;
+    const int end = __ldg(P.row + u + 1);
+    countOccurrences(P, S, u, b + static_cast<int>(lane), end < b + kPiece ? end : b + kPiece, 32);
+  }
+  if (!gridSync(c, epoch)) return;
+
+  // ---- groups resolved: degrees, list sizes, weight-increase masks ---------
+  for (long long s = tid; s < S.slots; s += T) {
+    const u64 key = __ldcg(S.key + s);
+    if (key == kNoKey) continue;
+    const int u = static_cast<int>(key >> 32);
+    const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s), cI = __ldcg(S.cI + s);
+    const int removed = occ < cD ? occ : cD;
+    const int appended = occ <= cD && cI > 0 ? 1 : 0;
+    const int r = __ldcg(S.rowSlot + u) - 1;
+    if (appended) atomicAdd(S.nApp + r, 1);
+    if (removed > 0) atomicAdd(S.nDead + r, removed);
+    if (appended != removed) atomicAdd(S.delta + u, appended - removed);
+    if (cI > 0 && occ > 0) {
+      const int *wn = P.insW + static_cast<long long>(__ldcg(S.lastIns + s)) * K;
+      const int *wo = P.w + static_cast<long long>(__ldcg(S.first + s)) * K;
+      unsigned bits = 0;
+      for (int k = 0; k < K; ++k) bits |= (wn[k] > wo[k] ? 1u : 0u) << k;
+      S.bits[s] = bits;
+    }
+  }
+  if (!gridSync(c, epoch)) return;
+
+  // ---- row segments of the lists; masks; sums of the degree changes --------
+  for (long long q0 = tid - lane; q0 < R; q0 += T) {
+    const long long r = q0 + lane;
+    const int a = warpReserve(S.counts + 2, r < R ? __ldcg(S.nApp + r) : 0);
+    const int d = warpReserve(S.counts + 3, r < R ? __ldcg(S.nDead + r) : 0);
+    if (r < R) {
+      S.segApp[r] = a;
+      S.segDead[r] = d;
+    }
+  }
+  for (long long i = tid; i < P.nIns; i += T) P.mask[i] = __ldcg(S.bits + S.entrySlot[P.nDel + i]);
+  // (a CTA's range in whole groups of four vertices)
+  const long long per = ((static_cast<long long>(n) + gridDim.x - 1) / gridDim.x + 3) / 4 * 4;
+  const long long lo = per * blockIdx.x < n ? per * blockIdx.x : n;
+  const long long hi = lo + per < n ? lo + per : n;
+  {
+    long long local = 0;
+    for (long long v = lo + 4LL * threadIdx.x; v < hi; v += 4LL * blockDim.x) {
+      const int4 d = __ldcg(reinterpret_cast<const int4 *>(S.delta + v));  // (zeros past n)
+      local += d.x + d.y + d.z + d.w;
+    }
+    const long long sum = blockSum(local);
+    if (threadIdx.x == 0) S.blockSums[blockIdx.x] = sum;
+  }
+  if (!gridSync(c, epoch)) return;
+
+  // ---- lists; new row offsets ----------------------------------------------
+  for (long long s = tid; s < S.slots; s += T) {
+    const u64 key = __ldcg(S.key + s);
+    if (key == kNoKey) continue;
+    const int u = static_cast<int>(key >> 32), v = static_cast<int>(key);
+    const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s);
+    const int r = __ldcg(S.rowSlot + u) - 1;
+    if (occ <= cD && __ldcg(S.cI + s) > 0) {
+      S.app[__ldcg(S.segApp + r) + atomicAdd(S.curApp + r, 1)] = __ldcg(S.firstIns + s);
+    }
+    // the first min(occ, cD) occurrences go
+    int left = occ < cD ? occ : cD;
+    for (int e = __ldcg(S.first + s); left > 0; ++e) {
+      if (__ldg(P.col + e) != v) continue;
+      S.dead[__ldcg(S.segDead + r) + atomicAdd(S.curDead + r, 1)] = e;
+      --left;
+    }
+  }
+  {
+    long long before = 0, all = 0;
+    for (int b = threadIdx.x; b < static_cast<int>(gridDim.x); b += blockDim.x) {
+      const long long x = __ldcg(S.blockSums + b);
+      all += x;
+      if (b < static_cast<int>(blockIdx.x)) before += x;
+    }
+    long long carry = blockSum(before);
+    all = blockSum(all);
+    for (long long t = lo; t < hi; t += 4LL * blockDim.x) {
+      const long long v = t + 4LL * threadIdx.x;
+      int4 d = make_int4(0, 0, 0, 0);
+      if (v < hi) d = __ldcg(reinterpret_cast<const int4 *>(S.delta + v));
+      const long long x = d.x + d.y + d.z + d.w;
+      long long tile;
+      long long run = carry + blockInclusiveScan(x, &tile) - x;
+      const int step[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (v + q < hi) P.newRow[v + q] = static_cast<int>(__ldg(P.row + v + q) + run);
+        run += step[q];
+      }
+      carry += tile;
+    }
+    if (tid == 0) {
+      P.newRow[n] = static_cast<int>(m + all);
+      S.result->newM = static_cast<int>(m + all);
+    }
+  }
+}
+
+/// edgeRow that also gives the row's start and how far the row moves: the
+/// window loads the offsets of its rows in both graphs, so the search and
+/// what the copy needs of the row are one round trip.
+__device__ __forceinline__ int edgeRowMove(const int *row, const int *newRow, int n, long long e, bool in,
+                                           int &r0, int &start, int &shift) {
+  int found = in ? -1 : r0;
+  for (int base = r0; base < n; base += 32) {
+    const int rr = base + static_cast<int>(laneId());
+    const int a = rr < n ? __ldg(row + rr) : 0;
+    const int moved = rr < n ? __ldcg(newRow + rr) - a : 0;
+    const int end = rr < n ? __ldg(row + rr + 1) : INT_MAX;
+    int at = 0;  // rows of the window that end at or before the edge
+#pragma unroll
+    for (int step = 16; step >= 1; step >>= 1) {
+      if (__shfl_sync(kFull, end, at + step - 1) <= e) at += step;
+    }
+    const int lastEnd = __shfl_sync(kFull, end, 31);
+    const int src = at < 32 ? at : 31;
+    const int st = __shfl_sync(kFull, a, src), mv = __shfl_sync(kFull, moved, src);
+    if (found < 0 && e < lastEnd) {
+      found = base + at;
+      start = st;
+      shift = mv;
+    }
+    if (__all_sync(kFull, found >= 0)) break;
+  }
+  r0 = __shfl_sync(kFull, found, 31);  // the largest; past the chunk the caller ends
+  return found;
+}
+
+/// The copy: every edge to its new place, appended edges behind their rows.
+/// A launch of its own, with half again as many warps as the persistent one
+/// can hold: it waits for memory.
+__global__ void __launch_bounds__(kCopyThreads, 5)
+copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedScratch S, EngineControl *c,
+          int stats) {
+  __shared__ unsigned long long sSum[kMaxK];
+  __shared__ int sMax[kMaxK];
+  if (__ldcg(&c->status) != 0 || __ldcg(&c->invalid) != 0) return;
+  const int n = static_cast<int>(P.n), m = static_cast<int>(P.m), K = P.K;
+  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const long long T = static_cast<long long>(gridDim.x) * blockDim.x;
+  const unsigned lane = laneId();
+  if (threadIdx.x < kMaxK) {
+    sSum[threadIdx.x] = 0;
+    sMax[threadIdx.x] = 1;
+  }
+  __syncthreads();
+  // Lanes 0 .. span - 1 (a multiple of K) move the weights, so a lane always
+  // holds the same objective and its statistics stay in two registers.
+  const int span = 32 / K * K;
+  const int myK = static_cast<int>(lane) % K;
+  long long sum = 0;
+  int most = 1;
+  EdgeChunks chunks(m, tid >> 5, T >> 5, &c->chunkNext);
+  long long wb, we;
+  int r0;
+  while (chunks.take(P.row, n, wb, we, r0)) {
+    // removed edges of the current row before the current 32
+    int carry = 0;
+    {
+      const int r = __ldcg(S.rowSlot + r0) - 1;
+      const int d = r >= 0 && __ldg(P.row + r0) < wb ? __ldcg(S.nDead + r) : 0;
+      const int *list = S.dead + (d > 0 ? __ldcg(S.segDead + r) : 0);
+      for (int i = static_cast<int>(lane); i < d; i += 32) carry += __ldcg(list + i) < wb;
+      carry = __reduce_add_sync(kFull, carry);
+    }
+    for (long long e0 = wb; e0 < we; e0 += 32) {
+      const int e = static_cast<int>(e0 + lane);
+      const bool in = e0 + lane < we;
+      const int col = in ? __ldg(P.col + e) : 0;
+      // (chunks start at multiples of 32)
+      const unsigned hits = __ldcg(S.hit + (e0 >> 5));
+      // the first turns' weights are requested before the rows are searched
+      const int edges = static_cast<int>(we - e0 < 32 ? we - e0 : 32);
+      const int *src = P.w + e0 * K;
+      int early[kEarly];
+#pragma unroll
+      for (int q = 0; q < kEarly; ++q) {
+        const int i = q * span + static_cast<int>(lane);
+        early[q] = static_cast<int>(lane) < span && i < edges * K ? __ldg(src + i) : 0;
+      }
+      int start = 0, moved = 0;
+      const int u = edgeRowMove(P.row, P.newRow, n, e, in, r0, start, moved);
+      bool live = in;
+      int other = -1;      // the insertion whose weights the edge takes
+      if (in && ((hits >> lane) & 1u)) {
+        const int g = findGroup(S, u, col);
+        const int cD = __ldcg(S.cD + g);
+        int before = 0;    // occurrences before this one
+        for (int x = __ldcg(S.first + g); x < e; ++x) before += __ldg(P.col + x) == col;
+        live = before >= cD;
+        if (before == cD && __ldcg(S.cI + g) > 0) other = __ldcg(S.lastIns + g);
+      }
+      const unsigned dead = __ballot_sync(kFull, in && !live);
+      const int from = start > e0 ? static_cast<int>(start - e0) : 0;  // the row's first lane
+      const unsigned mine = ((1u << lane) - 1u) & ~((1u << from) - 1u);
+      const int less = (start < e0 ? carry : 0) + __popc(dead & mine);
+      // new position, or -1
+      const int to = live ? e + moved - less : -1;
+      carry = __shfl_sync(kFull, less + (in && !live ? 1 : 0), 31);
+      if (to >= 0) P.newCol[to] = col;
+      const long long shift = static_cast<long long>(to - e) * K;
+      const bool plain = to >= 0 && other < 0;
+      auto move = [&](int base, int w) {  // all lanes call it
+        const int i = base + static_cast<int>(lane);
+        const bool has = static_cast<int>(lane) < span && i < edges * K;
+        const int owner = has ? i / K : 0;
+        const long long sh = __shfl_sync(kFull, shift, owner);
+        const int ok = __shfl_sync(kFull, static_cast<int>(plain), owner);
+        if (!has) return;
+        sum += w;
+        most = w > most ? w : most;
+        if (ok) P.newW[e0 * K + i + sh] = w;
+      };
+#pragma unroll
+      for (int q = 0; q < kEarly; ++q) {
+        if (q * span < edges * K) move(q * span, early[q]);
+      }
+      for (int base = kEarly * span; base < edges * K; base += span) {
+        const int i = base + static_cast<int>(lane);
+        move(base, static_cast<int>(lane) < span && i < edges * K ? __ldg(src + i) : 0);
+      }
+      if (to >= 0 && other >= 0) {
+        for (int k = 0; k < K; ++k) {
+          P.newW[static_cast<long long>(to) * K + k] = __ldg(P.insW + static_cast<long long>(other) * K + k);
+        }
+      }
+    }
+  }
+  // appended edges, at the end of their row in the order of their groups'
+  // first insertions
+  const int appended = __ldcg(S.counts + 2);
+  for (long long a = tid; a < appended; a += T) {
+    const int i = __ldcg(S.app + a);
+    const int u = __ldg(P.insFrom + i);
+    const int r = __ldcg(S.rowSlot + u) - 1;
+    const int count = __ldcg(S.nApp + r);
+    const int *list = S.app + __ldcg(S.segApp + r);
+    int rank = 0;
+    for (int x = 0; x < count; ++x) rank += __ldcg(list + x) < i;
+    const int to = __ldcg(P.newRow + u + 1) - count + rank;
+    P.newCol[to] = __ldg(P.insTo + i);
+    const long long last = __ldcg(S.lastIns + S.entrySlot[P.nDel + i]);
+    for (int k = 0; k < K; ++k) P.newW[static_cast<long long>(to) * K + k] = __ldg(P.insW + last * K + k);
+  }
+  if (!stats) return;
+  // the largest weight covers the insertions too
+  if (static_cast<int>(lane) < span) {
+    const long long all = static_cast<long long>(P.nIns) * K;
+    const long long warps = T >> 5;
+    for (long long i = (tid >> 5) * span + lane; i < all; i += warps * span) {
+      const int w = __ldg(P.insW + i);
+      most = w > most ? w : most;
+    }
+    atomicAdd(&sSum[myK], static_cast<unsigned long long>(sum));
+    atomicMax(&sMax[myK], most);
+  }
+  __syncthreads();
+  if (threadIdx.x < K) {
+    atomicAdd(reinterpret_cast<unsigned long long *>(&S.result->weightSum[threadIdx.x]), sSum[threadIdx.x]);
+    atomicMax(&S.result->maxWeight[threadIdx.x], static_cast<long long>(sMax[threadIdx.x]));
+  }
+}
+
+unsigned slotsFor(long long B) {
+  unsigned s = 64;
+  while (s < 2 * B) s *= 2;
+  return s;
+}
+
+template <typename X>
+X *carve(unsigned char *&p, long long count) {
+  X *r = reinterpret_cast<X *>(p);
+  p += (static_cast<long long>(sizeof(X)) * (count > 0 ? count : 1) + 255) / 256 * 256;
+  return r;
+}
+
+unsigned char *layout(unsigned char *p, long long n, long long m, long long nIns, long long nDel,
+                      FusedScratch &S) {
+  const long long B = nIns + nDel;
+  S.slots = slotsFor(B);
+  S.result = carve<FusedResult>(p, 1);
+  S.counts = carve<int>(p, 4);
+  S.key = carve<u64>(p, S.slots);
+  for (int **x : {&S.cD, &S.cI, &S.firstIns, &S.lastIns, &S.occ, &S.first}) *x = carve<int>(p, S.slots);
+  S.bits = carve<unsigned>(p, S.slots);
+  S.filterBits = std::min(8 * S.slots, 1u << 20);
+  S.filter = carve<unsigned>(p, S.filterBits / 32);
+  for (int **x : {&S.entrySlot, &S.rows, &S.nApp, &S.nDead, &S.segApp, &S.segDead, &S.curApp, &S.curDead}) {
+    *x = carve<int>(p, B);
+  }
+  S.pieces = carve<u64>(p, m / kPiece + B);
+  S.hit = carve<unsigned>(p, (m + 31) / 32);
+  S.app = carve<int>(p, nIns);
+  S.dead = carve<int>(p, nDel);
+  S.rowSlot = carve<int>(p, n + 4);
+  S.delta = carve<int>(p, n + 4);
+  return p;
+}
+
+}  // namespace
+
+size_t applyFusedBytes(long long n, long long m, long long nIns, long long nDel) {
+  FusedScratch S;
+  unsigned char *base = reinterpret_cast<unsigned char *>(static_cast<uintptr_t>(256));
+  return static_cast<size_t>(layout(base, n, m, nIns, nDel, S) - base) + 256;
+}
+
+cudaError_t applyFusedShape(int sms, int ctasPerSm, int &ctas) {
+  int perSm = 0;
+  cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, applyFused, kThreads, 0);
+  if (err != cudaSuccess) return err;
+  if (perSm < 1) return cudaErrorInvalidConfiguration;
+  if (ctasPerSm > 0 && ctasPerSm < perSm) perSm = ctasPerSm;
+  ctas = perSm * sms;
+  return cudaSuccess;
+}
+
+cudaError_t applyBatchFused(const ApplyParams &P, void *scratch, EngineControl *ctl, long long *blockSums,
+                            long long timeoutNs, int ctas, bool stats, FusedResult *pinned,
+                            EngineControl *pinnedCtl, cudaStream_t s) {
+  FusedScratch S;
+  layout(static_cast<unsigned char *>(scratch), P.n, P.m, P.nIns, P.nDel, S);
+  S.blockSums = blockSums;
+  ApplyParams p = P;
+  cudaError_t err = cudaMemsetAsync(ctl, 0, sizeof(EngineControl), s);
+  if (err != cudaSuccess) return err;
+  void *args[] = {&p, &S, &ctl, &timeoutNs};
+  err = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(applyFused), dim3(ctas), dim3(kThreads), args,
+                                    0, s);
+  if (err == cudaSuccess) {
+    const long long want = (std::max(P.m, static_cast<long long>(P.nIns)) + kCopyThreads - 1) / kCopyThreads;
+    const int grid = static_cast<int>(std::min(std::max(want, 1LL), 5LL * ctas));
+    copyFused<<<grid, kCopyThreads, 0, s>>>(P, S, ctl, stats ? 1 : 0);
+    err = cudaGetLastError();
+  }
+  if (err == cudaSuccess) {
+    err = cudaMemcpyAsync(pinned, S.result, sizeof(FusedResult), cudaMemcpyDeviceToHost, s);
+  }
+  if (err == cudaSuccess) {
+    err = cudaMemcpyAsync(pinnedCtl, ctl, sizeof(EngineControl), cudaMemcpyDeviceToHost, s);
+  }
+  if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+  return err;
+}
+
+}  // namespace mospb200

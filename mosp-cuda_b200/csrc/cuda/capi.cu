@@ -39,7 +39,7 @@ int cudaFail(cudaError_t err, const char *what) {
     if (err_ != cudaSuccess) return cudaFail(err_, #call); \
   } while (0)
 
-constexpr int kControlBlocks = 4;  // 0: update/scratch, 1: combined, 2: build, 3: costs
+constexpr int kControlBlocks = 5;  // 0: update/scratch, 1: combined, 2: build, 3: costs, 4: Step 1
 
 }  // namespace
 
@@ -93,6 +93,7 @@ struct mosp_workspace {
   // control blocks
   EngineControl *ctl = nullptr;
   EngineControl *hostCtl = nullptr;  // pinned
+  FusedResult *hostApply = nullptr;  // pinned
   long long *blockSums = nullptr;
   int blockSumsCap = 0;
   // combined graph
@@ -220,7 +221,8 @@ int ensureShape(mosp_workspace *ws) {
     return fail(MOSP_ERR_UNSUPPORTED, "the GPU does not support cooperative launches");
   }
   if (err != cudaSuccess) return cudaFail(err, "occupancy query");
-  const int maxCtas = std::max({ws->shape.engineCtas, ws->shape.buildCtas, ws->shape.costCtas});
+  const int maxCtas = std::max({ws->shape.engineCtas, ws->shape.buildCtas, ws->shape.costCtas,
+                                ws->shape.applyCtas});
   if (maxCtas > ws->blockSumsCap) {
     int st = deviceAlloc(&ws->blockSums, maxCtas);
     if (st != MOSP_OK) return st;
@@ -826,6 +828,10 @@ int mosp_workspace_create(mosp_workspace **out) {
           cudaSuccess) {
     st = fail(MOSP_ERR_OOM, "pinned allocation failed");
   }
+  if (st == MOSP_OK && cudaMallocHost(reinterpret_cast<void **>(&ws->hostApply), sizeof(FusedResult)) !=
+                           cudaSuccess) {
+    st = fail(MOSP_ERR_OOM, "pinned allocation failed");
+  }
   if (st != MOSP_OK) {
     mosp_workspace_destroy(ws);
     return st;
@@ -862,6 +868,7 @@ void mosp_workspace_destroy(mosp_workspace *ws) {
     if (e) cudaEventDestroy(e);
   }
   if (ws->hostCtl) cudaFreeHost(ws->hostCtl);
+  if (ws->hostApply) cudaFreeHost(ws->hostApply);
   if (dev >= 0) cudaSetDevice(dev);
   delete ws;
 }
@@ -1129,7 +1136,8 @@ int mosp_apply_batch_device(mosp_workspace *ws, int n, int K, int m, const int *
     return fail(MOSP_ERR_INVALID, "Error: invalid change-batch arguments (the updated graph needs "
                                   "room for m + n_ins edges).");
   }
-  const size_t need = applyScratchBytes(n, m, n_ins, n_del);
+  const bool fused = static_cast<long long>(n_ins) + n_del <= kFusedBatch;
+  const size_t need = fused ? applyFusedBytes(n, m, n_ins, n_del) : applyScratchBytes(n, m, n_ins, n_del);
   if (need > ws->applyBytes) {
     // grow by half again: batches of varying size then rarely reallocate
     // (a reallocation's cudaFree waits for the whole device)
@@ -1163,6 +1171,23 @@ int mosp_apply_batch_device(mosp_workspace *ws, int n, int K, int m, const int *
   P.newCol = d_new_col;
   P.newW = d_new_w;
   P.mask = d_mask;
+  if (fused) {
+    cudaStream_t s = asStream(stream);
+    const bool stats = h_max_weight != nullptr || h_weight_sum != nullptr;
+    MOSP_CUDA(applyBatchFused(P, ws->applyScratch, ws->ctl + 4, ws->blockSums, ws->timeoutNs,
+                              limitCtas(ws, ws->shape.applyCtas), stats, ws->hostApply, ws->hostCtl + 4, s));
+    const EngineControl &h = ws->hostCtl[4];
+    if (h.status != 0) return fail(MOSP_ERR_TIMEOUT, "Error: the batch application timed out.");
+    if (h.invalid) {
+      return fail(MOSP_ERR_INVALID, "Error: a changed edge's endpoint is out of range.");
+    }
+    *new_m = ws->hostApply->newM;
+    for (int k = 0; k < K; ++k) {
+      if (h_max_weight) h_max_weight[k] = ws->hostApply->maxWeight[k];
+      if (h_weight_sum) h_weight_sum[k] = ws->hostApply->weightSum[k];
+    }
+    return MOSP_OK;
+  }
   int counters[kApplyCounters + 1] = {0};
   long long stats[2 * kMaxK] = {0};
   const bool wantStats = h_max_weight != nullptr || h_weight_sum != nullptr;

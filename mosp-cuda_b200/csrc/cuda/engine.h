@@ -275,7 +275,7 @@ struct CostParams {
 // Host-side launchers (engine.cu). Each returns a cudaError_t of the
 // launch; device-side errors are reported through the control block.
 struct LaunchShape {
-  int engineCtas, buildCtas, costCtas;
+  int engineCtas, buildCtas, costCtas, applyCtas;
 };
 cudaError_t queryLaunchShape(int ctasPerSm, LaunchShape &shape);
 cudaError_t launchEngine(const EngineParams &p, int ctas, cudaStream_t s);
@@ -346,6 +346,26 @@ size_t applyScratchBytes(long long n, long long m, long long nIns, long long nDe
 /// the original edges (2K values).
 cudaError_t applyBatchGpu(ApplyParams P, void *scratch, int sms, cudaStream_t s, int *hostCounters,
                           long long *hostStats);
+
+// Step 1 in one cooperative launch (applyFused.cu), for batches of up to this
+// many changes
+constexpr long long kFusedBatch = 1 << 18;
+
+/// What a fused Step 1 leaves for the host.
+struct FusedResult {
+  int newM;
+  int pad;
+  long long maxWeight[kMaxK];
+  long long weightSum[kMaxK];
+};
+size_t applyFusedBytes(long long n, long long m, long long nIns, long long nDel);
+cudaError_t applyFusedShape(int sms, int ctasPerSm, int &ctas);
+/// Runs Step 1 on stream `s` with `ctas` CTAs and waits for it; the result
+/// and the control block come back in the pinned buffers (the result is valid
+/// if the control block's status and invalid are zero).
+cudaError_t applyBatchFused(const ApplyParams &P, void *scratch, EngineControl *ctl, long long *blockSums,
+                            long long timeoutNs, int ctas, bool stats, FusedResult *pinned,
+                            EngineControl *pinnedCtl, cudaStream_t s);
 
 /// Whether v is a root: the source, or one of the sorted batched roots.
 __device__ __forceinline__ bool isRoot(int source, const int *sources, int nSources, int v) {
