@@ -841,10 +841,10 @@ __device__ bool nearFarLoop(const EngineParams &P, const int *outRow,
 //
 // Measured on a B200 against one grid-wide sharded queue with a claim, a slot
 // and two counters per hop: a hop of a bare chain 0.72 us; tree from scratch
-// of a 497,700-vertex road network 10.05 -> 2.59 ms, update of a million
-// vertices with local detours (K = 3) 28.7 -> 8.8 ms, combined graph of
-// 249,500 vertices (K = 6) 5.26 -> 1.38 ms, update of 2M vertices with
-// long-range insertions (wide phases) 2.49 -> 2.43 ms.
+// of a 497,700-vertex road network 10.05 -> 2.43 ms, update of a million
+// vertices with local detours (K = 3) 28.7 -> 7.9 ms, combined graph of
+// 249,500 vertices (K = 6) 5.26 -> 1.34 ms, update of 2M vertices with
+// long-range insertions (wide phases) 2.49 -> 2.30 ms.
 //
 // A vertex enters the far pile when an atomicMin takes it from infinity (or,
 // in an update, from its tree distance) to a distance past the threshold;
@@ -1450,203 +1450,6 @@ __device__ __forceinline__ void chase(const EngineParams &P, const int *outRow, 
   }
 }
 
-/// The edges from the fourth on of the rows longer than a record (this
-/// lane's entry v with offer base `base` has one where `more`), one lane per
-/// row. All lanes call it.
-template <int Mode>
-__device__ __noinline__ int restOfRows(const EngineParams &P, bool donate, int farCount, bool more, int k,
-                                       int v, u64 base) {
-  AsyncCta &C = asyncCta();
-  const AsyncObj &O = C.obj[k];
-  const int *outRow = Mode == kModeCombined ? P.combRow : P.outRow;
-  const int *outCol = Mode == kModeCombined ? P.combCol : P.outCol;
-  int e = 0, end = 0;
-  if (more) {
-    e = ldLoop<Mode>(outRow + v) + kRecordEdges;
-    end = ldLoop<Mode>(outRow + v + 1);
-  }
-  while (__any_sync(kFull, e < end)) {
-    const bool in = e < end;
-    const int x = in ? ldLoop<Mode>(outCol + e) : P.source;
-    const u64 cw =
-        base + static_cast<u64>(in ? static_cast<unsigned>(ldLoop<Mode>(O.outW + e)) : 0u) * O.scale;
-    u64 old = 0;
-    if (in && x != P.source && cw <= O.mostWord) old = atomicMin(O.packed + x, cw);
-    pushEdges<Mode>(P, O, donate, farCount, k, x, cw, old);
-    ++e;
-  }
-  return farCount;
-}
-
-/// Thin wavefronts of a graph with row records: up to eight entries, four
-/// lanes each (lane sub of the quad takes the record's edge sub), expanded
-/// hop after hop by the same warp for as long as they improve something
-/// below the threshold. The record of a head is requested before its
-/// atomicMin, so a hop is one round trip to L2 and a short run of
-/// instructions (a lone warp issues them one after another, so they count
-/// as much as the round trip): words are compared without unpacking them,
-/// and the next hop's entries pass through slots in shared memory. More than
-/// eight go to an idle warp by mail, or to the ring.
-template <int Mode>
-__device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int farCount, int k, int v,
-                                         u64 base, int x, int t) {
-  AsyncCta &C = asyncCta();
-  const unsigned lane = laneId();
-  const int sub = static_cast<int>(lane & 3u);
-  const int q = static_cast<int>(lane >> 2);
-  HopSlot *slots = C.hop[threadIdx.x >> 5];
-  const AsyncObj *O = &C.obj[k];
-  u64 *packed = O->packed;
-  const int4 *rec = O->rec;
-  u64 thrWord = O->thrWord, mostWord = O->mostWord;
-  unsigned scale = O->scale, mask = O->mask;
-  const bool oneK = C.K == 1;
-  for (unsigned hops = 1;; ++hops) {
-    if ((hops & 4095u) == 0 && (ldShared(&C.abort) != 0 || globalNs() > C.deadline)) {
-      atomicCAS(&P.ctl->status, 0, MOSP_ERR_TIMEOUT);
-      stShared(&C.abort, 1);
-      return farCount;
-    }
-    const u64 cw = static_cast<u64>(static_cast<unsigned>(t)) * scale + base;
-    u64 old = 0;
-    int4 cols, wts;
-    if (x >= 0 && cw <= mostWord) {
-      // (volatile, so that they are requested before the atomicMin)
-      asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
-                   : "=r"(cols.x), "=r"(cols.y), "=r"(cols.z), "=r"(cols.w)
-                   : "l"(rec + 2LL * x));
-      asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
-                   : "=r"(wts.x), "=r"(wts.y), "=r"(wts.z), "=r"(wts.w)
-                   : "l"(rec + 2LL * x + 1));
-      old = atomicMin(packed + x, cw);
-    }
-    if (__any_sync(kFull, x == kMoreEdges)) {
-      farCount = restOfRows<Mode>(P, donate, farCount, x == kMoreEdges, k, v, base);
-    }
-    const bool imp = old > (cw | mask);
-    const bool near = imp && cw < thrWord;
-    const unsigned keep = __ballot_sync(kFull, near);
-    farAppend(P, farCount, imp && !near && newInFar<Mode>(*O, old, x), k, x, cw >> O->bits);
-    if (keep == 0) return farCount;
-    const int count = __popc(keep);
-    const int rank = __popc(keep & ((1u << lane) - 1u));
-    if (count > kQuadBatch) {
-      // the next eight by mail to an idle warp
-      int w = -1, busy = 0;
-      if (lane == 0) {
-        w = takeIdle();
-        busy = w < 0 && ldShared(&C.tail) - ldShared(&C.head) > kChaseRing;
-      }
-      w = __shfl_sync(kFull, w, 0);
-      busy = __shfl_sync(kFull, busy, 0);
-      int kept = kQuadBatch;
-      if (w >= 0) {
-        if (near && rank >= kQuadBatch && rank < 2 * kQuadBatch) {
-          C.mailbox[w][rank - kQuadBatch] = HopSlot{cw, x, k, cols, wts};
-        }
-        __syncwarp();
-        if (lane == 0) {
-          const int sent = count - kQuadBatch < kMail ? count - kQuadBatch : kMail;
-          atomicAdd(&C.mailed, static_cast<unsigned>(sent));
-          C.mail[w] = sent;
-          barArrive(&C.bar[w]);
-        }
-        kept = 2 * kQuadBatch;
-      }
-      // a CTA with work for all its warps keeps the breadth-first order
-      const unsigned give = __ballot_sync(kFull, near && (busy || rank >= kept));
-      if (give != 0) ringPush(P, give, donate, nearEntry(k, x, cw >> O->bits));
-      if (busy) return farCount;
-    }
-    // quad q goes on with the q-th of them
-    if (near && rank < kQuadBatch) slots[rank] = HopSlot{cw, x, k, cols, wts};
-    __syncwarp();
-    x = -1;
-    if (q < count) {
-      const HopSlot &h = slots[q];
-      v = h.v;
-      if (!oneK) {
-        k = h.k;
-        O = &C.obj[k];
-        packed = O->packed;
-        rec = O->rec;
-        thrWord = O->thrWord;
-        mostWord = O->mostWord;
-        scale = O->scale;
-        mask = O->mask;
-      }
-      x = reinterpret_cast<const int *>(&h.cols)[sub];
-      t = reinterpret_cast<const int *>(&h.wts)[sub];
-      base = nextBase(h.word, v, mask);
-      if (sub == 0) atomicAdd(&C.expanded[k], 1u);
-    }
-    __syncwarp();
-  }
-}
-
-/// One entry per lane of a graph with row records: its word and its record
-/// arrive together, its edges' atomicMin go out together, the improvements
-/// of the warp take one reservation of the ring.
-template <int Mode>
-__device__ __noinline__ int expandRecords(const EngineParams &P, bool donate, int farCount, int k, int v,
-                                          u64 base, bool live, int4 cols, int4 wts) {
-  AsyncCta &C = asyncCta();
-  const unsigned lane = laneId();
-  const AsyncObj &O = C.obj[k];
-  const unsigned scale = O.scale;
-  const u64 most = live ? O.mostWord : 0;  // 0: nothing passes
-  const u64 thrWord = O.thrWord;
-  const int x[4] = {cols.x, cols.y, cols.z, cols.w};
-  const u64 cw[4] = {static_cast<u64>(static_cast<unsigned>(wts.x)) * scale + base,
-                     static_cast<u64>(static_cast<unsigned>(wts.y)) * scale + base,
-                     static_cast<u64>(static_cast<unsigned>(wts.z)) * scale + base,
-                     static_cast<u64>(static_cast<unsigned>(wts.w)) * scale + base};
-  u64 old[4];
-#pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    old[h] = 0;
-    if (x[h] >= 0 && cw[h] <= most) old[h] = atomicMin(O.packed + x[h], cw[h]);
-  }
-  if (__any_sync(kFull, live && x[3] == kMoreEdges)) {
-    farCount = restOfRows<Mode>(P, donate, farCount, live && x[3] == kMoreEdges, k, v, base);
-  }
-  unsigned near = 0, far = 0;  // bit h: this lane's edge h
-  unsigned ballot[4];
-  int count = 0;
-#pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    const bool imp = old[h] > (cw[h] | O.mask);
-    const bool nr = imp && cw[h] < thrWord;
-    near |= static_cast<unsigned>(nr) << h;
-    far |= static_cast<unsigned>(imp && !nr && newInFar<Mode>(O, old[h], x[h])) << h;
-    ballot[h] = __ballot_sync(kFull, nr);
-    count += __popc(ballot[h]);
-  }
-  if (count > 0) {
-    unsigned at = 0;
-    int room = 0;
-    if (lane == 0) room = ringReserve(donate, count, at);
-    room = __shfl_sync(kFull, room, 0);
-    at = __shfl_sync(kFull, at, 0);
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      if (ballot[h] == 0) continue;
-      const u64 e = nearEntry(k, x[h], cw[h] >> O.bits);
-      if (!room) {
-        spillNear(P, ballot[h], e);
-      } else {
-        if ((near >> h) & 1u) ringWrite(P, at + __popc(ballot[h] & ((1u << lane) - 1u)), e);
-        at += __popc(ballot[h]);
-      }
-    }
-  }
-  if (__any_sync(kFull, far != 0)) {
-#pragma unroll
-    for (int h = 0; h < 4; ++h) farAppend(P, farCount, (far >> h) & 1u, k, x[h], cw[h] >> O.bits);
-  }
-  return farCount;
-}
-
 /// The rows of the lanes' entries (this lane's: edges [beg, end) of v at
 /// distance du in objective k; beg == end for none) as one flat range of
 /// edges, three per lane and turn. All lanes call it.
@@ -1711,6 +1514,176 @@ __device__ __forceinline__ void expandRows(const EngineParams &P, const int *out
 #pragma unroll
     for (int h = 0; h < SL; ++h) pushEdges<Mode>(P, C.obj[kk[h]], donate, farCount, kk[h], ww[h], cw[h], old[h]);
   }
+}
+
+/// Thin wavefronts of a graph with row records: up to eight entries, four
+/// lanes each (lane sub of the quad takes the record's edge sub), expanded
+/// hop after hop by the same warp for as long as they improve something
+/// below the threshold. The record of a head is requested before its
+/// atomicMin, so a hop is one round trip to L2 and a short run of
+/// instructions (a lone warp issues them one after another, so they count
+/// as much as the round trip): words are compared without unpacking them,
+/// and the next hop's entries pass through slots in shared memory. More than
+/// eight go to an idle warp by mail, or to the ring.
+template <int Mode>
+__device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int farCount, int k, int v,
+                                         u64 base, int x, int t) {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  const int sub = static_cast<int>(lane & 3u);
+  const int q = static_cast<int>(lane >> 2);
+  HopSlot *slots = C.hop[threadIdx.x >> 5];
+  const AsyncObj *O = &C.obj[k];
+  u64 *packed = O->packed;
+  const int4 *rec = O->rec;
+  u64 thrWord = O->thrWord, mostWord = O->mostWord;
+  unsigned scale = O->scale, mask = O->mask;
+  const bool oneK = C.K == 1;
+  for (unsigned hops = 1;; ++hops) {
+    if ((hops & 4095u) == 0 && (ldShared(&C.abort) != 0 || globalNs() > C.deadline)) {
+      atomicCAS(&P.ctl->status, 0, MOSP_ERR_TIMEOUT);
+      stShared(&C.abort, 1);
+      return farCount;
+    }
+    const u64 cw = static_cast<u64>(static_cast<unsigned>(t)) * scale + base;
+    u64 old = 0;
+    int4 cols, wts;
+    if (x >= 0 && cw <= mostWord) {
+      // (volatile, so that they are requested before the atomicMin)
+      asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(cols.x), "=r"(cols.y), "=r"(cols.z), "=r"(cols.w)
+                   : "l"(rec + 2LL * x));
+      asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(wts.x), "=r"(wts.y), "=r"(wts.z), "=r"(wts.w)
+                   : "l"(rec + 2LL * x + 1));
+      old = atomicMin(packed + x, cw);
+    }
+    const bool imp = old > (cw | mask);
+    const bool near = imp && cw < thrWord;
+    // a head whose row is longer than its record goes to the ring, for a batch
+    // by rows: its quad would load the rest of a long row one edge after
+    // another (R-MAT graph of 4,547 vertices, rows up to 2,000 edges: 885 ->
+    // 338 us per update)
+    const bool more = near && cols.w == kMoreEdges;
+    const unsigned keep = __ballot_sync(kFull, near && !more);
+    const unsigned longer = __ballot_sync(kFull, more);
+    if (longer != 0) ringPush(P, longer, donate, nearEntry(k, x, cw >> O->bits));
+    farAppend(P, farCount, imp && !near && newInFar<Mode>(*O, old, x), k, x, cw >> O->bits);
+    if (keep == 0) return farCount;
+    const int count = __popc(keep);
+    const int rank = __popc(keep & ((1u << lane) - 1u));
+    if (count > kQuadBatch) {
+      // the next eight by mail to an idle warp
+      int w = -1, busy = 0;
+      if (lane == 0) {
+        w = takeIdle();
+        busy = w < 0 && ldShared(&C.tail) - ldShared(&C.head) > kChaseRing;
+      }
+      w = __shfl_sync(kFull, w, 0);
+      busy = __shfl_sync(kFull, busy, 0);
+      int kept = kQuadBatch;
+      if (w >= 0) {
+        if (near && !more && rank >= kQuadBatch && rank < 2 * kQuadBatch) {
+          C.mailbox[w][rank - kQuadBatch] = HopSlot{cw, x, k, cols, wts};
+        }
+        __syncwarp();
+        if (lane == 0) {
+          const int sent = count - kQuadBatch < kMail ? count - kQuadBatch : kMail;
+          atomicAdd(&C.mailed, static_cast<unsigned>(sent));
+          C.mail[w] = sent;
+          barArrive(&C.bar[w]);
+        }
+        kept = 2 * kQuadBatch;
+      }
+      // a CTA with work for all its warps keeps the breadth-first order
+      const unsigned give = __ballot_sync(kFull, near && !more && (busy || rank >= kept));
+      if (give != 0) ringPush(P, give, donate, nearEntry(k, x, cw >> O->bits));
+      if (busy) return farCount;
+    }
+    // quad q goes on with the q-th of them
+    if (near && !more && rank < kQuadBatch) slots[rank] = HopSlot{cw, x, k, cols, wts};
+    __syncwarp();
+    x = -1;
+    if (q < count) {
+      const HopSlot &h = slots[q];
+      v = h.v;
+      if (!oneK) {
+        k = h.k;
+        O = &C.obj[k];
+        packed = O->packed;
+        rec = O->rec;
+        thrWord = O->thrWord;
+        mostWord = O->mostWord;
+        scale = O->scale;
+        mask = O->mask;
+      }
+      x = reinterpret_cast<const int *>(&h.cols)[sub];
+      t = reinterpret_cast<const int *>(&h.wts)[sub];
+      base = nextBase(h.word, v, mask);
+      if (sub == 0) atomicAdd(&C.expanded[k], 1u);
+    }
+    __syncwarp();
+  }
+}
+
+/// One entry per lane of a graph with row records: its word and its record
+/// arrive together, its edges' atomicMin go out together, the improvements
+/// of the warp take one reservation of the ring.
+template <int Mode>
+__device__ __noinline__ int expandRecords(const EngineParams &P, bool donate, int farCount, int k, int v,
+                                          u64 base, bool live, int4 cols, int4 wts) {
+  AsyncCta &C = asyncCta();
+  const unsigned lane = laneId();
+  const AsyncObj &O = C.obj[k];
+  const unsigned scale = O.scale;
+  const u64 most = live ? O.mostWord : 0;  // 0: nothing passes
+  const u64 thrWord = O.thrWord;
+  const int x[4] = {cols.x, cols.y, cols.z, cols.w};
+  const u64 cw[4] = {static_cast<u64>(static_cast<unsigned>(wts.x)) * scale + base,
+                     static_cast<u64>(static_cast<unsigned>(wts.y)) * scale + base,
+                     static_cast<u64>(static_cast<unsigned>(wts.z)) * scale + base,
+                     static_cast<u64>(static_cast<unsigned>(wts.w)) * scale + base};
+  u64 old[4];
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    old[h] = 0;
+    if (x[h] >= 0 && cw[h] <= most) old[h] = atomicMin(O.packed + x[h], cw[h]);
+  }
+  unsigned near = 0, far = 0;  // bit h: this lane's edge h
+  unsigned ballot[4];
+  int count = 0;
+#pragma unroll
+  for (int h = 0; h < 4; ++h) {
+    const bool imp = old[h] > (cw[h] | O.mask);
+    const bool nr = imp && cw[h] < thrWord;
+    near |= static_cast<unsigned>(nr) << h;
+    far |= static_cast<unsigned>(imp && !nr && newInFar<Mode>(O, old[h], x[h])) << h;
+    ballot[h] = __ballot_sync(kFull, nr);
+    count += __popc(ballot[h]);
+  }
+  if (count > 0) {
+    unsigned at = 0;
+    int room = 0;
+    if (lane == 0) room = ringReserve(donate, count, at);
+    room = __shfl_sync(kFull, room, 0);
+    at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      if (ballot[h] == 0) continue;
+      const u64 e = nearEntry(k, x[h], cw[h] >> O.bits);
+      if (!room) {
+        spillNear(P, ballot[h], e);
+      } else {
+        if ((near >> h) & 1u) ringWrite(P, at + __popc(ballot[h] & ((1u << lane) - 1u)), e);
+        at += __popc(ballot[h]);
+      }
+    }
+  }
+  if (__any_sync(kFull, far != 0)) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) farAppend(P, farCount, (far >> h) & 1u, k, x[h], cw[h] >> O.bits);
+  }
+  return farCount;
 }
 
 /// An idle warp's wait (warps other than 0): the entries that came by mail,
@@ -1939,7 +1912,18 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
     }
     if (live && lead) atomicAdd(&C.expanded[k], 1u);
     donate = __shfl_sync(kFull, hungry, 0) > 0;
+    bool rows = !records;
     if constexpr (Rec) {
+      // a row longer than its record: this batch by rows
+      if (records && __any_sync(kFull, live && (thin ? cols.x : cols.w) == kMoreEdges)) {
+        rows = true;
+        if (live) {
+          beg = ldLoop<Mode>(outRow + v);
+          end = ldLoop<Mode>(outRow + v + 1);
+        }
+      }
+    }
+    if (Rec && !rows) {
       const u64 base = offerBase(O, du, v);
       if (thin) {
         farCount = chaseRecords<Mode>(P, donate, farCount, k, v, base, live ? cols.x : -1, wts.x);

@@ -148,10 +148,9 @@ struct alignas(128) AsyncShard {
 };
 constexpr int kAsyncShards = 16;  // shards of the spill queue
 
-// Row records of the asynchronous loop: the first edges of a row, side by
-// side with their weights, in one 32-byte sector per objective and vertex.
-constexpr int kRecordEdges = 3;  // edges in the record of a row of more than four
-constexpr int kMoreEdges = -2;   // fourth head of such a record
+// Row records of the asynchronous loop: the edges of a row, side by side with
+// their weights, in one 32-byte sector per objective and vertex.
+constexpr int kMoreEdges = -2;   // fourth head of a record: the row has more than four edges
 
 /// A far pile of the asynchronous loop holds a vertex at most this often:
 /// once as it leaves infinity or its valid tree distance, once more when an
