@@ -220,8 +220,9 @@ int mosp_workspace_set_ctas_per_sm(mosp_workspace *ws, int ctas_per_sm);
  * one 1,024-thread CTA per SM on every SM (the occupancy-sized grid of the
  * reference, src/sospUpdateGpu.cu:553-595); a smaller count launches fewer
  * CTAs (cheaper grid barriers, fewer warps). hub_edges (0 = 2,048, else at
- * least 64): rows with more edges are expanded and reduced by a whole CTA,
- * and a graph with such rows runs the bulk near-far loop. Results do not
+ * least 64): a graph with rows of more edges runs the bulk near-far loop,
+ * and a whole CTA expands and reduces each such row (at 0, each row of more
+ * than 512 edges). Results do not
  * depend on either; mosp_autotune_update picks both. No counterpart in the
  * reference. */
 int mosp_workspace_set_grid(mosp_workspace *ws, int ctas, int hub_edges);

@@ -19,9 +19,9 @@
 //     vertex, so a pointer-jumping step is two dependent loads;
 //   * list appends are staged per CTA in shared memory and written out
 //     with one reservation per list and iteration; a warp spreads the
-//     edges of its items over its lanes, and rows of more than 2,048 edges
-//     (power-law hubs) go to the whole CTA, in launches whose graph has
-//     them;
+//     edges of its items over its lanes, and rows of more than 512 edges
+//     go to the whole CTA, in launches whose graph has power-law hubs
+//     (rows of more than 2,048);
 //   * the pull pass scans in-rows four edges per round with their loads
 //     in flight together;
 //   * the lowest-id parent recovery of distance-only objectives is
@@ -161,18 +161,27 @@ enum : int { kDone = 0, kPush = 1, kSplit = 2 };
 // path. Entries that do not fit the buffer take the direct global path.
 // ---------------------------------------------------------------------------
 constexpr int kStage = kStageEntriesMax;
-// Rows with more edges than this are expanded (push) or reduced (pull) by a
-// whole CTA instead of one warp: a power-law hub row (10^5 edges) would
-// otherwise keep one warp busy for the whole iteration. A launch turns
-// this on only when its graph has such rows (EngineControl::heavy, set in
-// the first phase), so graphs without them take no extra CTA barriers.
+// Long rows are expanded (push) or reduced (pull) by a whole CTA instead of
+// one warp: a power-law hub row (10^5 edges) would otherwise keep one warp
+// busy for the whole iteration. A launch turns this on only when its graph
+// has rows of more edges than this (EngineControl::heavy, set in the first
+// phase), so graphs without them take no extra CTA barriers.
 constexpr int kHeavyDegDefault = 2048;  // EngineParams::heavyDeg when 0
-constexpr int kHeavyCap = 64;
+constexpr int kHeavyCap = 128;
 
-/// Rows above this many edges go to a whole CTA (and keep a launch in the
-/// bulk loop); a launch parameter, so the autotuner can move it.
+/// A graph with rows above this many edges runs the bulk loop; a launch
+/// parameter, so the autotuner can move it.
 __device__ __forceinline__ int heavyDegOf(const EngineParams &P) {
   return P.heavyDeg > 0 ? P.heavyDeg : kHeavyDegDefault;
+}
+
+/// In such a launch, rows above this many edges go to a whole CTA: a quarter of
+/// the default threshold, since a warp with 2,000 edges of its own keeps the
+/// grid waiting (R-MAT graph of scale 22, K = 5: update and combined loops
+/// 1.32 -> 0.95 ms; of 60,001 vertices 0.24 -> 0.20 ms), while graphs with no
+/// longer rows than that stay faster in the asynchronous loop.
+__device__ __forceinline__ int ctaRowOf(const EngineParams &P) {
+  return P.heavyDeg > 0 ? P.heavyDeg : kHeavyDegDefault / 4;
 }
 
 struct StageHeader {
@@ -437,7 +446,7 @@ __device__ __forceinline__ void expandWarp(const EngineParams &P, const LoopShar
   if (__ballot_sync(kFull, deg > 0) == 0) return;
   // heavy rows go to the CTA's queue (expanded by the whole CTA after this
   // round of items) when the launch has any
-  if (heavyOn && deg > heavyDegOf(P)) {
+  if (heavyOn && deg > ctaRowOf(P)) {
     const int slot = atomicAdd(&H.heavyCount, 1);
     if (slot < kHeavyCap) {
       H.heavyK[slot] = k;
@@ -2823,9 +2832,12 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
         __syncthreads();
       };
       const long long tileStride = static_cast<long long>(gridDim.x) * blockDim.x;
-      for (long long tile = static_cast<long long>(blockIdx.x) * blockDim.x; tile < total;
-           tile += tileStride) {
-        const long long j = tile + threadIdx.x;
+      for (long long tile = static_cast<long long>(blockIdx.x) * blockDim.x;
+           tile - static_cast<long long>(blockIdx.x) * blockDim.x < total; tile += tileStride) {
+        // the tiles of all CTAs interleaved, so that few candidates (the
+        // heads of a small batch, hubs among them) spread over the grid
+        const long long j = tile - static_cast<long long>(blockIdx.x) * blockDim.x +
+                            static_cast<long long>(threadIdx.x) * gridDim.x + blockIdx.x;
         const bool valid = j < total;
         int k = 0;
         if (valid) {
@@ -2843,7 +2855,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
           end = __ldg(P.inRow + v + 1);
         }
         // heavy in-rows are reduced by the whole CTA after the tile
-        if (heavyOn && end - beg > heavyDegOf(P)) {
+        if (heavyOn && end - beg > ctaRowOf(P)) {
           const int slot = atomicAdd(&H.heavyCount, 1);
           if (slot < kHeavyCap) {
             H.heavyK[slot] = k;

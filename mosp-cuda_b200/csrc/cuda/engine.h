@@ -208,7 +208,8 @@ struct EngineParams {
   int4 *rec;                   // row records (two int4 per vertex; objective k from
                                // 2 * k * stride) or null: the launch uses none
   int stageEntries;            // entries of the per-CTA append stage (dynamic shared memory)
-  int heavyDeg;                // rows above this many edges: whole-CTA handling (0: 2,048)
+  int heavyDeg;                // a row above this many edges: bulk loop, longer rows by whole
+                               // CTAs (0: 2,048 for the loop, 512 for the rows)
   EngineControl *ctl;
   // combined graph (Steps 2-3)
   const int *combParents;      // K trees, objective-major
