@@ -849,10 +849,10 @@ __device__ bool nearFarLoop(const EngineParams &P, const int *outRow,
 // loads of a hop one round trip to L2 that runs beside the atomicMin.
 //
 // Measured on a B200 against one grid-wide sharded queue with a claim, a slot
-// and two counters per hop: a hop of a bare chain 0.72 us; tree from scratch
-// of a 497,700-vertex road network 10.05 -> 2.43 ms, update of a million
-// vertices with local detours (K = 3) 28.7 -> 7.9 ms, combined graph of
-// 249,500 vertices (K = 6) 5.26 -> 1.34 ms, update of 2M vertices with
+// and two counters per hop: a hop of a bare chain 0.59 us; tree from scratch
+// of a 497,700-vertex road network 10.05 -> 2.32 ms, update of a million
+// vertices with local detours (K = 3) 28.7 -> 7.8 ms, combined graph of
+// 249,500 vertices (K = 6) 5.26 -> 1.27 ms, update of 2M vertices with
 // long-range insertions (wide phases) 2.49 -> 2.30 ms.
 //
 // A vertex enters the far pile when an atomicMin takes it from infinity (or,
@@ -1547,12 +1547,15 @@ __device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int
   const int4 *rec = O->rec;
   u64 thrWord = O->thrWord, mostWord = O->mostWord;
   unsigned scale = O->scale, mask = O->mask;
-  const bool oneK = C.K == 1;
+  const bool oneK = Mode != kModeUpdate || C.K == 1;
+  // expansions, counted here where there is one objective: an atomicAdd to
+  // shared memory per hop costs 70 ns of it on a bare chain
+  unsigned done = 0;
   for (unsigned hops = 1;; ++hops) {
     if ((hops & 4095u) == 0 && (ldShared(&C.abort) != 0 || globalNs() > C.deadline)) {
       atomicCAS(&P.ctl->status, 0, MOSP_ERR_TIMEOUT);
       stShared(&C.abort, 1);
-      return farCount;
+      break;
     }
     const u64 cw = static_cast<u64>(static_cast<unsigned>(t)) * scale + base;
     u64 old = 0;
@@ -1575,10 +1578,13 @@ __device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int
     // 338 us per update)
     const bool more = near && cols.w == kMoreEdges;
     const unsigned keep = __ballot_sync(kFull, near && !more);
-    const unsigned longer = __ballot_sync(kFull, more);
-    if (longer != 0) ringPush(P, longer, donate, nearEntry(k, x, cw >> O->bits));
-    farAppend(P, farCount, imp && !near && newInFar<Mode>(*O, old, x), k, x, cw >> O->bits);
-    if (keep == 0) return farCount;
+    // (the update has something for the far pile in most hops: one ballot less)
+    if (Mode == kModeUpdate || __any_sync(kFull, imp && (more || !near))) {
+      const unsigned longer = __ballot_sync(kFull, more);
+      if (longer != 0) ringPush(P, longer, donate, nearEntry(k, x, cw >> O->bits));
+      farAppend(P, farCount, imp && !near && newInFar<Mode>(*O, old, x), k, x, cw >> O->bits);
+    }
+    if (keep == 0) break;
     const int count = __popc(keep);
     const int rank = __popc(keep & ((1u << lane) - 1u));
     if (count > kQuadBatch) {
@@ -1607,12 +1613,13 @@ __device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int
       // a CTA with work for all its warps keeps the breadth-first order
       const unsigned give = __ballot_sync(kFull, near && !more && (busy || rank >= kept));
       if (give != 0) ringPush(P, give, donate, nearEntry(k, x, cw >> O->bits));
-      if (busy) return farCount;
+      if (busy) break;
     }
     // quad q goes on with the q-th of them
     if (near && !more && rank < kQuadBatch) slots[rank] = HopSlot{cw, x, k, cols, wts};
     __syncwarp();
     x = -1;
+    if (Mode != kModeUpdate) done += count < kQuadBatch ? count : kQuadBatch;
     if (q < count) {
       const HopSlot &h = slots[q];
       v = h.v;
@@ -1629,10 +1636,12 @@ __device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int
       x = reinterpret_cast<const int *>(&h.cols)[sub];
       t = reinterpret_cast<const int *>(&h.wts)[sub];
       base = nextBase(h.word, v, mask);
-      if (sub == 0) atomicAdd(&C.expanded[k], 1u);
+      if (Mode == kModeUpdate && sub == 0) atomicAdd(&C.expanded[k], 1u);
     }
     __syncwarp();
   }
+  if (Mode != kModeUpdate && lane == 0 && done != 0) atomicAdd(&C.expanded[0], done);
+  return farCount;
 }
 
 /// One entry per lane of a graph with row records: its word and its record
