@@ -10,24 +10,27 @@
 //   its first and last insertion: minimum and maximum of file positions;
 //   occurrences of v in row u and the first one: count and minimum over the
 //   row's edges.
-// Order matters in two places. The place of a live edge is its old one less
-// the removed edges of its row before it: a ballot over the 32 edges a warp
-// copies, carried along the row. The place of an appended edge is the number
+// Order matters in two places. A live edge moves by the edges appended less
+// those removed before it, in whatever row: each block of 32 edges has the sum
+// up to its first edge (a scan of the groups' changes) and bits for the changes
+// inside it. Only a block with several edges appended at one place goes by its
+// rows. The place of an appended edge is the number
 // of appended groups of its row with an earlier first insertion, counted over
 // the row's own list, which costs the square of the insertions into one row:
 // with all of a batch of 65,536 in one row 1.9 ms (sorted form 10.6), of
 // 262,144 14 ms (24). That sets kFusedBatch.
 //
-// The copy is one pass over all edges in chunks on demand: a warp takes 32
-// edges, finds their rows by a shuffle search and moves their heads and their
-// 32 K weights as one consecutive range each, so loads and stores coalesce
-// whatever K is; the weight statistics are taken from the same loads. Bound
-// by HBM: the graph read and written once.
+// The copy is one pass over all edges: a warp takes 128 of them, which need no
+// row, and moves their heads and their 128 K weights as one consecutive range
+// each, so loads and stores coalesce whatever K is, eight weights per lane in
+// flight; the weight statistics are taken from the same loads. Bound by HBM:
+// the graph read and written once (2.6 TB/s of both on 65M edges; searching
+// the rows of 32 edges at a time instead, 1.4).
 //
 // Measured on a B200, sorted form and this one: 50,000 changes on a road
-// network of 5.56M edges, K = 3 (178 MB read and written): 578 -> 223 us;
+// network of 5.56M edges, K = 3 (178 MB read and written): 578 -> 160 us;
 // 24 changes on 4,200 edges: 307 -> 78 us; 20,000 on an R-MAT graph of 3.9M
-// edges, K = 4: 2112 -> 235 us; 60,000 on one of 65M, K = 5: 12.8 -> 2.2 ms.
+// edges, K = 4: 2112 -> 171 us; 60,000 on one of 65M, K = 5: 12.8 -> 1.2 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -41,7 +44,19 @@ constexpr u64 kNoKey = ~0ULL;
 constexpr int kLaneRow = 16;  // touched rows of at most so many edges are searched by one lane,
 constexpr int kPiece = 64;    // longer ones in pieces of so many by a warp each
 constexpr int kCopyThreads = 256;
-constexpr int kEarly = 4;     // turns of the copy whose weights are loaded ahead
+constexpr int kCopyEdges = 128;  // edges a warp of the copy takes at a time
+constexpr int kTurns = 8;        // turns of its weights in flight
+constexpr unsigned kByRows = ~0U;  // Block::app: more than one edge appended at one place
+constexpr int kNoMove = INT_MIN;
+constexpr int kMaxCtas = 2048;
+
+/// What moves 32 consecutive edges of the old graph.
+struct alignas(16) Block {
+  int shift;      // how far the first one moves (the scan of its changes)
+  unsigned dead;  // edges that go: those behind them move one less
+  unsigned app;   // edges before which one is appended: they move one more
+  unsigned other;  // edges that take an insertion's weights
+};
 
 struct FusedScratch {
   // groups: a hash table of `slots` (a power of two, at least twice the batch)
@@ -53,15 +68,16 @@ struct FusedScratch {
   unsigned filterBits;
   int *entrySlot;  // slot of batch entry j (deletions first)
   // touched rows, in no order
-  int *rows, *nApp, *nDead, *segApp, *segDead, *curApp, *curDead;
+  int *rows, *nApp, *segApp, *curApp;
   u64 *pieces;     // of the longer touched rows: vertex << 32 | piece
-  unsigned *hit;   // one bit per edge: it belongs to a group
+  Block *block;    // per 32 edges, and one behind them
   int *app;        // insertions that append, by row segment
-  int *dead;       // removed edges, by row segment
+  int2 *other;     // edges that take an insertion's weights: edge, slot
   // per vertex: touched row + 1 (0: none), and its change of degree
   int *rowSlot, *delta;
-  int *counts;     // touched rows, pieces, appended, removed
-  long long *blockSums;
+  int *counts;     // touched rows, pieces, appended, edges with an insertion's weights
+  long long *blockSums;  // of the CTAs: degree changes, then (moveSums) block moves
+  long long *moveSums;
   FusedResult *result;
 };
 
@@ -77,19 +93,6 @@ __device__ __forceinline__ unsigned hashOf(u64 key) {
 /// The filter bit of a key with this hash.
 __device__ __forceinline__ unsigned filterBit(const FusedScratch &S, unsigned hash) {
   return (hash >> 9) & (S.filterBits - 1);
-}
-
-/// The group of edge (u, v), or -1. (At most half of the slots are taken, so
-/// the probe ends.)
-__device__ __forceinline__ int findGroup(const FusedScratch &S, int u, int v) {
-  const u64 key = (static_cast<u64>(static_cast<unsigned>(u)) << 32) | static_cast<unsigned>(v);
-  unsigned s = hashOf(key) & (S.slots - 1);
-  while (true) {
-    const u64 at = __ldcg(S.key + s);
-    if (at == key) return static_cast<int>(s);
-    if (at == kNoKey) return -1;
-    s = (s + 1) & (S.slots - 1);
-  }
 }
 
 /// Edges b, b + step, ... (< end) of touched row u: occurrences of their
@@ -128,7 +131,6 @@ __device__ __forceinline__ void countOccurrences(const ApplyParams &P, const Fus
       const int e = e0 + q * step;
       atomicAdd(S.occ + s[q], 1);
       atomicMin(S.first + s[q], e);
-      atomicOr(S.hit + (e >> 5), 1u << (e & 31));
     }
   }
 }
@@ -155,10 +157,53 @@ __device__ __forceinline__ int warpReserve(int *counter, int x) {
   return __shfl_sync(kFull, base, 0) + before;
 }
 
+/// One group of the batch: the change of its row's degree, the edges it
+/// removes and appends as moves of the edges behind them, the list size of
+/// its row, its weight-increase mask, and the edge (other) that takes its last
+/// insertion's weights.
+__device__ __forceinline__ void resolveGroup(const ApplyParams &P, const FusedScratch &S, int s, u64 key,
+                                             int &other) {
+  const int u = static_cast<int>(key >> 32), v = static_cast<int>(key);
+  const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s), cI = __ldcg(S.cI + s);
+  const int removed = occ < cD ? occ : cD;
+  const int appended = occ <= cD && cI > 0 ? 1 : 0;
+  if (appended) {
+    const int r = __ldcg(S.rowSlot + u) - 1;
+    atomicAdd(S.nApp + r, 1);
+    const int e = __ldg(P.row + u + 1);
+    atomicAdd(&S.block[(e + 31) >> 5].shift, 1);
+    if ((e & 31) != 0) {
+      const unsigned bit = 1u << (e & 31);
+      if (atomicOr(&S.block[e >> 5].app, bit) & bit) atomicOr(&S.block[e >> 5].app, kByRows);
+    }
+  }
+  if (appended != removed) atomicAdd(S.delta + u, appended - removed);
+  // the first `removed` occurrences go; the next one takes the weights
+  const int seen = removed + (cI > 0 && occ > cD ? 1 : 0);
+  int e = __ldcg(S.first + s);
+  for (int i = 0; i < seen; ++e) {
+    if (__ldg(P.col + e) != v) continue;
+    if (i++ < removed) {
+      atomicOr(&S.block[e >> 5].dead, 1u << (e & 31));
+      atomicAdd(&S.block[(e >> 5) + 1].shift, -1);
+    } else {
+      atomicOr(&S.block[e >> 5].other, 1u << (e & 31));
+      other = e;
+    }
+  }
+  if (cI > 0 && occ > 0) {
+    const int *wn = P.insW + static_cast<long long>(__ldcg(S.lastIns + s)) * P.K;
+    const int *wo = P.w + static_cast<long long>(__ldcg(S.first + s)) * P.K;
+    unsigned bits = 0;
+    for (int k = 0; k < P.K; ++k) bits |= (wn[k] > wo[k] ? 1u : 0u) << k;
+    S.bits[s] = bits;
+  }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedScratch S, EngineControl *c,
            long long timeoutNs) {
-  const int n = static_cast<int>(P.n), m = static_cast<int>(P.m), K = P.K;
+  const int n = static_cast<int>(P.n), m = static_cast<int>(P.m);
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const long long T = static_cast<long long>(gridDim.x) * blockDim.x;
   const unsigned lane = laneId();
@@ -177,9 +222,9 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
     S.lastIns[s] = -1;
     S.bits[s] = 0;
   }
-  for (long long i = tid; i < (m + 31LL) / 32; i += T) S.hit[i] = 0;
+  for (long long i = tid; i <= (m + 31LL) / 32; i += T) S.block[i] = Block{0, 0, 0, 0};
   for (long long i = tid; i < S.filterBits / 32; i += T) S.filter[i] = 0;
-  for (long long r = tid; r < B; r += T) S.nApp[r] = S.nDead[r] = S.curApp[r] = S.curDead[r] = 0;
+  for (long long r = tid; r < B; r += T) S.nApp[r] = S.curApp[r] = 0;
   if (tid < 4) S.counts[tid] = 0;
   if (tid < kMaxK) {
     S.result->maxWeight[tid] = 1;
@@ -254,43 +299,33 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
   }
   if (!gridSync(c, epoch)) return;
 
-  // ---- groups resolved: degrees, list sizes, weight-increase masks ---------
-  for (long long s = tid; s < S.slots; s += T) {
-    const u64 key = __ldcg(S.key + s);
-    if (key == kNoKey) continue;
-    const int u = static_cast<int>(key >> 32);
-    const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s), cI = __ldcg(S.cI + s);
-    const int removed = occ < cD ? occ : cD;
-    const int appended = occ <= cD && cI > 0 ? 1 : 0;
-    const int r = __ldcg(S.rowSlot + u) - 1;
-    if (appended) atomicAdd(S.nApp + r, 1);
-    if (removed > 0) atomicAdd(S.nDead + r, removed);
-    if (appended != removed) atomicAdd(S.delta + u, appended - removed);
-    if (cI > 0 && occ > 0) {
-      const int *wn = P.insW + static_cast<long long>(__ldcg(S.lastIns + s)) * K;
-      const int *wo = P.w + static_cast<long long>(__ldcg(S.first + s)) * K;
-      unsigned bits = 0;
-      for (int k = 0; k < K; ++k) bits |= (wn[k] > wo[k] ? 1u : 0u) << k;
-      S.bits[s] = bits;
-    }
+  // ---- groups resolved: degrees, what moves edges, list sizes, weight-
+  // increase masks
+  for (long long s0 = tid - lane; s0 < S.slots; s0 += T) {
+    const long long s = s0 + lane;
+    const u64 key = s < S.slots ? __ldcg(S.key + s) : kNoKey;
+    int other = -1;  // the group's edge that takes the last insertion's weights
+    if (key != kNoKey) resolveGroup(P, S, static_cast<int>(s), key, other);
+    const int at = warpReserve(S.counts + 3, other >= 0 ? 1 : 0);
+    if (other >= 0) S.other[at] = make_int2(other, static_cast<int>(s));
   }
   if (!gridSync(c, epoch)) return;
-
   // ---- row segments of the lists; masks; sums of the degree changes --------
   for (long long q0 = tid - lane; q0 < R; q0 += T) {
     const long long r = q0 + lane;
     const int a = warpReserve(S.counts + 2, r < R ? __ldcg(S.nApp + r) : 0);
-    const int d = warpReserve(S.counts + 3, r < R ? __ldcg(S.nDead + r) : 0);
-    if (r < R) {
-      S.segApp[r] = a;
-      S.segDead[r] = d;
-    }
+    if (r < R) S.segApp[r] = a;
   }
   for (long long i = tid; i < P.nIns; i += T) P.mask[i] = __ldcg(S.bits + S.entrySlot[P.nDel + i]);
   // (a CTA's range in whole groups of four vertices)
   const long long per = ((static_cast<long long>(n) + gridDim.x - 1) / gridDim.x + 3) / 4 * 4;
   const long long lo = per * blockIdx.x < n ? per * blockIdx.x : n;
   const long long hi = lo + per < n ? lo + per : n;
+  // (and of the blocks)
+  const long long blocks = (m + 31LL) / 32;
+  const long long bPer = (blocks + gridDim.x - 1) / gridDim.x;
+  const long long bLo = bPer * blockIdx.x < blocks ? bPer * blockIdx.x : blocks;
+  const long long bHi = bLo + bPer < blocks ? bLo + bPer : blocks;
   {
     long long local = 0;
     for (long long v = lo + 4LL * threadIdx.x; v < hi; v += 4LL * blockDim.x) {
@@ -298,7 +333,13 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
       local += d.x + d.y + d.z + d.w;
     }
     const long long sum = blockSum(local);
-    if (threadIdx.x == 0) S.blockSums[blockIdx.x] = sum;
+    local = 0;
+    for (long long b = bLo + threadIdx.x; b < bHi; b += blockDim.x) local += __ldcg(&S.block[b].shift);
+    const long long moves = blockSum(local);
+    if (threadIdx.x == 0) {
+      S.blockSums[blockIdx.x] = sum;
+      S.moveSums[blockIdx.x] = moves;
+    }
   }
   if (!gridSync(c, epoch)) return;
 
@@ -306,18 +347,10 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
   for (long long s = tid; s < S.slots; s += T) {
     const u64 key = __ldcg(S.key + s);
     if (key == kNoKey) continue;
-    const int u = static_cast<int>(key >> 32), v = static_cast<int>(key);
     const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s);
-    const int r = __ldcg(S.rowSlot + u) - 1;
     if (occ <= cD && __ldcg(S.cI + s) > 0) {
+      const int r = __ldcg(S.rowSlot + static_cast<int>(key >> 32)) - 1;
       S.app[__ldcg(S.segApp + r) + atomicAdd(S.curApp + r, 1)] = __ldcg(S.firstIns + s);
-    }
-    // the first min(occ, cD) occurrences go
-    int left = occ < cD ? occ : cD;
-    for (int e = __ldcg(S.first + s); left > 0; ++e) {
-      if (__ldg(P.col + e) != v) continue;
-      S.dead[__ldcg(S.segDead + r) + atomicAdd(S.curDead + r, 1)] = e;
-      --left;
     }
   }
   {
@@ -349,46 +382,45 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
       S.result->newM = static_cast<int>(m + all);
     }
   }
+  // ---- where the blocks of the copy begin -----------------------------------
+  {
+    long long before = 0;
+    for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += blockDim.x) before += __ldcg(S.moveSums + b);
+    long long carry = blockSum(before);
+    for (long long t = bLo; t < bHi; t += blockDim.x) {
+      const long long b = t + threadIdx.x;
+      long long tile;
+      const long long incl = carry + blockInclusiveScan(b < bHi ? __ldcg(&S.block[b].shift) : 0, &tile);
+      if (b < bHi) S.block[b].shift = static_cast<int>(incl);
+      carry += tile;
+    }
+  }
 }
 
-/// edgeRow that also gives the row's start and how far the row moves: the
-/// window loads the offsets of its rows in both graphs, so the search and
-/// what the copy needs of the row are one round trip.
-__device__ __forceinline__ int edgeRowMove(const int *row, const int *newRow, int n, long long e, bool in,
-                                           int &r0, int &start, int &shift) {
-  int found = in ? -1 : r0;
-  for (int base = r0; base < n; base += 32) {
-    const int rr = base + static_cast<int>(laneId());
-    const int a = rr < n ? __ldg(row + rr) : 0;
-    const int moved = rr < n ? __ldcg(newRow + rr) - a : 0;
-    const int end = rr < n ? __ldg(row + rr + 1) : INT_MAX;
-    int at = 0;  // rows of the window that end at or before the edge
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-      if (__shfl_sync(kFull, end, at + step - 1) <= e) at += step;
-    }
-    const int lastEnd = __shfl_sync(kFull, end, 31);
-    const int src = at < 32 ? at : 31;
-    const int st = __shfl_sync(kFull, a, src), mv = __shfl_sync(kFull, moved, src);
-    if (found < 0 && e < lastEnd) {
-      found = base + at;
-      start = st;
-      shift = mv;
-    }
-    if (__all_sync(kFull, found >= 0)) break;
-  }
-  r0 = __shfl_sync(kFull, found, 31);  // the largest; past the chunk the caller ends
-  return found;
+/// How far edge e of row u moves, where its block is one that goes by rows.
+__device__ __forceinline__ int moveByRow(const ApplyParams &P, const Block &B, int u, int e) {
+  const int e0 = e & ~31, start = __ldg(P.row + u);
+  unsigned gone = B.dead & ((1u << (e & 31)) - 1u);
+  if (start <= e0) return B.shift - __popc(gone);
+  gone &= ~((1u << (start - e0)) - 1u);
+  return __ldcg(P.newRow + u) - start - __popc(gone);
+}
+
+/// The same for a block with at most one appended edge at each place.
+__device__ __forceinline__ int moveByBits(const Block &B, int bit) {
+  return B.shift - __popc(B.dead & ((1u << bit) - 1u)) + __popc(B.app & ((2u << bit) - 1u));
 }
 
 /// The copy: every edge to its new place, appended edges behind their rows.
-/// A launch of its own, with half again as many warps as the persistent one
-/// can hold: it waits for memory.
-__global__ void __launch_bounds__(kCopyThreads, 5)
+/// A launch of its own: small CTAs, so that one that has run out of edges makes
+/// room, and its own share of the registers for the loads in flight (the call on
+/// 5.56M edges, K = 3: 217 us with the rows of 32 edges searched, 160 without).
+__global__ void __launch_bounds__(kCopyThreads, 4)
 copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedScratch S, EngineControl *c,
           int stats) {
   __shared__ unsigned long long sSum[kMaxK];
   __shared__ int sMax[kMaxK];
+  __shared__ int sMove[kCopyThreads / 32][kCopyEdges];
   if (__ldcg(&c->status) != 0 || __ldcg(&c->invalid) != 0) return;
   const int n = static_cast<int>(P.n), m = static_cast<int>(P.m), K = P.K;
   const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -405,81 +437,77 @@ copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedSc
   const int myK = static_cast<int>(lane) % K;
   long long sum = 0;
   int most = 1;
-  EdgeChunks chunks(m, tid >> 5, T >> 5, &c->chunkNext);
-  long long wb, we;
-  int r0;
-  while (chunks.take(P.row, n, wb, we, r0)) {
-    // removed edges of the current row before the current 32
-    int carry = 0;
-    {
-      const int r = __ldcg(S.rowSlot + r0) - 1;
-      const int d = r >= 0 && __ldg(P.row + r0) < wb ? __ldcg(S.nDead + r) : 0;
-      const int *list = S.dead + (d > 0 ? __ldcg(S.segDead + r) : 0);
-      for (int i = static_cast<int>(lane); i < d; i += 32) carry += __ldcg(list + i) < wb;
-      carry = __reduce_add_sync(kFull, carry);
+  const int step = span / K;                      // edges a turn moves
+  const int ownEdge = static_cast<int>(lane) / K;  // this lane's among them
+  int *moves = sMove[threadIdx.x >> 5];
+  for (long long e0 = (tid >> 5) * kCopyEdges; e0 < m; e0 += (T >> 5) * kCopyEdges) {
+    const int edges = static_cast<int>(m - e0 < kCopyEdges ? m - e0 : kCopyEdges);
+    const int *src = P.w + e0 * K;
+    const int ints = static_cast<int>(lane) < span ? edges * K : 0;
+    int w[kTurns];
+#pragma unroll
+    for (int q = 0; q < kTurns; ++q) {
+      const int i = q * span + static_cast<int>(lane);
+      w[q] = i < ints ? __ldg(src + i) : 0;
     }
-    for (long long e0 = wb; e0 < we; e0 += 32) {
-      const int e = static_cast<int>(e0 + lane);
-      const bool in = e0 + lane < we;
-      const int col = in ? __ldg(P.col + e) : 0;
-      // (chunks start at multiples of 32)
-      const unsigned hits = __ldcg(S.hit + (e0 >> 5));
-      // the first turns' weights are requested before the rows are searched
-      const int edges = static_cast<int>(we - e0 < 32 ? we - e0 : 32);
-      const int *src = P.w + e0 * K;
-      int early[kEarly];
+    int col[kCopyEdges / 32];
+    Block B[kCopyEdges / 32];
 #pragma unroll
-      for (int q = 0; q < kEarly; ++q) {
-        const int i = q * span + static_cast<int>(lane);
-        early[q] = static_cast<int>(lane) < span && i < edges * K ? __ldg(src + i) : 0;
-      }
-      int start = 0, moved = 0;
-      const int u = edgeRowMove(P.row, P.newRow, n, e, in, r0, start, moved);
-      bool live = in;
-      int other = -1;      // the insertion whose weights the edge takes
-      if (in && ((hits >> lane) & 1u)) {
-        const int g = findGroup(S, u, col);
-        const int cD = __ldcg(S.cD + g);
-        int before = 0;    // occurrences before this one
-        for (int x = __ldcg(S.first + g); x < e; ++x) before += __ldg(P.col + x) == col;
-        live = before >= cD;
-        if (before == cD && __ldcg(S.cI + g) > 0) other = __ldcg(S.lastIns + g);
-      }
-      const unsigned dead = __ballot_sync(kFull, in && !live);
-      const int from = start > e0 ? static_cast<int>(start - e0) : 0;  // the row's first lane
-      const unsigned mine = ((1u << lane) - 1u) & ~((1u << from) - 1u);
-      const int less = (start < e0 ? carry : 0) + __popc(dead & mine);
-      // new position, or -1
-      const int to = live ? e + moved - less : -1;
-      carry = __shfl_sync(kFull, less + (in && !live ? 1 : 0), 31);
-      if (to >= 0) P.newCol[to] = col;
-      const long long shift = static_cast<long long>(to - e) * K;
-      const bool plain = to >= 0 && other < 0;
-      auto move = [&](int base, int w) {  // all lanes call it
-        const int i = base + static_cast<int>(lane);
-        const bool has = static_cast<int>(lane) < span && i < edges * K;
-        const int owner = has ? i / K : 0;
-        const long long sh = __shfl_sync(kFull, shift, owner);
-        const int ok = __shfl_sync(kFull, static_cast<int>(plain), owner);
-        if (!has) return;
-        sum += w;
-        most = w > most ? w : most;
-        if (ok) P.newW[e0 * K + i + sh] = w;
-      };
+    for (int j = 0; j < kCopyEdges / 32; ++j) {
+      const int i = 32 * j + static_cast<int>(lane);
+      col[j] = i < edges ? __ldg(P.col + e0 + i) : 0;
+      const int4 b = 32 * j < edges ? __ldcg(reinterpret_cast<const int4 *>(S.block + (e0 >> 5) + j))
+                                    : make_int4(0, 0, 0, 0);
+      B[j] = Block{b.x, static_cast<unsigned>(b.y), static_cast<unsigned>(b.z), static_cast<unsigned>(b.w)};
+    }
 #pragma unroll
-      for (int q = 0; q < kEarly; ++q) {
-        if (q * span < edges * K) move(q * span, early[q]);
+    for (int j = 0; j < kCopyEdges / 32; ++j) {
+      const int i = 32 * j + static_cast<int>(lane);
+      const int e = static_cast<int>(e0) + i;
+      int move = moveByBits(B[j], static_cast<int>(lane));
+      if (B[j].app == kByRows) {
+        // (the same for the whole warp; 32 j < edges, as the rest is zero)
+        int r0 = chunkRow(P.row, n, e0 + 32 * j);
+        const int u = edgeRow(P.row, n, e, i < edges, r0);
+        move = i < edges ? moveByRow(P, B[j], u, e) : 0;
       }
-      for (int base = kEarly * span; base < edges * K; base += span) {
-        const int i = base + static_cast<int>(lane);
-        move(base, static_cast<int>(lane) < span && i < edges * K ? __ldg(src + i) : 0);
+      const bool stays = i < edges && ((B[j].dead >> lane) & 1u) == 0;
+      if (stays) P.newCol[e + move] = col[j];
+      moves[i] = stays && ((B[j].other >> lane) & 1u) == 0 ? move * K : kNoMove;
+    }
+    __syncwarp();
+    int *dst = P.newW + e0 * K;
+    for (int t = 0; t * step < edges; t += kTurns) {
+#pragma unroll
+      for (int q = 0; q < kTurns; ++q) {
+        const int i = (t + q) * span + static_cast<int>(lane);
+        if (i < ints) {
+          sum += w[q];
+          most = w[q] > most ? w[q] : most;
+          const int move = moves[(t + q) * step + ownEdge];
+          if (move != kNoMove) dst[i + static_cast<long long>(move)] = w[q];
+        }
       }
-      if (to >= 0 && other >= 0) {
-        for (int k = 0; k < K; ++k) {
-          P.newW[static_cast<long long>(to) * K + k] = __ldg(P.insW + static_cast<long long>(other) * K + k);
+      if ((t + kTurns) * step < edges) {
+#pragma unroll
+        for (int q = 0; q < kTurns; ++q) {
+          const int i = (t + kTurns + q) * span + static_cast<int>(lane);
+          w[q] = i < ints ? __ldg(src + i) : 0;
         }
       }
     }
+    __syncwarp();
+  }
+  // the insertions' weights of edges that stay
+  const int others = __ldcg(S.counts + 3);
+  for (long long a = tid; a < others; a += T) {
+    const int2 o = __ldcg(S.other + a);
+    const int4 b = __ldcg(reinterpret_cast<const int4 *>(S.block + (o.x >> 5)));
+    const Block B{b.x, static_cast<unsigned>(b.y), static_cast<unsigned>(b.z), static_cast<unsigned>(b.w)};
+    const int u = static_cast<int>(__ldcg(S.key + o.y) >> 32);
+    const long long to = o.x + (B.app == kByRows ? moveByRow(P, B, u, o.x) : moveByBits(B, o.x & 31));
+    const long long last = __ldcg(S.lastIns + o.y);
+    for (int k = 0; k < K; ++k) P.newW[to * K + k] = __ldg(P.insW + last * K + k);
   }
   // appended edges, at the end of their row in the order of their groups'
   // first insertions
@@ -540,13 +568,14 @@ unsigned char *layout(unsigned char *p, long long n, long long m, long long nIns
   S.bits = carve<unsigned>(p, S.slots);
   S.filterBits = std::min(8 * S.slots, 1u << 20);
   S.filter = carve<unsigned>(p, S.filterBits / 32);
-  for (int **x : {&S.entrySlot, &S.rows, &S.nApp, &S.nDead, &S.segApp, &S.segDead, &S.curApp, &S.curDead}) {
+  for (int **x : {&S.entrySlot, &S.rows, &S.nApp, &S.segApp, &S.curApp}) {
     *x = carve<int>(p, B);
   }
   S.pieces = carve<u64>(p, m / kPiece + B);
-  S.hit = carve<unsigned>(p, (m + 31) / 32);
+  S.block = carve<Block>(p, (m + 31) / 32 + 1);
+  S.moveSums = carve<long long>(p, kMaxCtas);
   S.app = carve<int>(p, nIns);
-  S.dead = carve<int>(p, nDel);
+  S.other = carve<int2>(p, nIns);
   S.rowSlot = carve<int>(p, n + 4);
   S.delta = carve<int>(p, n + 4);
   return p;
@@ -566,7 +595,7 @@ cudaError_t applyFusedShape(int sms, int ctasPerSm, int &ctas) {
   if (err != cudaSuccess) return err;
   if (perSm < 1) return cudaErrorInvalidConfiguration;
   if (ctasPerSm > 0 && ctasPerSm < perSm) perSm = ctasPerSm;
-  ctas = perSm * sms;
+  ctas = std::min(perSm * sms, kMaxCtas);
   return cudaSuccess;
 }
 
@@ -584,7 +613,7 @@ cudaError_t applyBatchFused(const ApplyParams &P, void *scratch, EngineControl *
                                     0, s);
   if (err == cudaSuccess) {
     const long long want = (std::max(P.m, static_cast<long long>(P.nIns)) + kCopyThreads - 1) / kCopyThreads;
-    const int grid = static_cast<int>(std::min(std::max(want, 1LL), 5LL * ctas));
+    const int grid = static_cast<int>(std::min(std::max(want, 1LL), 4LL * ctas));
     copyFused<<<grid, kCopyThreads, 0, s>>>(P, S, ctl, stats ? 1 : 0);
     err = cudaGetLastError();
   }

@@ -144,6 +144,22 @@ __device__ long long blockSum(long long x) {
 // per warp would leave half of the grid idle on power-law graphs: where rows
 // are short a slice takes several times as long.
 // ---------------------------------------------------------------------------
+/// The last row that starts at or before edge e: 32 probes a step, so five
+/// dependent loads for a million rows where halving takes twenty. All lanes
+/// call it.
+__device__ __forceinline__ int chunkRow(const int *outRow, int n, long long e) {
+  int row = 0;
+  for (int hi = n; hi - row > 1;) {
+    const int mid = row + static_cast<int>(static_cast<long long>(hi - row) * (laneId() + 1) / 33);
+    const int below = __popc(__ballot_sync(kFull, __ldg(outRow + mid) <= e));
+    const int lo = __shfl_sync(kFull, mid, below > 0 ? below - 1 : 0);
+    const int up = __shfl_sync(kFull, mid, below < 32 ? below : 31);
+    if (below < 32) hi = up;
+    if (below > 0) row = lo;
+  }
+  return row;
+}
+
 struct EdgeChunks {
   long long size, m, nwarps;
   long long mine;  // the warp's first chunk; the others come off the counter
@@ -172,17 +188,7 @@ struct EdgeChunks {
     wb = size * i;
     we = wb + size < m ? wb + size : m;
     if (wb >= we) return false;
-    // the last row that starts at or before wb: 32 probes a step, so five
-    // dependent loads for a million rows where halving takes twenty
-    row = 0;
-    for (int hi = n; hi - row > 1;) {
-      const int mid = row + static_cast<int>(static_cast<long long>(hi - row) * (laneId() + 1) / 33);
-      const int below = __popc(__ballot_sync(kFull, __ldg(outRow + mid) <= wb));
-      const int lo = __shfl_sync(kFull, mid, below > 0 ? below - 1 : 0);
-      const int up = __shfl_sync(kFull, mid, below < 32 ? below : 31);
-      if (below < 32) hi = up;
-      if (below > 0) row = lo;
-    }
+    row = chunkRow(outRow, n, wb);
     return true;
   }
 };

@@ -98,3 +98,26 @@ def test_no_edges():
     check(np.zeros(6, np.int32), np.zeros(0, np.int32), np.zeros((0, 2), np.int32),
           {"ins_from": np.array([4, 0, 4]), "ins_to": np.array([1, 2, 1]),
            "ins_w": np.array([[3, 4], [5, 6], [7, 8]]), "del_from": np.array([2]), "del_to": np.array([3])})
+
+
+@pytest.mark.parametrize("every", [1, 2, 5])
+@pytest.mark.parametrize("last", [0, 1, 31])
+@pytest.mark.parametrize("degrees", [[1] * 96, [32] * 4, [0, 0, 0, 16] * 10, [31, 1, 0, 33, 0, 0, 63, 65], [130, 0, 0]])
+def test_moves_within_blocks_of_edges(degrees, last, every):
+    """Appended, removed and overwritten edges at every place of the copy's
+    blocks of 32: an append before each edge of a block, rows that end at a
+    block's end, several appends at one place (also through empty rows), a
+    last block of 1, 31 and 32 edges."""
+    rng = np.random.default_rng(1000 * every + 10 * last + len(degrees))
+    degrees = degrees + [last]
+    n, K = len(degrees) + 200, 3
+    row, col = rows_of(degrees + [0] * 200, n, rng, 0)
+    w = rng.integers(1, 1000, (len(col), K)).astype(np.int32)
+    tail = np.repeat(np.arange(n), np.diff(row))
+    rows = np.repeat(np.arange(0, len(degrees), every), 1 + (every == 5))  # one or two per row
+    take = np.arange(0, len(col), 7)
+    batch = {"ins_from": np.concatenate([rows, tail[take + (take + 1 < len(col))]]),
+             "ins_to": np.concatenate([rng.integers(0, n, len(rows)), col[take + (take + 1 < len(col))]]),
+             "del_from": tail[take], "del_to": col[take]}
+    batch["ins_w"] = rng.integers(1, 900, (len(batch["ins_from"]), K))
+    check(row, col, w, batch)
