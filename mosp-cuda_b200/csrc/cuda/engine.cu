@@ -3211,8 +3211,20 @@ __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBas
 // balanced over edges. (With rows dealt to warps, the
 // one that held the low ids of an R-MAT graph walked most of its hubs: 3.9M
 // edges, K = 4: 4.13 -> 0.36 ms; 16.1M, K = 3: 11.2 -> 1.8 ms; road network
-// of 5.6M edges, K = 3: 0.24 -> 0.22 ms.)
+// of 5.6M edges, K = 3: 0.24 -> 0.20 ms.)
+//
+// Once the reverse arrays outgrow L2, every scattered 4-byte store is a
+// 32-byte sector read and written in HBM, K + 1 times per edge. There the
+// scatter writes one number per edge, whose array stays in L2 for longer, and
+// a second pass gathers the edge's K adjacent weights and stores in order:
+// 3.9M edges, K = 4: 0.36 -> 0.30 ms; 16.1M, K = 3: 1.74 -> 0.95; 65M, K = 5:
+// 18.3 -> 8.8. The rule's line: R-MAT graphs with K = 3 take 0.163 and 0.174 ms
+// (direct, by order) at 31 MB of reverse arrays, 0.317 and 0.290 at 63 MB;
+// 16.1M edges with K = 1 0.744 and 0.741; road networks, whose stores stay
+// close, are the same within 2 % on either side.
 // ---------------------------------------------------------------------------
+constexpr long long kScatterBytes = 48LL << 20;
+
 __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant__ BuildParams B) {
   EngineControl *c = B.ctl;
   const int n = B.n, m = B.m, K = B.K;
@@ -3277,7 +3289,9 @@ __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant_
   }
   if (!gridSync(c, epoch)) return;
 
-  // fill: edge e of row u goes to position rank[e] of its head's row
+  // fill: edge e of row u goes to position rank[e] of its head's row, or
+  // (byOrder) leaves its number there, and its row in place of the rank
+  const bool byOrder = K > 1 && 4LL * m * (K + 1) > kScatterBytes;
   EdgeChunks chunks(m, tid >> 5, nwarps, &c->chunkNext);
   long long wb, we;
   int r0;
@@ -3289,10 +3303,38 @@ __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant_
       const int pos = in ? __ldcg(B.inRow + x) + __ldcg(B.rank + e) : 0;
       const int row = edgeRow(B.outRow, n, e, in, r0);
       if (!in) continue;
+      if (byOrder) {
+        B.inCol[pos] = static_cast<int>(e);
+        B.rank[e] = row;
+        continue;
+      }
       B.inCol[pos] = row;
       for (int k = 0; k < K; ++k) {
         B.inW[static_cast<long long>(k) * m + pos] = __ldg(B.edgeMajorW + e * K + k);
       }
+    }
+  }
+  if (!byOrder) return;
+  if (!gridSync(c, epoch)) return;
+  // the reverse rows in order, four edges per thread in flight
+  for (long long i0 = tid; i0 < m; i0 += 4 * T) {
+    int e[4], row[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = i0 + q * T < m ? __ldcg(B.inCol + i0 + q * T) : 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row[q] = __ldcg(B.rank + e[q]);
+    for (int k = 0; k < K; ++k) {
+      int w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[q] = __ldg(B.edgeMajorW + static_cast<long long>(e[q]) * K + k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (i0 + q * T < m) B.inW[static_cast<long long>(k) * m + i0 + q * T] = w[q];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (i0 + q * T < m) B.inCol[i0 + q * T] = row[q];
     }
   }
 }

@@ -53,6 +53,14 @@ def test_reverse_csr(n, m, K, hub, gaps):
     assert np.array_equal(got[np.lexsort(got.T[::-1])], exp[np.lexsort(exp.T[::-1])])
 
 
+@pytest.mark.parametrize("n,m,K,hub,gaps", [(100001, 1400003, 8, True, False), (900001, 1500000, 8, False, True),
+                                            (100001, 2700000, 4, False, False), (50000, 8000000, 2, False, False)])
+def test_reverse_csr_larger_than_l2_keeps(n, m, K, hub, gaps):
+    """Reverse arrays of more than 48 MB, which are stored in order."""
+    assert 4 * m * (K + 1) > 48 << 20
+    test_reverse_csr(n, m, K, hub, gaps)
+
+
 @pytest.mark.parametrize("high", [False, True])
 @pytest.mark.parametrize("K", [1, 4, 5, 8, 9])
 def test_full_recovery(K, high):
