@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -57,12 +58,14 @@ struct mosp_workspace {
   // engine lists: kCap objectives x nCap vertices
   long long nCap = 0;
   int kCap = 0;
+  unsigned char *listSlab = nullptr;  // holds the next seven
   u64 *packed = nullptr;
   int *val = nullptr, *stamp = nullptr, *inFar = nullptr, *cand = nullptr;
   int *far0 = nullptr, *far1 = nullptr;
   // near lists (vertex, distance tag): kCap objectives x nearCap entries
   long long nearCap = 0;
   int nearK = 0;
+  unsigned char *nearSlab = nullptr;  // holds the next four
   int *nearV0 = nullptr, *nearV1 = nullptr;
   u64 *nearD0 = nullptr, *nearD1 = nullptr;
   int *gen = nullptr;  // device stamp generation
@@ -98,6 +101,7 @@ struct mosp_workspace {
   int blockSumsCap = 0;
   // combined graph
   long long combN = 0, combEdgesCap = 0;
+  unsigned char *combSlab = nullptr, *combEdgeSlab = nullptr;  // rows, edges
   int *combDeg = nullptr, *combRow = nullptr, *combCol = nullptr, *combW = nullptr;
   // reverse-CSR build: in-degrees and edge ranks
   long long cursorCap = 0;
@@ -105,6 +109,7 @@ struct mosp_workspace {
   // path costs
   long long costN = 0;
   int costKG = 0;
+  unsigned char *costSlab = nullptr;  // holds the next five
   int *edgeOf = nullptr, *anc0 = nullptr, *anc1 = nullptr;
   long long *acc0 = nullptr, *acc1 = nullptr;
   // per-launch timing (mosp_workspace_enable_timing)
@@ -166,11 +171,37 @@ int deviceAlloc(T **ptr, size_t count) {
   return MOSP_OK;
 }
 
-void releaseNear(mosp_workspace *ws) {
-  for (void *p : {static_cast<void *>(ws->nearV0), static_cast<void *>(ws->nearV1),
-                  static_cast<void *>(ws->nearD0), static_cast<void *>(ws->nearD1)}) {
-    if (p) cudaFree(p);
+struct Part {
+  void **ptr;
+  size_t bytes;
+};
+template <typename T>
+Part part(T *&ptr, size_t count) {
+  return {reinterpret_cast<void **>(&ptr), count * sizeof(T)};
+}
+
+/// Several arrays in one allocation, each from a 256-byte boundary: an
+/// allocation takes 0.35 ms and its release 0.28 ms whatever the size, which was
+/// most of a workspace's first call (update of 60,001 vertices: 6.8 -> 2.9 ms).
+int deviceAllocParts(unsigned char **slab, std::initializer_list<Part> parts) {
+  size_t bytes = 0;
+  for (const Part &p : parts) {
+    *p.ptr = nullptr;
+    bytes += (p.bytes + 255) / 256 * 256;
   }
+  const int st = deviceAlloc(slab, bytes);
+  if (st != MOSP_OK) return st;
+  unsigned char *at = *slab;
+  for (const Part &p : parts) {
+    *p.ptr = at;
+    at += (p.bytes + 255) / 256 * 256;
+  }
+  return MOSP_OK;
+}
+
+void releaseNear(mosp_workspace *ws) {
+  if (ws->nearSlab) cudaFree(ws->nearSlab);
+  ws->nearSlab = nullptr;
   ws->nearV0 = ws->nearV1 = nullptr;
   ws->nearD0 = ws->nearD1 = nullptr;
   ws->nearCap = 0;
@@ -189,12 +220,8 @@ void releaseAsync(mosp_workspace *ws) {
 }
 
 void releaseLists(mosp_workspace *ws) {
-  for (void *p : {static_cast<void *>(ws->packed), static_cast<void *>(ws->val),
-                  static_cast<void *>(ws->stamp), static_cast<void *>(ws->inFar),
-                  static_cast<void *>(ws->cand), static_cast<void *>(ws->far0),
-                  static_cast<void *>(ws->far1)}) {
-    if (p) cudaFree(p);
-  }
+  if (ws->listSlab) cudaFree(ws->listSlab);
+  ws->listSlab = nullptr;
   ws->packed = nullptr;
   ws->val = ws->stamp = ws->inFar = ws->cand = nullptr;
   ws->far0 = ws->far1 = nullptr;
@@ -250,11 +277,9 @@ int reserveNear(mosp_workspace *ws, long long n, long long m, int K) {
   const int kk = std::max(K, ws->nearK);
   releaseNear(ws);
   const size_t total = static_cast<size_t>(cap) * kk;
-  int st = MOSP_OK;
-  if ((st = deviceAlloc(&ws->nearV0, total)) != MOSP_OK) return st;
-  if ((st = deviceAlloc(&ws->nearV1, total)) != MOSP_OK) return st;
-  if ((st = deviceAlloc(&ws->nearD0, total)) != MOSP_OK) return st;
-  if ((st = deviceAlloc(&ws->nearD1, total)) != MOSP_OK) return st;
+  const int st = deviceAllocParts(&ws->nearSlab, {part(ws->nearD0, total), part(ws->nearD1, total),
+                                                  part(ws->nearV0, total), part(ws->nearV1, total)});
+  if (st != MOSP_OK) return st;
   ws->nearCap = cap;
   ws->nearK = kk;
   return MOSP_OK;
@@ -304,15 +329,10 @@ int reserveLists(mosp_workspace *ws, long long n, int K) {
   const int newK = std::max(K, ws->kCap);
   releaseLists(ws);
   const size_t total = static_cast<size_t>(newN) * newK;
-  int st = MOSP_OK;
-  if ((st = deviceAlloc(&ws->packed, total)) != MOSP_OK) return st;
-  for (int **p : {&ws->val, &ws->stamp, &ws->inFar, &ws->cand, &ws->far0, &ws->far1}) {
-    const bool pile = p == &ws->far0 || p == &ws->far1;
-    if ((st = deviceAlloc(p, pile ? kFarCopies * total : total)) != MOSP_OK) {
-      releaseLists(ws);
-      return st;
-    }
-  }
+  const int st = deviceAllocParts(
+      &ws->listSlab, {part(ws->packed, total), part(ws->val, total), part(ws->stamp, total), part(ws->inFar, total),
+                      part(ws->cand, total), part(ws->far0, kFarCopies * total), part(ws->far1, kFarCopies * total)});
+  if (st != MOSP_OK) return st;
   MOSP_CUDA(cudaMemset(ws->stamp, 0, total * sizeof(int)));
   MOSP_CUDA(cudaMemset(ws->inFar, 0, total * sizeof(int)));
   MOSP_CUDA(cudaMemset(ws->gen, 0, sizeof(int)));
@@ -352,14 +372,18 @@ int maybeResetGenerations(mosp_workspace *ws, int finalGen, cudaStream_t s) {
 int reserveCombined(mosp_workspace *ws, long long n, int K) {
   int st = MOSP_OK;
   if (n > ws->combN) {
-    if ((st = deviceAlloc(&ws->combDeg, n + 1)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->combRow, n + 1)) != MOSP_OK) return st;
+    ws->combN = 0;
+    if ((st = deviceAllocParts(&ws->combSlab, {part(ws->combDeg, n + 1), part(ws->combRow, n + 1)})) != MOSP_OK) {
+      return st;
+    }
     ws->combN = n;
   }
   const long long edges = n * K;
   if (edges > ws->combEdgesCap) {
-    if ((st = deviceAlloc(&ws->combCol, edges)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->combW, edges)) != MOSP_OK) return st;
+    ws->combEdgesCap = 0;
+    if ((st = deviceAllocParts(&ws->combEdgeSlab, {part(ws->combCol, edges), part(ws->combW, edges)})) != MOSP_OK) {
+      return st;
+    }
     ws->combEdgesCap = edges;
   }
   return MOSP_OK;
@@ -847,12 +871,9 @@ void mosp_workspace_destroy(mosp_workspace *ws) {
   if (ws->device >= 0) cudaSetDevice(ws->device);
   releaseLists(ws);
   for (void *p : {static_cast<void *>(ws->ctl), static_cast<void *>(ws->gen),
-                  static_cast<void *>(ws->blockSums), static_cast<void *>(ws->combDeg),
-                  static_cast<void *>(ws->combRow), static_cast<void *>(ws->combCol),
-                  static_cast<void *>(ws->combW), static_cast<void *>(ws->cursor),
-                  static_cast<void *>(ws->edgeOf), static_cast<void *>(ws->anc0),
-                  static_cast<void *>(ws->anc1), static_cast<void *>(ws->acc0),
-                  static_cast<void *>(ws->acc1), static_cast<void *>(ws->recMark),
+                  static_cast<void *>(ws->blockSums), static_cast<void *>(ws->combSlab),
+                  static_cast<void *>(ws->combEdgeSlab), static_cast<void *>(ws->cursor),
+                  static_cast<void *>(ws->costSlab), static_cast<void *>(ws->recMark),
                   static_cast<void *>(ws->recVerts), static_cast<void *>(ws->recChunks),
                   static_cast<void *>(ws->recDist)}) {
     if (p) cudaFree(p);
@@ -1615,11 +1636,11 @@ int mosp_path_costs(mosp_workspace *ws, int n, int m, int KG, const int *d_out_r
   if (n > ws->costN || KG > ws->costKG) {
     const long long nn = std::max<long long>(n, ws->costN);
     const int kk = std::max(KG, ws->costKG);
-    if ((st = deviceAlloc(&ws->edgeOf, nn)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->anc0, nn)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->anc1, nn)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->acc0, nn * kk)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->acc1, nn * kk)) != MOSP_OK) return st;
+    ws->costN = 0;
+    if ((st = deviceAllocParts(&ws->costSlab, {part(ws->acc0, nn * kk), part(ws->acc1, nn * kk), part(ws->edgeOf, nn),
+                                               part(ws->anc0, nn), part(ws->anc1, nn)})) != MOSP_OK) {
+      return st;
+    }
     ws->costN = nn;
     ws->costKG = kk;
   }
