@@ -1552,7 +1552,10 @@ __device__ __noinline__ int chaseRecords(const EngineParams &P, bool donate, int
   // shared memory per hop costs 70 ns of it on a bare chain
   unsigned done = 0;
   for (unsigned hops = 1;; ++hops) {
-    if ((hops & 4095u) == 0 && (ldShared(&C.abort) != 0 || globalNs() > C.deadline)) {
+    // (one verdict for the warp: lanes may read the clock and the flag
+    // differently, and one that left alone would keep the others waiting at
+    // the next ballot)
+    if ((hops & 4095u) == 0 && __any_sync(kFull, ldShared(&C.abort) != 0 || globalNs() > C.deadline)) {
       atomicCAS(&P.ctl->status, 0, MOSP_ERR_TIMEOUT);
       stShared(&C.abort, 1);
       break;
@@ -1721,16 +1724,18 @@ __device__ __forceinline__ int asyncWait(const EngineParams &P, const Sync &sync
     }
     if (wait) {
       unsigned turns = 0;
+      bool came = true;
       while (!barTryWait(&C.bar[warp], parity)) {
         ++turns;
-        if (ldShared(&C.abort) != 0) break;
-        if ((turns & 255u) == 0 && globalNs() > sync.deadline + 1000000000ULL) {
-          asyncAbort(P);
+        if ((turns & 255u) == 0 && globalNs() > sync.deadline + 1000000000ULL) asyncAbort(P);
+        if (ldShared(&C.abort) != 0) {
+          came = false;
           break;
         }
       }
       parity ^= 1u;
-      mail = ldShared(&C.mail[warp]);
+      // (who gives up has no mail: its count and slots may hold anything)
+      if (came) mail = ldShared(&C.mail[warp]);
     }
   }
   parity = __shfl_sync(kFull, parity, 0);
