@@ -1301,6 +1301,7 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
     if (lane == 0) {
       __threadfence();
       stShared(&C.over, 1);
+      __threadfence_block();  // over before the look at the idle warps
     }
     __syncwarp();
     wakeAll();
@@ -1818,6 +1819,7 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
       const int mail = asyncWait(P, sync, parity);
       if constexpr (Rec) {
         if (mail > 0) {
+          __syncwarp();  // lane 0's wait orders the mail for the others too
           owed += mail;
           const int q = static_cast<int>(lane >> 2);
           u64 base = 0;
@@ -1831,7 +1833,8 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
             t = reinterpret_cast<const int *>(&h.wts)[lane & 3u];
             if ((lane & 3u) == 0) atomicAdd(&C.expanded[k], 1u);
           }
-          __syncwarp();
+          // (every lane's edge goes into the first hop's ballot, so the slots
+          // are read before lane 0 can call the warp idle again)
           farCount = chaseRecords<Mode>(P, donate, farCount, k, v, base, x, t);
         }
       }
