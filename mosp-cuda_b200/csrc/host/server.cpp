@@ -21,13 +21,13 @@
 //     may allocate (CSR growth, Step 1 scratch, staging) fits in the free
 //     device memory minus a reserve, unless nothing else is running;
 //   * overlap on the device: with W > 1 workers each worker's persistent
-//     cooperative launches (graph build, update, combined graph, costs) use
-//     at most SMs / W CTAs of one SM each, so the grids of W passes fit on
-//     the GPU side by side and run at the same time on disjoint SMs (each
-//     grid waits at its barriers only for its own CTAs). Full-grid work
+//     cooperative launches (Step 1, graph build, update, combined graph,
+//     costs) use at most SMs / W CTAs of one SM each, so the grids of W passes
+//     fit on the GPU side by side and run at the same time on disjoint SMs
+//     (each grid waits at its barriers only for its own CTAs). Full-grid work
 //     (adding a graph, or all passes when overlap is off) takes the engine
-//     lock exclusively; passes take it shared. Host work, copies and Step 1
-//     kernels of all workers overlap with the engine launches.
+//     lock exclusively; passes take it shared (DeviceTurn). Host work and
+//     copies of all workers overlap with the launches.
 // A response carries the graph's combined tree after the pass that included
 // the request and the version (number of batches applied to the graph) of
 // that state; equal versions give equal results however the batches were
@@ -348,6 +348,26 @@ struct mosp_server {
     return best;
   }
 
+  /// A pass's turn on the device, held around its cooperative launches: the
+  /// workspace's grids are limited to this worker's share of the SMs and the
+  /// engine lock is shared, or the grids are full and the lock is exclusive.
+  struct DeviceTurn {
+    std::shared_lock<std::shared_mutex> shared;
+    std::unique_lock<std::shared_mutex> whole;
+    DeviceTurn(mosp_server &srv, mosp_workspace *ws)
+        : shared(srv.gpuLock, std::defer_lock), whole(srv.gpuLock, std::defer_lock) {
+      const bool side = srv.overlap && srv.workers > 1;
+      int sms = 0;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, srv.device);
+      mosp_workspace_set_grid(ws, side ? std::max(1, sms / srv.workers) : 0, 0);
+      if (side) {
+        shared.lock();
+      } else {
+        whole.lock();
+      }
+    }
+  };
+
   void worker(int index);
   int runPass(mosp_workspace *ws, cudaStream_t s, Staging &st, Graph &g,
               std::vector<std::shared_ptr<Request>> &group, std::string &err);
@@ -464,11 +484,14 @@ int mosp_server::runPass(mosp_workspace *ws, cudaStream_t s, Staging &st, Graph 
     const int o = 1 - g.cur;
     int newM = 0;
     long long amx[MOSP_MAX_OBJECTIVES], asum[MOSP_MAX_OBJECTIVES];
-    rc = mosp_apply_batch_device(ws, n, KG, static_cast<int>(g.m), g.row[g.cur], g.col[g.cur],
-                                 g.w[g.cur], static_cast<int>(nIns), st.insFrom.p, st.insTo.p,
-                                 st.insW.p, static_cast<int>(nDel), st.delFrom.p, st.delTo.p,
-                                 g.row[o], g.col[o], g.w[o], g.edgeCap, &newM, st.mask.p, amx, asum,
-                                 s);
+    {
+      const DeviceTurn turn(*this, ws);
+      rc = mosp_apply_batch_device(ws, n, KG, static_cast<int>(g.m), g.row[g.cur], g.col[g.cur],
+                                   g.w[g.cur], static_cast<int>(nIns), st.insFrom.p, st.insTo.p,
+                                   st.insW.p, static_cast<int>(nDel), st.delFrom.p, st.delTo.p,
+                                   g.row[o], g.col[o], g.w[o], g.edgeCap, &newM, st.mask.p, amx, asum,
+                                   s);
+    }
     if (rc != MOSP_OK) {
       err = mosp_last_error();
       return rc;
@@ -536,19 +559,7 @@ int mosp_server::runPass(mosp_workspace *ws, cudaStream_t s, Staging &st, Graph 
   for (int k = 0; k < K; ++k) delta[k] = mosp_default_delta(g.m, n, g.weightSum[k]);
   const Clock::time_point tEngine = Clock::now();
   {
-    std::shared_lock<std::shared_mutex> shared(gpuLock, std::defer_lock);
-    std::unique_lock<std::shared_mutex> whole(gpuLock, std::defer_lock);
-    // with overlap, this worker's share of the SMs for its cooperative
-    // grids, so that every worker's grids fit on the GPU together
-    const bool side = overlap && workers > 1;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    mosp_workspace_set_grid(ws, side ? std::max(1, sms / workers) : 0, 0);
-    if (side) {
-      shared.lock();
-    } else {
-      whole.lock();
-    }
+    const DeviceTurn turn(*this, ws);
     if (enginesActive.fetch_add(1) > 0) {
       std::lock_guard<std::mutex> lk(mu);
       ++stats.overlapped;
