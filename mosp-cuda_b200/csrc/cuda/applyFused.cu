@@ -96,15 +96,16 @@ __device__ __forceinline__ unsigned filterBit(const FusedScratch &S, unsigned ha
 }
 
 /// Edges b, b + step, ... (< end) of touched row u: occurrences of their
-/// groups. Four at a time, their loads and probes in flight together.
-__device__ __forceinline__ void countOccurrences(const ApplyParams &P, const FusedScratch &S, int u, int b,
-                                                 int end, int step) {
-  for (int e0 = b; e0 < end; e0 += 4 * step) {
+/// groups. Four at a time, their loads and probes in flight together. (Edges
+/// past the end of a row count up to 2^31 + 127: unsigned.)
+__device__ __forceinline__ void countOccurrences(const ApplyParams &P, const FusedScratch &S, int u, unsigned b,
+                                                 unsigned end, unsigned step) {
+  for (unsigned e0 = b; e0 < end; e0 += 4 * step) {
     u64 key[4], at[4];
     unsigned s[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int e = e0 + q * step;
+      const unsigned e = e0 + q * step;
       key[q] = (static_cast<u64>(static_cast<unsigned>(u)) << 32) |
                static_cast<unsigned>(e < end ? __ldg(P.col + e) : -1);
       s[q] = hashOf(key[q]);
@@ -128,9 +129,9 @@ __device__ __forceinline__ void countOccurrences(const ApplyParams &P, const Fus
         at[q] = __ldcg(S.key + s[q]);
       }
       if (at[q] == kNoKey) continue;
-      const int e = e0 + q * step;
+      const unsigned e = e0 + q * step;
       atomicAdd(S.occ + s[q], 1);
-      atomicMin(S.first + s[q], e);
+      atomicMin(S.first + s[q], static_cast<int>(e));
     }
   }
 }
@@ -170,7 +171,7 @@ __device__ __forceinline__ void resolveGroup(const ApplyParams &P, const FusedSc
   if (appended) {
     const int r = __ldcg(S.rowSlot + u) - 1;
     atomicAdd(S.nApp + r, 1);
-    const int e = __ldg(P.row + u + 1);
+    const unsigned e = __ldg(P.row + u + 1);
     atomicAdd(&S.block[(e + 31) >> 5].shift, 1);
     if ((e & 31) != 0) {
       const unsigned bit = 1u << (e & 31);
@@ -269,7 +270,7 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
     }
     const int r = warpReserve(S.counts + 0, newRow ? 1 : 0);
     const int deg = newRow ? __ldg(P.row + u + 1) - __ldg(P.row + u) : 0;
-    const int mine = deg > kLaneRow ? (deg + kPiece - 1) / kPiece : 0;
+    const int mine = deg > kLaneRow ? static_cast<int>((deg + kPiece - 1u) / kPiece) : 0;
     const int at = warpReserve(S.counts + 1, mine);
     if (newRow) {
       S.rows[r] = u;
@@ -295,7 +296,7 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
     const int u = static_cast<int>(piece >> 32);
     const int b = __ldg(P.row + u) + static_cast<int>(piece) * kPiece;
     const int end = __ldg(P.row + u + 1);
-    countOccurrences(P, S, u, b + static_cast<int>(lane), end < b + kPiece ? end : b + kPiece, 32);
+    countOccurrences(P, S, u, b + lane, end - b < kPiece ? end : b + kPiece, 32);
   }
   if (!gridSync(c, epoch)) return;
 
@@ -463,13 +464,13 @@ copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedSc
 #pragma unroll
     for (int j = 0; j < kCopyEdges / 32; ++j) {
       const int i = 32 * j + static_cast<int>(lane);
-      const int e = static_cast<int>(e0) + i;
+      const long long e = e0 + i;
       int move = moveByBits(B[j], static_cast<int>(lane));
       if (B[j].app == kByRows) {
         // (the same for the whole warp; 32 j < edges, as the rest is zero)
         int r0 = chunkRow(P.row, n, e0 + 32 * j);
         const int u = edgeRow(P.row, n, e, i < edges, r0);
-        move = i < edges ? moveByRow(P, B[j], u, e) : 0;
+        move = i < edges ? moveByRow(P, B[j], u, static_cast<int>(e)) : 0;
       }
       const bool stays = i < edges && ((B[j].dead >> lane) & 1u) == 0;
       if (stays) P.newCol[e + move] = col[j];

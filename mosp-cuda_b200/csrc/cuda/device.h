@@ -200,8 +200,8 @@ struct EdgeChunks {
 __device__ __forceinline__ int edgeRow(const int *outRow, int n, long long e, bool in, int &r0) {
   int row = in ? -1 : r0;
   for (int base = r0; base < n; base += 32) {
-    const int rr = base + static_cast<int>(laneId());
-    const int end = rr < n ? __ldg(outRow + rr + 1) : INT_MAX;
+    const unsigned rr = base + laneId();  // (past INT_MAX for the last rows)
+    const int end = rr < static_cast<unsigned>(n) ? __ldg(outRow + rr + 1) : INT_MAX;
     int at = 0;  // rows of the window that end at or before the edge
 #pragma unroll
     for (int step = 16; step >= 1; step >>= 1) {
