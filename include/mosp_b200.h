@@ -129,8 +129,9 @@ void mosp_workspace_destroy(mosp_workspace *ws);
  * (no-op if large enough). */
 int mosp_workspace_reserve(mosp_workspace *ws, int n, int K);
 
-/* mosp_workspace_reserve plus everything the near-far loops of graphs with
- * up to m edges need (near lists, the asynchronous loop's spill queue and row records), so that
+/* mosp_workspace_reserve plus everything that mosp_build_device_graph and
+ * the near-far loops need on graphs with up to m edges (the build's scratch,
+ * near lists, the asynchronous loop's spill queue and row records), so that
  * later calls on such graphs allocate nothing in the workspace (e.g. a
  * serving loop reserves before its first request). */
 int mosp_workspace_reserve_graph(mosp_workspace *ws, int n, long long m, int K);

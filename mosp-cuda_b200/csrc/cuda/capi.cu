@@ -389,6 +389,24 @@ int reserveCombined(mosp_workspace *ws, long long n, int K) {
   return MOSP_OK;
 }
 
+/// Scratch of the reverse-CSR build: in-degrees and edge ranks. A resident
+/// graph gains edges from batch to batch, so it grows by half again (a
+/// reallocation's cudaFree waits for the whole device).
+int reserveBuild(mosp_workspace *ws, long long n, long long m) {
+  const long long need = n + 1 + m;
+  if (need <= ws->cursorCap) return MOSP_OK;
+  const long long want = std::max(need, ws->cursorCap + ws->cursorCap / 2);
+  ws->cursorCap = 0;
+  int st = MOSP_OK;
+  for (const long long size : {want, need}) {
+    if ((st = deviceAlloc(&ws->cursor, size)) == MOSP_OK) {
+      ws->cursorCap = size;
+      break;
+    }
+  }
+  return st;
+}
+
 cudaStream_t asStream(void *s) { return static_cast<cudaStream_t>(s); }
 
 /// Bits of the parent field and the distance bound (reference
@@ -910,6 +928,7 @@ int mosp_workspace_reserve_graph(mosp_workspace *ws, int n, long long m, int K) 
   // the update's near lists and queue, and those of the combined step
   if ((st = reserveNear(ws, nn, std::max(m, nn * K), K)) != MOSP_OK) return st;
   if ((st = reserveAsync(ws, nn, K)) != MOSP_OK) return st;
+  if ((st = reserveBuild(ws, nn, m)) != MOSP_OK) return st;
   // (a batch may leave a graph with fewer edges)
   reserveRecords(ws, recordsPay(nn, m - m / 8) ? K : 1);
   return MOSP_OK;
@@ -1101,12 +1120,7 @@ int mosp_build_device_graph(mosp_workspace *ws, int n, int m, int K, const int *
                  d_in_col == nullptr || d_in_w == nullptr))) {
     return fail(MOSP_ERR_INVALID, "Error: invalid device graph arguments.");
   }
-  if (static_cast<long long>(n) + 1 + m > ws->cursorCap) {
-    const long long need = static_cast<long long>(n) + 1 + m;
-    ws->cursorCap = 0;
-    if ((st = deviceAlloc(&ws->cursor, need)) != MOSP_OK) return st;
-    ws->cursorCap = need;
-  }
+  if ((st = reserveBuild(ws, n, m)) != MOSP_OK) return st;
   cudaStream_t s = asStream(stream);
   BuildParams b{};
   b.n = n;

@@ -322,6 +322,8 @@ struct mosp_server {
     const long long edges = g.m + ins;
     if (edges > g.edgeCap) bytes += 2 * edges * (8 + 4LL * g.KG);
     if (edges > g.derivedCap) bytes += edges * (4 + 8LL * g.KG);
+    // the build's scratch, past what the workers have reserved
+    if (edges > maxM + kPassChanges) bytes += 6LL * (g.n + edges);
     return bytes;
   }
 
