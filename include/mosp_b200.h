@@ -130,10 +130,13 @@ void mosp_workspace_destroy(mosp_workspace *ws);
 int mosp_workspace_reserve(mosp_workspace *ws, int n, int K);
 
 /* mosp_workspace_reserve plus everything that mosp_build_device_graph and
- * the near-far loops need on graphs with up to m edges (the build's scratch,
- * near lists, the asynchronous loop's spill queue and row records), so that
- * later calls on such graphs allocate nothing in the workspace (e.g. a
- * serving loop reserves before its first request). */
+ * the updates need on graphs with up to m edges (the build's scratch, near
+ * lists, the asynchronous loop's spill queue and row records, the full parent
+ * recovery's distances), so that later builds and updates of such graphs
+ * allocate nothing in the workspace (e.g. a serving loop reserves before its
+ * first request). Not covered: the scratch of a change batch and of path
+ * costs, and with mosp_workspace_set_canonical_trees the restricted
+ * recovery's lists, which the first call that needs them allocates. */
 int mosp_workspace_reserve_graph(mosp_workspace *ws, int n, long long m, int K);
 
 /* Batched instances: many independent graphs stored as one disjoint union

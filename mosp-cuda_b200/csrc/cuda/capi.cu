@@ -665,6 +665,18 @@ struct UpdateArgs {
 };
 
 /// Build the parameters of a fused K-objective update.
+/// The full parent recovery's distances side by side, for `count`
+/// objectives; without room for them (false) it reads the objectives' own
+/// arrays.
+bool reserveRecDist(mosp_workspace *ws, long long n, long long count) {
+  const long long need = n * (count <= 4 ? 1 : (count + 7) / 8 * 2);
+  if (need > ws->recDistCap) {
+    ws->recDistCap = 0;
+    if (deviceAlloc(&ws->recDist, need) == MOSP_OK) ws->recDistCap = need;
+  }
+  return need <= ws->recDistCap;
+}
+
 /// Buffers of the restricted parent recovery: per objective and vertex of
 /// the engine lists one mark byte and two list slots (the changed and the
 /// scan list), and two chunk lists with room for every chunk of every row
@@ -744,14 +756,7 @@ int prepareUpdate(mosp_workspace *ws, const UpdateArgs &a, EngineParams &p, int 
     p.recChunkList = ws->recChunks;
     p.recChunkCap = static_cast<int>(ws->recChunkCap);
   } else if (const long long fall = std::count(bitsOut, bitsOut + a.K, 0)) {
-    // the full recovery's distances side by side; without room for them it
-    // reads the objectives' own arrays
-    const long long need = static_cast<long long>(a.n) * (fall <= 4 ? 1 : (fall + 7) / 8 * 2);
-    if (need > ws->recDistCap) {
-      ws->recDistCap = 0;
-      if (deviceAlloc(&ws->recDist, need) == MOSP_OK) ws->recDistCap = need;
-    }
-    if (need <= ws->recDistCap) p.recDist = ws->recDist;
+    if (reserveRecDist(ws, a.n, fall)) p.recDist = ws->recDist;
   }
   return MOSP_OK;
 }
@@ -929,8 +934,10 @@ int mosp_workspace_reserve_graph(mosp_workspace *ws, int n, long long m, int K) 
   if ((st = reserveNear(ws, nn, std::max(m, nn * K), K)) != MOSP_OK) return st;
   if ((st = reserveAsync(ws, nn, K)) != MOSP_OK) return st;
   if ((st = reserveBuild(ws, nn, m)) != MOSP_OK) return st;
-  // (a batch may leave a graph with fewer edges)
-  reserveRecords(ws, recordsPay(nn, m - m / 8) ? K : 1);
+  // (a graph with fewer edges may take records where m edges do not, and one
+  // with larger weights recovers its parents)
+  reserveRecords(ws, K);
+  if (!ws->canonicalTrees) reserveRecDist(ws, nn, K);
   return MOSP_OK;
 }
 

@@ -52,3 +52,40 @@ def test_builds_of_a_growing_graph():
         # (growth by half again: 10.1, 15.2, 22.7 and 34.1 million entries)
         assert len(seen) == (1 if reserved else 1 + math.ceil(math.log((n + m) / (n + m0), 1.5)))
         ws.close()
+
+
+def update_of(ws, n, m, K, max_weight, gen):
+    """K trees of a random graph, then an update without changes, which leaves
+    them."""
+    col, w, (out_w, in_row, in_col, in_w) = device_graph(n, m, K, gen)
+    row = rows_of(n, m)
+    dist = torch.zeros(K * n, dtype=torch.int64, device="cuda")
+    par = torch.zeros(K * n, dtype=torch.int32, device="cuda")
+    cd, cp = torch.zeros(n, dtype=torch.int64, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")
+    none = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ws.build_device_graph(n, m, K, row, col, w, out_w, in_row, in_col, in_w)
+    for k in range(K):
+        ws.sosp_from_scratch(n, m, row, col, out_w[k * m:], 0, 100, max_weight, dist[k * n:], par[k * n:])
+    want = dist.clone(), par.clone()
+    ws.update_device(n, m, K, row, col, out_w, in_row, in_col, in_w, none, none, [0] * (K + 1), none, 0, 0,
+                     [100] * K, [max_weight] * K, None, dist, par, cd, cp)
+    assert torch.equal(dist, want[0]) and torch.equal(par, want[1])
+
+
+@pytest.mark.parametrize("max_weight", [100, 1 << 30])
+def test_sparser_graph_than_reserved(max_weight):
+    """Reserved for 5 edges per vertex, where the loop takes no row records;
+    updates of graphs with 4 and 2 (records), with parents beside the distances
+    and recovered after them."""
+    n, m, K = 10 ** 6, 5 * 10 ** 6, 2
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    update_of(mb.Workspace(timeout_ms=20000), 1000, 3000, K, max_weight, gen)  # kernels and caches are loaded
+    ws = mb.Workspace(timeout_ms=20000)
+    mb.check(mb.lib().mosp_workspace_reserve_graph(ws._h, n, m, K))
+    for edges in (m, 4 * n, 2 * n):
+        pool = torch.zeros(1 << 27, dtype=torch.int64, device="cuda")
+        del pool  # (kept by torch, which takes the graph and the trees from it)
+        before = free_bytes()
+        update_of(ws, n, edges, K, max_weight, gen)
+        assert free_bytes() == before
+    ws.close()
