@@ -58,6 +58,13 @@ struct mosp_workspace {
   // engine lists: kCap objectives x nCap vertices
   long long nCap = 0;
   int kCap = 0;
+  // entries per vertex and objective of a far pile: kFarCopies, which the
+  // asynchronous loop needs, or 1 (it is off, or the device was full)
+  int farCopies = 0;
+  // the device was too full for the far piles, the records, the recovery's
+  // distances, the build's ranks: not tried again before the next larger size
+  bool farShort = false, recShort = false, recDistShort = false;
+  long long rankShort = 0;
   unsigned char *listSlab = nullptr;  // holds the next seven
   u64 *packed = nullptr;
   int *val = nullptr, *stamp = nullptr, *inFar = nullptr, *cand = nullptr;
@@ -103,7 +110,7 @@ struct mosp_workspace {
   long long combN = 0, combEdgesCap = 0;
   unsigned char *combSlab = nullptr, *combEdgeSlab = nullptr;  // rows, edges
   int *combDeg = nullptr, *combRow = nullptr, *combCol = nullptr, *combW = nullptr;
-  // reverse-CSR build: in-degrees and edge ranks
+  // reverse-CSR build: in-degrees and (where there is room) edge ranks
   long long cursorCap = 0;
   int *cursor = nullptr;
   // path costs
@@ -227,8 +234,66 @@ void releaseLists(mosp_workspace *ws) {
   ws->far0 = ws->far1 = nullptr;
   ws->nCap = 0;
   ws->kCap = 0;
+  ws->farCopies = 0;
+  ws->recShort = ws->recDistShort = false;
   releaseNear(ws);
   releaseAsync(ws);
+}
+
+/// The engine lists of nCap vertices and kCap objectives, cleared.
+int makeLists(mosp_workspace *ws, long long n, int K, int copies) {
+  const size_t total = static_cast<size_t>(n) * K;
+  const int st = deviceAllocParts(
+      &ws->listSlab, {part(ws->packed, total), part(ws->val, total), part(ws->stamp, total), part(ws->inFar, total),
+                      part(ws->cand, total), part(ws->far0, copies * total), part(ws->far1, copies * total)});
+  if (st != MOSP_OK) return st;
+  MOSP_CUDA(cudaMemset(ws->stamp, 0, total * sizeof(int)));
+  MOSP_CUDA(cudaMemset(ws->inFar, 0, total * sizeof(int)));
+  MOSP_CUDA(cudaMemset(ws->gen, 0, sizeof(int)));
+  MOSP_CUDA(cudaStreamSynchronize(nullptr));  // (the launches' streams may not wait for this one)
+  ws->nCap = n;
+  ws->kCap = K;
+  ws->farCopies = copies;
+  return MOSP_OK;
+}
+
+/// On a full device: gives back the arrays that only make calls faster (row
+/// records, the recovery's distances, the build's ranks), the second time the
+/// asynchronous loop's far piles and queue. False when there is nothing left
+/// to give. The launch parameters are filled in after the last allocation of
+/// a call, and every call waits for its launches.
+bool makeRoom(mosp_workspace *ws) {
+  bool any = false;
+  for (void *p : {static_cast<void *>(ws->rec), static_cast<void *>(ws->recDist), static_cast<void *>(ws->cursor)}) {
+    any = any || p != nullptr;
+    if (p) cudaFree(p);
+  }
+  ws->rec = ws->recDist = nullptr;
+  ws->cursor = nullptr;
+  ws->recCap = ws->recDistCap = ws->cursorCap = 0;
+  if (any) return true;
+  if (ws->farCopies <= 1) return false;
+  if (ws->aqSlots) cudaFree(ws->aqSlots);
+  ws->aqSlots = nullptr;
+  ws->aqCap = 0;
+  ws->farShort = true;
+  if (makeLists(ws, ws->nCap, ws->kCap, 1) == MOSP_OK) return true;
+  releaseLists(ws);
+  return false;
+}
+
+/// Allocations that a call cannot do without.
+template <typename T>
+int alloc(mosp_workspace *ws, T **ptr, size_t count) {
+  int st = deviceAlloc(ptr, count);
+  while (st == MOSP_ERR_OOM && makeRoom(ws)) st = deviceAlloc(ptr, count);
+  return st;
+}
+
+int allocParts(mosp_workspace *ws, unsigned char **slab, std::initializer_list<Part> parts) {
+  int st = deviceAllocParts(slab, parts);
+  while (st == MOSP_ERR_OOM && makeRoom(ws)) st = deviceAllocParts(slab, parts);
+  return st;
 }
 
 /// CTAs of a persistent launch whose occupancy-sized grid is `full`: that
@@ -251,7 +316,7 @@ int ensureShape(mosp_workspace *ws) {
   const int maxCtas = std::max({ws->shape.engineCtas, ws->shape.buildCtas, ws->shape.costCtas,
                                 ws->shape.applyCtas});
   if (maxCtas > ws->blockSumsCap) {
-    int st = deviceAlloc(&ws->blockSums, maxCtas);
+    int st = alloc(ws, &ws->blockSums, maxCtas);
     if (st != MOSP_OK) return st;
     ws->blockSumsCap = maxCtas;
   }
@@ -277,8 +342,8 @@ int reserveNear(mosp_workspace *ws, long long n, long long m, int K) {
   const int kk = std::max(K, ws->nearK);
   releaseNear(ws);
   const size_t total = static_cast<size_t>(cap) * kk;
-  const int st = deviceAllocParts(&ws->nearSlab, {part(ws->nearD0, total), part(ws->nearD1, total),
-                                                  part(ws->nearV0, total), part(ws->nearV1, total)});
+  const int st = allocParts(ws, &ws->nearSlab, {part(ws->nearD0, total), part(ws->nearD1, total),
+                                                part(ws->nearV0, total), part(ws->nearV1, total)});
   if (st != MOSP_OK) return st;
   ws->nearCap = cap;
   ws->nearK = kk;
@@ -297,19 +362,25 @@ long long asyncSlotsFor(long long n, int K, long long fixed = 0) {
 }
 
 int reserveAsync(mosp_workspace *ws, long long n, int K) {
-  if (ws->asyncMode == 0) return MOSP_OK;
+  if (ws->asyncMode == 0 || ws->farCopies < kFarCopies) return MOSP_OK;
   int st = MOSP_OK;
   if (ws->aqCtr == nullptr) {
-    if ((st = deviceAlloc(&ws->aqCtr, 3 * kAsyncShards)) != MOSP_OK) return st;
+    if ((st = alloc(ws, &ws->aqCtr, 3 * kAsyncShards)) != MOSP_OK) return st;
   }
   const long long need = asyncSlotsFor(n, K, ws->asyncSlots);
   if (need == ws->aqCap && ws->aqSlots != nullptr) return MOSP_OK;
   if (ws->asyncSlots == 0 && need < ws->aqCap && ws->aqSlots != nullptr) return MOSP_OK;
-  if ((st = deviceAlloc(&ws->aqSlots, need)) != MOSP_OK) {
-    ws->aqCap = 0;
-    return st;
+  ws->aqCap = 0;
+  st = alloc(ws, &ws->aqSlots, need);
+  if (ws->farCopies < kFarCopies) {
+    // (the room for it came from the loop's own far piles: the bulk loop runs)
+    if (ws->aqSlots) cudaFree(ws->aqSlots);
+    ws->aqSlots = nullptr;
+    return MOSP_OK;
   }
+  if (st != MOSP_OK) return st;
   MOSP_CUDA(cudaMemset(ws->aqSlots, 0xff, need * sizeof(u64)));
+  MOSP_CUDA(cudaStreamSynchronize(nullptr));
   ws->aqCap = need;
   return MOSP_OK;
 }
@@ -318,26 +389,24 @@ int reserveAsync(mosp_workspace *ws, long long n, int K) {
 /// the loop faster: a launch without room for them runs without.
 void reserveRecords(mosp_workspace *ws, int K) {
   const long long need = 2 * ws->nCap * K;
-  if (ws->asyncMode == 0 || need <= ws->recCap) return;
+  if (ws->asyncMode == 0 || ws->farCopies < kFarCopies || need <= ws->recCap || ws->recShort) return;
   ws->recCap = 0;
   if (deviceAlloc(&ws->rec, need) == MOSP_OK) ws->recCap = need;
+  ws->recShort = ws->recCap == 0;
 }
 
 int reserveLists(mosp_workspace *ws, long long n, int K) {
-  if (n <= ws->nCap && K <= ws->kCap) return MOSP_OK;
+  const bool fits = n <= ws->nCap && K <= ws->kCap;
+  const int want = ws->asyncMode != 0 ? kFarCopies : 1;
+  if (fits && (ws->farCopies >= want || ws->farShort)) return MOSP_OK;
   const long long newN = std::max(n, ws->nCap);
   const int newK = std::max(K, ws->kCap);
   releaseLists(ws);
-  const size_t total = static_cast<size_t>(newN) * newK;
-  const int st = deviceAllocParts(
-      &ws->listSlab, {part(ws->packed, total), part(ws->val, total), part(ws->stamp, total), part(ws->inFar, total),
-                      part(ws->cand, total), part(ws->far0, kFarCopies * total), part(ws->far1, kFarCopies * total)});
+  int st = makeLists(ws, newN, newK, want);
+  while (st == MOSP_ERR_OOM && makeRoom(ws)) st = makeLists(ws, newN, newK, want);
+  if (st == MOSP_ERR_OOM && want > 1) st = makeLists(ws, newN, newK, 1);
   if (st != MOSP_OK) return st;
-  MOSP_CUDA(cudaMemset(ws->stamp, 0, total * sizeof(int)));
-  MOSP_CUDA(cudaMemset(ws->inFar, 0, total * sizeof(int)));
-  MOSP_CUDA(cudaMemset(ws->gen, 0, sizeof(int)));
-  ws->nCap = newN;
-  ws->kCap = newK;
+  ws->farShort = ws->farCopies < want;
   ws->dirty = false;
   return MOSP_OK;
 }
@@ -373,7 +442,7 @@ int reserveCombined(mosp_workspace *ws, long long n, int K) {
   int st = MOSP_OK;
   if (n > ws->combN) {
     ws->combN = 0;
-    if ((st = deviceAllocParts(&ws->combSlab, {part(ws->combDeg, n + 1), part(ws->combRow, n + 1)})) != MOSP_OK) {
+    if ((st = allocParts(ws, &ws->combSlab, {part(ws->combDeg, n + 1), part(ws->combRow, n + 1)})) != MOSP_OK) {
       return st;
     }
     ws->combN = n;
@@ -381,7 +450,7 @@ int reserveCombined(mosp_workspace *ws, long long n, int K) {
   const long long edges = n * K;
   if (edges > ws->combEdgesCap) {
     ws->combEdgesCap = 0;
-    if ((st = deviceAllocParts(&ws->combEdgeSlab, {part(ws->combCol, edges), part(ws->combW, edges)})) != MOSP_OK) {
+    if ((st = allocParts(ws, &ws->combEdgeSlab, {part(ws->combCol, edges), part(ws->combW, edges)})) != MOSP_OK) {
       return st;
     }
     ws->combEdgesCap = edges;
@@ -389,22 +458,27 @@ int reserveCombined(mosp_workspace *ws, long long n, int K) {
   return MOSP_OK;
 }
 
-/// Scratch of the reverse-CSR build: in-degrees and edge ranks. A resident
-/// graph gains edges from batch to batch, so it grows by half again (a
-/// reallocation's cudaFree waits for the whole device).
+/// Scratch of the reverse-CSR build: in-degrees and, where there is room,
+/// edge ranks. A resident graph gains edges from batch to batch, so it grows
+/// by half again (a reallocation's cudaFree waits for the whole device).
 int reserveBuild(mosp_workspace *ws, long long n, long long m) {
   const long long need = n + 1 + m;
   if (need <= ws->cursorCap) return MOSP_OK;
+  if (ws->rankShort > 0 && need >= ws->rankShort && n + 1 <= ws->cursorCap) return MOSP_OK;
   const long long want = std::max(need, ws->cursorCap + ws->cursorCap / 2);
   ws->cursorCap = 0;
-  int st = MOSP_OK;
+  ws->rankShort = 0;
   for (const long long size : {want, need}) {
-    if ((st = deviceAlloc(&ws->cursor, size)) == MOSP_OK) {
+    if (deviceAlloc(&ws->cursor, size) == MOSP_OK) {
       ws->cursorCap = size;
-      break;
+      return MOSP_OK;
     }
   }
-  return st;
+  const int st = alloc(ws, &ws->cursor, n + 1);
+  if (st != MOSP_OK) return st;
+  ws->cursorCap = n + 1;
+  ws->rankShort = need;
+  return MOSP_OK;
 }
 
 cudaStream_t asStream(void *s) { return static_cast<cudaStream_t>(s); }
@@ -467,7 +541,7 @@ void fillLists(EngineParams &p, mosp_workspace *ws, int block) {
   // asynchronous loop unless it is off or the graph last seen here had hub
   // rows; its launches need a smaller stage (the pull pass stays staged up
   // to K tiles), which leaves more of the SM's memory to L1
-  const bool async = ws->asyncMode != 0 && ws->aqSlots != nullptr &&
+  const bool async = ws->asyncMode != 0 && ws->aqSlots != nullptr && ws->farCopies == kFarCopies &&
                      ws->aqCap >= asyncSlotsFor(p.n, p.K, ws->asyncSlots) &&
                      !ws->heavySeen[block == 1 ? 1 : 0];
   if (async) {
@@ -484,6 +558,7 @@ void fillLists(EngineParams &p, mosp_workspace *ws, int block) {
   } else {
     p.stageEntries = kStageEntriesMax;
   }
+  if (p.recDist != nullptr) p.recDist = ws->recDist;  // (given back since: null)
   p.timeoutNs = ws->timeoutNs;
   p.genPtr = ws->gen;
   p.packed = ws->packed;
@@ -499,7 +574,7 @@ void fillLists(EngineParams &p, mosp_workspace *ws, int block) {
   p.farL0 = ws->far0;
   p.farL1 = ws->far1;
   p.stride = ws->nCap;
-  p.strideFar = kFarCopies * ws->nCap;
+  p.strideFar = ws->farCopies * ws->nCap;
   p.ctl = ws->ctl + block;
   p.blockSums = ws->blockSums;
 }
@@ -670,9 +745,10 @@ struct UpdateArgs {
 /// arrays.
 bool reserveRecDist(mosp_workspace *ws, long long n, long long count) {
   const long long need = n * (count <= 4 ? 1 : (count + 7) / 8 * 2);
-  if (need > ws->recDistCap) {
+  if (need > ws->recDistCap && !ws->recDistShort) {
     ws->recDistCap = 0;
     if (deviceAlloc(&ws->recDist, need) == MOSP_OK) ws->recDistCap = need;
+    ws->recDistShort = ws->recDistCap == 0;
   }
   return need <= ws->recDistCap;
 }
@@ -688,15 +764,15 @@ int reserveRecovery(mosp_workspace *ws, long long m, int K) {
   if (marks > ws->recMarkCap) {
     ws->recMarkCap = 0;
     // whole 32-bit words: the marks are set with atomicOr on their word
-    if ((st = deviceAlloc(&ws->recMark, (marks + 3) / 4 * 4)) != MOSP_OK) return st;
-    if ((st = deviceAlloc(&ws->recVerts, 2 * marks)) != MOSP_OK) return st;
+    if ((st = alloc(ws, &ws->recMark, (marks + 3) / 4 * 4)) != MOSP_OK) return st;
+    if ((st = alloc(ws, &ws->recVerts, 2 * marks)) != MOSP_OK) return st;
     ws->recMarkCap = marks;
   }
   const long long chunks = static_cast<long long>(K) * (m / kRecLightRow + 1) + 64;
   if (chunks > INT_MAX) return fail(MOSP_ERR_INVALID, "Error: graph too large for the parent recovery lists.");
   if (chunks > ws->recChunkCap) {
     ws->recChunkCap = 0;
-    if ((st = deviceAlloc(&ws->recChunks, 2 * chunks)) != MOSP_OK) return st;
+    if ((st = alloc(ws, &ws->recChunks, 2 * chunks)) != MOSP_OK) return st;
     ws->recChunkCap = chunks;
   }
   return MOSP_OK;
@@ -958,7 +1034,7 @@ int mosp_workspace_set_sources(mosp_workspace *ws, const int *h_sources, int cou
   ws->nSources = 0;
   ws->hostSources.clear();
   if (count <= 1) return MOSP_OK;
-  if ((st = deviceAlloc(&ws->sources, count)) != MOSP_OK) return st;
+  if ((st = alloc(ws, &ws->sources, count)) != MOSP_OK) return st;
   MOSP_CUDA(cudaMemcpy(ws->sources, roots.data(), count * sizeof(int), cudaMemcpyHostToDevice));
   ws->hostSources = std::move(roots);
   ws->nSources = count;
@@ -996,6 +1072,7 @@ int mosp_workspace_set_async(mosp_workspace *ws, int on, long long queue_slots) 
   }
   ws->asyncMode = on;
   ws->asyncSlots = queue_slots;
+  ws->farShort = false;
   return MOSP_OK;
 }
 
@@ -1062,7 +1139,7 @@ int mosp_workspace_buffer(mosp_workspace *ws, int slot, unsigned long long bytes
   if (bytes > ws->userBytes[slot] || ws->user[slot] == nullptr) {
     char *p = static_cast<char *>(ws->user[slot]);
     const unsigned long long grow = std::max(bytes, ws->userBytes[slot] + ws->userBytes[slot] / 8);
-    if ((st = deviceAlloc(&p, grow)) != MOSP_OK) {
+    if ((st = alloc(ws, &p, grow)) != MOSP_OK) {
       ws->user[slot] = nullptr;
       ws->userBytes[slot] = 0;
       return st;
@@ -1142,7 +1219,7 @@ int mosp_build_device_graph(mosp_workspace *ws, int n, int m, int K, const int *
   b.inCol = d_in_col;
   b.inW = d_in_w;
   b.cursor = ws->cursor;
-  b.rank = ws->cursor + n + 1;
+  b.rank = static_cast<long long>(n) + 1 + m <= ws->cursorCap ? ws->cursor + n + 1 : nullptr;
   b.blockSums = ws->blockSums;
   b.ctl = ws->ctl + 2;
   MOSP_CUDA(cudaMemsetAsync(ws->ctl + 2, 0, sizeof(EngineControl), s));
@@ -1188,7 +1265,7 @@ int mosp_apply_batch_device(mosp_workspace *ws, int n, int K, int m, const int *
     ws->applyScratch = nullptr;
     ws->applyBytes = 0;
     unsigned char *p = nullptr;
-    if ((st = deviceAlloc(&p, want)) != MOSP_OK) return st;
+    if ((st = alloc(ws, &p, want)) != MOSP_OK) return st;
     ws->applyScratch = p;
     ws->applyBytes = want;
   }
@@ -1478,8 +1555,8 @@ int mosp_autotune_update(mosp_workspace *ws, int n, int m, int K, const int *d_o
   // trial and at the end
   long long *saveDist = nullptr;
   int *saveParent = nullptr;
-  if ((st = deviceAlloc(&saveDist, kn)) != MOSP_OK) return st;
-  if ((st = deviceAlloc(&saveParent, kn)) != MOSP_OK) {
+  if ((st = alloc(ws, &saveDist, kn)) != MOSP_OK) return st;
+  if ((st = alloc(ws, &saveParent, kn)) != MOSP_OK) {
     cudaFree(saveDist);
     return st;
   }
@@ -1658,7 +1735,7 @@ int mosp_path_costs(mosp_workspace *ws, int n, int m, int KG, const int *d_out_r
     const long long nn = std::max<long long>(n, ws->costN);
     const int kk = std::max(KG, ws->costKG);
     ws->costN = 0;
-    if ((st = deviceAllocParts(&ws->costSlab, {part(ws->acc0, nn * kk), part(ws->acc1, nn * kk), part(ws->edgeOf, nn),
+    if ((st = allocParts(ws, &ws->costSlab, {part(ws->acc0, nn * kk), part(ws->acc1, nn * kk), part(ws->edgeOf, nn),
                                                part(ws->anc0, nn), part(ws->anc1, nn)})) != MOSP_OK) {
       return st;
     }

@@ -3260,6 +3260,8 @@ __device__ void scratchOrCombined(const EngineParams &P, Sync &epoch, int genBas
 // ---------------------------------------------------------------------------
 constexpr long long kScatterBytes = 48LL << 20;
 
+/// Ranked: B.rank is there.
+template <bool Ranked>
 __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant__ BuildParams B) {
   EngineControl *c = B.ctl;
   const int n = B.n, m = B.m, K = B.K;
@@ -3311,22 +3313,23 @@ __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant_
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const long long e = e0 + q * T;
-      if (e < m) B.rank[e] = r[q];
+      if (Ranked && e < m) B.rank[e] = r[q];
     }
   }
   if (bad) c->invalid = 1;
   if (!gridSync(c, epoch)) return;
   if (__ldcg(&c->invalid) != 0) return;
   long long total = 0;
-  if (!gridExclusiveScan(B.cursor, B.inRow, nullptr, static_cast<long long>(n) + 1, B.blockSums, c, epoch,
-                         &total)) {
+  if (!gridExclusiveScan(B.cursor, B.inRow, Ranked ? nullptr : B.cursor, static_cast<long long>(n) + 1, B.blockSums, c,
+                         epoch, &total)) {
     return;
   }
   if (!gridSync(c, epoch)) return;
 
   // fill: edge e of row u goes to position rank[e] of its head's row, or
-  // (byOrder) leaves its number there, and its row in place of the rank
-  const bool byOrder = K > 1 && 4LL * m * (K + 1) > kScatterBytes;
+  // (byOrder) leaves its number there, and its row in place of the rank;
+  // without ranks to the next position, by a second atomic
+  const bool byOrder = Ranked && K > 1 && 4LL * m * (K + 1) > kScatterBytes;
   EdgeChunks chunks(m, tid >> 5, nwarps, &c->chunkNext);
   long long wb, we;
   int r0;
@@ -3335,7 +3338,12 @@ __global__ void __launch_bounds__(kThreads, 1) buildGraph(const __grid_constant_
       const long long e = e0 + lane;
       const bool in = e < we;
       const int x = in ? __ldg(B.outCol + e) : 0;
-      const int pos = in ? __ldcg(B.inRow + x) + __ldcg(B.rank + e) : 0;
+      int pos = 0;
+      if constexpr (Ranked) {
+        pos = in ? __ldcg(B.inRow + x) + __ldcg(B.rank + e) : 0;
+      } else {
+        pos = in ? atomicAdd(B.cursor + x, 1) : 0;
+      }
       const int row = edgeRow(B.outRow, n, e, in, r0);
       if (!in) continue;
       if (byOrder) {
@@ -3612,8 +3620,9 @@ cudaError_t queryLaunchShape(int ctasPerSm, LaunchShape &shape) {
   if ((err = ctasFor(sospEngine<kModeScratch>, sms, ctasPerSm, b, kStageBytes)) != cudaSuccess) return err;
   if ((err = ctasFor(sospEngine<kModeCombined>, sms, ctasPerSm, d, kStageBytes)) != cudaSuccess) return err;
   shape.engineCtas = a < b ? (a < d ? a : d) : (b < d ? b : d);
-  if ((err = ctasFor(buildGraph, sms, ctasPerSm, e)) != cudaSuccess) return err;
-  shape.buildCtas = e;
+  if ((err = ctasFor(buildGraph<true>, sms, ctasPerSm, e)) != cudaSuccess) return err;
+  if ((err = ctasFor(buildGraph<false>, sms, ctasPerSm, a)) != cudaSuccess) return err;
+  shape.buildCtas = a < e ? a : e;
   if ((err = ctasFor(pathCosts, sms, ctasPerSm, e)) != cudaSuccess) return err;
   shape.costCtas = e;
   return applyFusedShape(sms, ctasPerSm, shape.applyCtas);
@@ -3681,8 +3690,9 @@ cudaError_t launchEngineEx(const EngineParams &p, int ctas, cudaStream_t s) {
 
 cudaError_t launchBuild(const BuildParams &p, int ctas, cudaStream_t s) {
   void *args[] = {const_cast<BuildParams *>(&p)};
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(buildGraph), dim3(ctas),
-                                     dim3(kThreads), args, 0, s);
+  const void *fn = p.rank != nullptr ? reinterpret_cast<const void *>(buildGraph<true>)
+                                     : reinterpret_cast<const void *>(buildGraph<false>);
+  return cudaLaunchCooperativeKernel(fn, dim3(ctas), dim3(kThreads), args, 0, s);
 }
 
 cudaError_t launchCosts(const CostParams &p, int ctas, cudaStream_t s) {

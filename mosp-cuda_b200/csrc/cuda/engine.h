@@ -252,7 +252,7 @@ struct BuildParams {
   const int *outRow, *outCol, *edgeMajorW;
   int *outW, *inRow, *inCol, *inW;
   int *cursor;  // in-degrees [n + 1]
-  int *rank;    // edge e among the edges into its head [m]
+  int *rank;    // edge e among the edges into its head [m], or null: no room
   long long *blockSums;
   EngineControl *ctl;
 };
