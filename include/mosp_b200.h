@@ -258,7 +258,11 @@ int mosp_workspace_last_phases(mosp_workspace *ws, int which,
  * launch: time (ns), iterations and list items of the iterations that split
  * a far pile (index 0) and of the pure push iterations (index 1); ns[2..6]
  * (ns has 7 entries) split the push iterations of CTA 0 into decision step,
- * own items, wait for the CTA's other warps, list flush and grid barrier. */
+ * own items, wait for the CTA's other warps, list flush and grid barrier.
+ * A launch of the asynchronous loop: ns[0] its time, ns[1] the warp rounds
+ * before a CTA took spilled entries in a phase, ns[2..6] the durations of the
+ * first four phases and of the rest; iters its phases and warp rounds; items
+ * the entries taken from the spill queue and from the CTAs' own work. */
 int mosp_workspace_loop_profile(mosp_workspace *ws, int which,
                                 unsigned long long *ns, long long *iters,
                                 long long *items);

@@ -943,7 +943,10 @@ struct AsyncCta {
   int over;          // the phase is over
   int abort;         // the launch stops
   long long base;    // first far-pile index of the share
-  unsigned rounds, items, taken;  // statistics
+  // statistics: rounds, those of a phase from the CTA's first claim of spilled
+  // entries on (fed; at round fedFrom), entries
+  int fed;
+  unsigned rounds, fedRounds, fedFrom, items, taken;
   unsigned expanded[kMaxK];
   int mail[kWarps];  // entries in a warp's mail
   u64 bar[kWarps];   // its mbarrier
@@ -1330,6 +1333,10 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
       __threadfence();  // acquire: the producers' counts and slots
       C.owed += n;
       C.taken += n;
+      if (C.fed == 0) {
+        C.fed = 1;
+        C.fedFrom = ldShared(&C.rounds);
+      }
       r0 = atomicAdd(&C.tail, n);
       if (C.dry != 0) {
         C.dry = 0;
@@ -2009,7 +2016,8 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
     C.lock = 0;
     C.abort = 0;
     C.idle = 0;
-    C.rounds = C.items = C.taken = 0;
+    C.fed = 0;
+    C.rounds = C.fedRounds = C.items = C.taken = 0;
     C.K = K;
     C.deadline = sync.deadline;
   }
@@ -2076,6 +2084,8 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
         C.owed = 1;
         C.dry = 0;
         C.over = 0;
+        if (C.fed != 0) C.fedRounds += C.rounds - C.fedFrom;
+        C.fed = 0;
         C.phase = phase;
         if (blockIdx.x == 0) {
           // the counters of the next phase (last looked at before this one)
@@ -2118,11 +2128,11 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopIters[1]),
               static_cast<unsigned long long>(C.rounds));
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopNs[1]),
-              static_cast<unsigned long long>(C.rounds));
+              static_cast<unsigned long long>(C.rounds - C.fedRounds));
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopItems[0]),
               static_cast<unsigned long long>(C.taken));
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->loopItems[1]),
-              static_cast<unsigned long long>(C.items));
+              static_cast<unsigned long long>(C.items - C.taken));
   }
   if (threadIdx.x < K && C.expanded[threadIdx.x] != 0) {
     atomicAdd(reinterpret_cast<unsigned long long *>(&c->pushes[threadIdx.x]),

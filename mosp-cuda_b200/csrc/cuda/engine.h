@@ -95,9 +95,9 @@ struct alignas(128) EngineControl {
   // near-far loop profile. Bulk loop (written by CTA 0): time and items of
   // iterations that split a far pile ([0]) and of pure push iterations
   // ([1]). Asynchronous loop: loopNs[0] its time, loopIters[0] its phases,
-  // loopIters[1] warp rounds, loopNs[1] of which on the CTA's own work, loopItems
-  // entries taken from the spill queue ([0]) and from the CTAs' own rings
-  // and far-pile shares ([1])
+  // loopIters[1] warp rounds, loopNs[1] of which before the CTA took spilled
+  // entries in its phase, loopItems entries taken from the spill queue ([0])
+  // and from the CTAs' own rings and far-pile shares ([1])
   unsigned long long loopNs[2];
   long long loopIters[2];
   long long loopItems[2];

@@ -446,8 +446,9 @@ class Workspace:
         """Near-far loop of the last launch. Bulk loop: {split|push: (ms,
         iterations, items)} and the parts of a push iteration; asynchronous
         loop: its time and phases, the durations of the first four phases
-        (the rest summed), warp rounds and the entries taken from the spill
-        queue and from the CTAs' own rings and far-pile shares."""
+        (the rest summed), warp rounds (local: before the CTA took spilled
+        entries in its phase) and the entries taken from the spill queue and
+        from the CTAs' own rings and far-pile shares."""
         ns = (C.c_ulonglong * 7)()
         it = (C.c_longlong * 2)()
         items = (C.c_longlong * 2)()
