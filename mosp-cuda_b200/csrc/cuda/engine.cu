@@ -2885,13 +2885,21 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
         }
         __syncthreads();
       };
+      // The tiles of all CTAs are interleaved, so that few candidates spread
+      // over the grid: by single candidates where the graph has hubs, whose
+      // in-rows then meet different CTAs, else by 32, whose loads are one line.
+      // Pull phase by CTA tiles, by 32 and by ones, us: R-MAT of 262,144
+      // vertices, K = 4: 848 candidates 36, 28, 18; 52,582: 61, 46, 40; scale
+      // 22, K = 5, 270,959: 121, 120, 115; road networks: 64 of 20,020
+      // vertices, 1.3M candidates: 61, 50, 83; 640,000 vertices, 413,402: 46,
+      // 43, 54; 93,300 vertices, 83,544: 9.9, 9.4, 11.1.
+      const unsigned group = heavyOn ? 1 : 32;
       const long long tileStride = static_cast<long long>(gridDim.x) * blockDim.x;
       for (long long tile = static_cast<long long>(blockIdx.x) * blockDim.x;
            tile - static_cast<long long>(blockIdx.x) * blockDim.x < total; tile += tileStride) {
-        // the tiles of all CTAs interleaved, so that few candidates (the
-        // heads of a small batch, hubs among them) spread over the grid
         const long long j = tile - static_cast<long long>(blockIdx.x) * blockDim.x +
-                            static_cast<long long>(threadIdx.x) * gridDim.x + blockIdx.x;
+                            (static_cast<long long>(threadIdx.x / group) * gridDim.x + blockIdx.x) * group +
+                            threadIdx.x % group;
         const bool valid = j < total;
         int k = 0;
         if (valid) {
