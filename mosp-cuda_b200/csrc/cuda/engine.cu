@@ -886,13 +886,19 @@ constexpr int kOctDeg = 32;          // longest row of such a batch
 constexpr int kQuadBatch = 8;        // the same with row records (four lanes each)
 constexpr int kChaseRing = 64;       // ring entries above which a warp keeps no entries of its own
 // What a batch of the loop reads: the CSR; row records for few entries and the
-// CSR for full batches; row records for all. Full batches read the records
-// while all of them fit L2; past that the CSR, which is half their size and
-// shares lines between neighbours, is the better source (near-far loop of an
-// update: 96 MB of records 6.06 ms against 6.85 ms, 123 MB 1.13 against 0.97,
-// 189 MB 1.42 against 1.20).
+// CSR for full batches; row records for all. An update's full batches read the
+// CSR, those of a launch from scratch the records, whatever their size: loops
+// of road networks with records and with the CSR in full batches, us:
+//   update, long-range changes (wide phases), 5, 28, 95 and 180 MB of records:
+//     K = 1 332/310, 555/506, 980/818, 1385/1110; K = 3 286/283, 539/485,
+//     880/735; 64 networks, K = 3, 117 MB 1102/957
+//   update, short detours (narrow phases), 5, 28, 95 MB: K = 3 706/703,
+//     2390/2363, 5105/5056
+//   combined graph, 3, 30, 100 and 180 MB: wide 310/340, 411/443, 535/549,
+//     663/669; narrow 633/636, 1505/1510, 4659/4674, 6026/6050
+//   tree from scratch, 3, 15, 60, 176 MB: 925/922, 2282/2290, 5104/5111,
+//     9732/9750
 enum : int { kCsrOnly = 0, kThinRecords = 1, kRecords = 2 };
-constexpr long long kRecordBytes = 100LL << 20;
 constexpr unsigned kThinShare = 64;  // far-pile entries per CTA up to which a phase is wider
 constexpr unsigned kSpinLimit = 1u << 24;
 #ifndef MOSP_EDGE_SLOTS_ASYNC
@@ -1962,7 +1968,7 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
         farCount = chaseRecords<Mode>(P, donate, farCount, k, v, base, live ? cols.x : -1, wts.x);
         continue;
       }
-      if (wideRecords) {
+      if constexpr (wideRecords) {
         farCount = expandRecords<Mode>(P, donate, farCount, k, v, base, live, cols, wts);
         continue;
       }
@@ -2528,11 +2534,9 @@ __device__ bool runNearFar(const EngineParams &P, const int *outRow, const int *
                      P.aqShards <= kAsyncShards && P.n <= (1 << 27) &&
                      P.stageEntries >= kStageEntriesAsync &&
                      __ldcg(&P.ctl->heavy) == 0;
-  if (async && rec && 32LL * P.n * P.K <= kRecordBytes) {
-    return asyncNearFar<Mode, kRecords>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
-  }
   if (async && rec) {
-    return asyncNearFar<Mode, kThinRecords>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
+    constexpr int Kind = Mode == kModeUpdate ? kThinRecords : kRecords;
+    return asyncNearFar<Mode, Kind>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
   }
   if (async) return asyncNearFar<Mode, kCsrOnly>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
   return nearFarLoop<Mode>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
