@@ -899,6 +899,13 @@ constexpr int kChaseRing = 64;       // ring entries above which a warp keeps no
 //   tree from scratch, 3, 15, 60, 176 MB: 925/922, 2282/2290, 5104/5111,
 //     9732/9750
 enum : int { kCsrOnly = 0, kThinRecords = 1, kRecords = 2 };
+// The records are used where at most one row in kLongRows is longer than one:
+// a batch with such a row has loaded its records for nothing. Tree from
+// scratch and update with short changes, 302,500 vertices, with records and
+// without, us: grids, 0.5% of the rows longer 1702/2268, 3661/4830; random
+// graphs, 0% 657/783, 1832/2097; 4.7% 822/689, 1525/1437; 17% 880/683,
+// 1433/1222.
+constexpr long long kLongRows = 50;
 constexpr unsigned kThinShare = 64;  // far-pile entries per CTA up to which a phase is wider
 constexpr unsigned kSpinLimit = 1u << 24;
 #ifndef MOSP_EDGE_SLOTS_ASYNC
@@ -2497,6 +2504,7 @@ __device__ __forceinline__ void collectInvalid(const EngineParams &P, int k, lon
 template <int Mode>
 __device__ void buildRecords(const EngineParams &P, const int *outRow, const int *outCol,
                              const int *const *outWk, long long tid, long long T) {
+  int longer = 0;
   for (long long v = tid; v < P.n; v += T) {
     const int b = ldLoop<Mode>(outRow + v);
     const int deg = ldLoop<Mode>(outRow + v + 1) - b;
@@ -2505,7 +2513,10 @@ __device__ void buildRecords(const EngineParams &P, const int *outRow, const int
     for (int q = 0; q < 4; ++q) c[q] = q < deg ? ldLoop<Mode>(outCol + b + q) : -1;
 #pragma unroll
     for (int q = 0; q < 4; ++q) c[q] = c[q] == P.source ? -1 : c[q];
-    if (deg > 4) c[3] = kMoreEdges;
+    if (deg > 4) {
+      c[3] = kMoreEdges;
+      ++longer;
+    }
     for (int k = 0; k < P.K; ++k) {
       int w[4];
 #pragma unroll
@@ -2515,11 +2526,16 @@ __device__ void buildRecords(const EngineParams &P, const int *outRow, const int
       r[1] = make_int4(w[0], w[1], w[2], w[3]);
     }
   }
+  __syncwarp();
+  longer = __reduce_add_sync(kFull, longer);
+  if (laneId() == 0 && longer > 0) atomicAdd(&P.ctl->longRows, longer);
 }
 
 /// The near-far loop of a launch: asynchronous when the launch asks for it
-/// and the graph has no hub rows (which the bulk loop hands to whole CTAs);
-/// the same decision in every CTA (the hub flag is set before a barrier).
+/// and the graph has no hub rows (which the bulk loop hands to whole CTAs),
+/// with row records where the launch made them (rec) and they hold nearly all
+/// rows; the same decision in every CTA (the hub flag and the count of longer
+/// rows are final before a barrier).
 template <int Mode>
 __device__ bool runNearFar(const EngineParams &P, const int *outRow, const int *outCol,
                            const int *const *outWk, Sync &epoch, u64 *deltaOverride, int genBase,
@@ -2534,7 +2550,7 @@ __device__ bool runNearFar(const EngineParams &P, const int *outRow, const int *
                      P.aqShards <= kAsyncShards && P.n <= (1 << 27) &&
                      P.stageEntries >= kStageEntriesAsync &&
                      __ldcg(&P.ctl->heavy) == 0;
-  if (async && rec) {
+  if (async && rec && kLongRows * __ldcg(&P.ctl->longRows) <= P.n) {
     constexpr int Kind = Mode == kModeUpdate ? kThinRecords : kRecords;
     return asyncNearFar<Mode, Kind>(P, outRow, outCol, outWk, epoch, deltaOverride, genBase);
   }

@@ -112,6 +112,7 @@ struct alignas(128) EngineControl {
   int recScan[kMaxK];
   int recChunks[2];
   int recWide;        // full parent recovery: a distance of 2^31 or more (recDist is not used)
+  int longRows;       // rows longer than a row record
   unsigned chunkNext; // next chunk of a pass over all edges (at most one per launch)
 };
 
@@ -159,7 +160,13 @@ constexpr int kMoreEdges = -2;   // fourth head of a record: the row has more th
 constexpr int kFarCopies = 3;
 
 /// Whether a launch makes row records: graphs of at most 3.5 edges per
-/// vertex.
+/// vertex, most of which have few longer rows. Grids of 302,500 vertices, K = 3,
+/// with records and without, pass in us: 2 edges per vertex, update with
+/// long-range changes 1102/1356, with short ones 4012/5585, tree from scratch
+/// 2434/3409; 2.8: 1047/1092, 3661/4830, 1702/2268; 3.4: 1067/1070, 3965/5207,
+/// 1826/2377; 4: 1182/1202, 4167/5280, 1919/2470; 5: 1385/1215, 7389/5079,
+/// 5035/2497 (every row is longer). A random graph of 3.4 has 17% longer rows,
+/// where the records are not used; making them takes 10 us of a pass of 700.
 __host__ __device__ inline bool recordsPay(long long n, long long m) { return 2 * m <= 7 * n; }
 
 // Phase boundaries recorded in EngineControl::phaseNs.
