@@ -18,7 +18,9 @@
 // of appended groups of its row with an earlier first insertion, counted over
 // the row's own list, which costs the square of the insertions into one row:
 // with all of a batch of 65,536 in one row 1.9 ms (sorted form 10.6), of
-// 262,144 14 ms (24). That sets kFusedBatch.
+// 262,144 14 ms (24). That sets kFusedBatch. Like the sorted form, one lane
+// walks the row of a group that touches more than one of its parallel edges,
+// from the first of them to the last it touches.
 //
 // The copy is one pass over all edges: a warp takes 128 of them, which need no
 // row, and moves their heads and their 128 K weights as one consecutive range
@@ -64,7 +66,8 @@ struct FusedScratch {
   int *cD, *cI, *firstIns, *lastIns, *occ, *first;
   unsigned *bits;
   unsigned slots;
-  unsigned *filter;  // filterBits bits, 16 or more per group, set where a group hashes
+  unsigned *filter;  // filterBits bits, set where a group hashes: 16 or more per group for up to
+                     // 65,536 changes, no fewer than 4 past that (128 KB: what L1 holds)
   unsigned filterBits;
   int *entrySlot;  // slot of batch entry j (deletions first)
   // touched rows, in no order
@@ -81,6 +84,7 @@ struct FusedScratch {
   FusedResult *result;
 };
 
+/// The 64-bit finaliser of MurmurHash3 (public domain), to spread the ids.
 __device__ __forceinline__ unsigned hashOf(u64 key) {
   key ^= key >> 33;
   key *= 0xff51afd7ed558ccdULL;

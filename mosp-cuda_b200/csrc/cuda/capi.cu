@@ -539,8 +539,8 @@ void fillLists(EngineParams &p, mosp_workspace *ws, int block) {
   if (p.mode == kModeUpdate && p.recMark != nullptr) p.flags |= kFlagCanonical;
   p.heavyDeg = ws->heavyDeg;
   // asynchronous loop unless it is off or the graph last seen here had hub
-  // rows; its launches need a smaller stage (the pull pass stays staged up
-  // to K tiles), which leaves more of the SM's memory to L1
+  // rows; its stage holds the CTA's ring, far buffers and state, and at least
+  // K tiles for the pull pass
   const bool async = ws->asyncMode != 0 && ws->aqSlots != nullptr && ws->farCopies == kFarCopies &&
                      ws->aqCap >= asyncSlotsFor(p.n, p.K, ws->asyncSlots) &&
                      !ws->heavySeen[block == 1 ? 1 : 0];

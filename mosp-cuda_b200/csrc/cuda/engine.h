@@ -126,7 +126,8 @@ enum : int {
                          // no hub rows
   kFlagPullOnly = 8,     // always pull into the candidates (never push from the
                          // valid vertices)
-                         // 16: not used (was: per-warp continuation)
+                         // (16 is free: the asynchronous loop always goes on
+                         // inside its warps)
   kFlagCanonical = 32    // the input trees follow the lowest-id tie rule: with
                          // kFlagHostRecovery, distance-only objectives recover
                          // parents only where the batch can change them
