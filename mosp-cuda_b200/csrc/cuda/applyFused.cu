@@ -20,7 +20,9 @@
 // with all of a batch of 65,536 in one row 1.9 ms (sorted form 10.6), of
 // 262,144 14 ms (24). That sets kFusedBatch. Like the sorted form, one lane
 // walks the row of a group that touches more than one of its parallel edges,
-// from the first of them to the last it touches.
+// from the first of them to the last it touches, 16 heads at a time (two edges
+// 100,000 apart: 2.0 ms, head by head 11.4, sorted form 9.3; 1,000 deletions
+// of one edge: 0.11 ms, with an atomic each 0.56, sorted form 0.43).
 //
 // The copy is one pass over all edges: a warp takes 128 of them, which need no
 // row, and moves their heads and their 128 K weights as one consecutive range
@@ -45,6 +47,7 @@ namespace {
 constexpr u64 kNoKey = ~0ULL;
 constexpr int kLaneRow = 16;  // touched rows of at most so many edges are searched by one lane,
 constexpr int kPiece = 64;    // longer ones in pieces of so many by a warp each
+constexpr int kWalk = 16;     // heads in flight on the walk to a group's next parallel edge
 constexpr int kCopyThreads = 256;
 constexpr int kCopyEdges = 128;  // edges a warp of the copy takes at a time
 constexpr int kTurns = 8;        // turns of its weights in flight
@@ -185,15 +188,36 @@ __device__ __forceinline__ void resolveGroup(const ApplyParams &P, const FusedSc
   if (appended != removed) atomicAdd(S.delta + u, appended - removed);
   // the first `removed` occurrences go; the next one takes the weights
   const int seen = removed + (cI > 0 && occ > cD ? 1 : 0);
-  int e = __ldcg(S.first + s);
-  for (int i = 0; i < seen; ++e) {
-    if (__ldg(P.col + e) != v) continue;
-    if (i++ < removed) {
-      atomicOr(&S.block[e >> 5].dead, 1u << (e & 31));
-      atomicAdd(&S.block[(e >> 5) + 1].shift, -1);
-    } else {
-      atomicOr(&S.block[e >> 5].other, 1u << (e & 31));
-      other = e;
+  const unsigned end = static_cast<unsigned>(__ldg(P.row + u + 1));
+  unsigned e0 = static_cast<unsigned>(__ldcg(S.first + s));
+  for (int i = 0; i < seen && e0 < end; e0 += kWalk) {
+    int head[kWalk];
+#pragma unroll
+    for (int q = 0; q < kWalk; ++q) head[q] = e0 + q < end && (q == 0 || seen > 1) ? __ldg(P.col + e0 + q) : -1;
+    unsigned hits = 0;
+#pragma unroll
+    for (int q = 0; q < kWalk; ++q) hits |= (head[q] == v ? 1u : 0u) << q;
+    unsigned gone = hits;
+    for (int left = __popc(hits); left > removed - i; --left) gone &= ~(0x80000000u >> __clz(gone));
+    if (gone != 0) {
+      // (the block of e0 and the next one)
+      const u64 dead = static_cast<u64>(gone) << (e0 & 31u);
+      Block *b = S.block + (e0 >> 5);
+      const unsigned lo = static_cast<unsigned>(dead), hi = static_cast<unsigned>(dead >> 32);
+      if (lo != 0) {
+        atomicOr(&b[0].dead, lo);
+        atomicAdd(&b[1].shift, -__popc(lo));
+      }
+      if (hi != 0) {
+        atomicOr(&b[1].dead, hi);
+        atomicAdd(&b[2].shift, -__popc(hi));
+      }
+      i += __popc(gone);
+    }
+    if (hits != gone && i < seen) {
+      other = static_cast<int>(e0) + __ffs(hits ^ gone) - 1;
+      atomicOr(&S.block[other >> 5].other, 1u << (other & 31));
+      ++i;
     }
   }
   if (cI > 0 && occ > 0) {
