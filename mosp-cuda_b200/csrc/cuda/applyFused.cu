@@ -14,15 +14,16 @@
 // those removed before it, in whatever row: each block of 32 edges has the sum
 // up to its first edge (a scan of the groups' changes) and bits for the changes
 // inside it. Only a block with several edges appended at one place goes by its
-// rows. The place of an appended edge is the number
-// of appended groups of its row with an earlier first insertion, counted over
-// the row's own list, which costs the square of the insertions into one row:
-// with all of a batch of 65,536 in one row 1.9 ms (sorted form 10.6), of
-// 262,144 14 ms (24). That sets kFusedBatch. Like the sorted form, one lane
-// walks the row of a group that touches more than one of its parallel edges,
-// from the first of them to the last it touches, 16 heads at a time (two edges
-// 100,000 apart: 2.0 ms, head by head 11.4, sorted form 9.3; 1,000 deletions
-// of one edge: 0.11 ms, with an atomic each 0.56, sorted form 0.43).
+// rows. The place of an appended edge is the number of appended groups of its
+// row with an earlier first insertion: counted over the row's own list, or,
+// where a row takes more than a sixteenth of a batch of more than 8,192
+// insertions, over bits by file position (200,000 edges appended to one row:
+// 1.16 ms, by lists alone 8.8, sorted form 6.3). Either costs the square of the
+// insertions into one row, which sets kFusedBatch. Like the sorted form, one
+// lane walks the row of a group that touches more than one of its parallel
+// edges, from the first of them to the last it touches, 16 heads at a time (two
+// edges 100,000 apart: 2.0 ms, head by head 11.4, sorted form 9.3; 1,000
+// deletions of one edge: 0.11 ms, with an atomic each 0.56, sorted form 0.43).
 //
 // The copy is one pass over all edges: a warp takes 128 of them, which need no
 // row, and moves their heads and their 128 K weights as one consecutive range
@@ -51,9 +52,12 @@ constexpr int kWalk = 16;     // heads in flight on the walk to a group's next p
 constexpr int kCopyThreads = 256;
 constexpr int kCopyEdges = 128;  // edges a warp of the copy takes at a time
 constexpr int kTurns = 8;        // turns of its weights in flight
+constexpr int kMarkRows = 16;    // rows with bits of their own: more than one in so many of the insertions,
+constexpr int kMarkLeast = 8192;  // in batches of more than so many
 constexpr unsigned kByRows = ~0U;  // Block::app: more than one edge appended at one place
 constexpr int kNoMove = INT_MIN;
 constexpr int kMaxCtas = 2048;
+constexpr int kCounts = 5;  // FusedScratch::counts
 
 /// What moves 32 consecutive edges of the old graph.
 struct alignas(16) Block {
@@ -75,13 +79,16 @@ struct FusedScratch {
   int *entrySlot;  // slot of batch entry j (deletions first)
   // touched rows, in no order
   int *rows, *nApp, *segApp, *curApp;
+  int *markOf;      // of a row that many edges are appended to: its bits, else -1
+  unsigned *marks;  // kMarkRows rows of markWords: a bit per insertion whose group appends
+  int markWords;    // (a multiple of 4; 0: no such rows)
   u64 *pieces;     // of the longer touched rows: vertex << 32 | piece
   Block *block;    // per 32 edges, and one behind them
   int *app;        // insertions that append, by row segment
   int2 *other;     // edges that take an insertion's weights: edge, slot
   // per vertex: touched row + 1 (0: none), and its change of degree
   int *rowSlot, *delta;
-  int *counts;     // touched rows, pieces, appended, edges with an insertion's weights
+  int *counts;     // touched rows, pieces, appended, edges with an insertion's weights, rows with bits
   long long *blockSums;  // of the CTAs: degree changes, then (moveSums) block moves
   long long *moveSums;
   FusedResult *result;
@@ -253,8 +260,9 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
   }
   for (long long i = tid; i <= (m + 31LL) / 32; i += T) S.block[i] = Block{0, 0, 0, 0};
   for (long long i = tid; i < S.filterBits / 32; i += T) S.filter[i] = 0;
+  for (long long i = tid; i < static_cast<long long>(kMarkRows) * S.markWords; i += T) S.marks[i] = 0;
   for (long long r = tid; r < B; r += T) S.nApp[r] = S.curApp[r] = 0;
-  if (tid < 4) S.counts[tid] = 0;
+  if (tid < kCounts) S.counts[tid] = 0;
   if (tid < kMaxK) {
     S.result->maxWeight[tid] = 1;
     S.result->weightSum[tid] = 0;
@@ -342,8 +350,12 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
   // ---- row segments of the lists; masks; sums of the degree changes --------
   for (long long q0 = tid - lane; q0 < R; q0 += T) {
     const long long r = q0 + lane;
-    const int a = warpReserve(S.counts + 2, r < R ? __ldcg(S.nApp + r) : 0);
-    if (r < R) S.segApp[r] = a;
+    const int count = r < R ? __ldcg(S.nApp + r) : 0;
+    const int a = warpReserve(S.counts + 2, count);
+    if (r < R) {
+      S.segApp[r] = a;
+      S.markOf[r] = S.markWords > 0 && count > P.nIns / kMarkRows ? atomicAdd(S.counts + 4, 1) : -1;
+    }
   }
   for (long long i = tid; i < P.nIns; i += T) P.mask[i] = __ldcg(S.bits + S.entrySlot[P.nDel + i]);
   // (a CTA's range in whole groups of four vertices)
@@ -379,7 +391,9 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
     const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s);
     if (occ <= cD && __ldcg(S.cI + s) > 0) {
       const int r = __ldcg(S.rowSlot + static_cast<int>(key >> 32)) - 1;
-      S.app[__ldcg(S.segApp + r) + atomicAdd(S.curApp + r, 1)] = __ldcg(S.firstIns + s);
+      const int i = __ldcg(S.firstIns + s), bits = __ldcg(S.markOf + r);
+      S.app[__ldcg(S.segApp + r) + atomicAdd(S.curApp + r, 1)] = i;
+      if (bits >= 0) atomicOr(S.marks + static_cast<long long>(bits) * S.markWords + (i >> 5), 1u << (i & 31));
     }
   }
   {
@@ -546,9 +560,19 @@ copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedSc
     const int u = __ldg(P.insFrom + i);
     const int r = __ldcg(S.rowSlot + u) - 1;
     const int count = __ldcg(S.nApp + r);
-    const int *list = S.app + __ldcg(S.segApp + r);
     int rank = 0;
-    for (int x = 0; x < count; ++x) rank += __ldcg(list + x) < i;
+    if (const int bits = __ldcg(S.markOf + r); bits >= 0) {
+      const unsigned *marks = S.marks + static_cast<long long>(bits) * S.markWords;
+      for (int x = 0; x < i >> 7; ++x) {
+        const uint4 b = __ldg(reinterpret_cast<const uint4 *>(marks) + x);
+        rank += __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
+      }
+      for (int x = i >> 7 << 2; x < i >> 5; ++x) rank += __popc(__ldg(marks + x));
+      rank += __popc(__ldg(marks + (i >> 5)) & ((1u << (i & 31)) - 1u));
+    } else {
+      const int *list = S.app + __ldcg(S.segApp + r);
+      for (int x = 0; x < count; ++x) rank += __ldcg(list + x) < i;
+    }
     const int to = __ldcg(P.newRow + u + 1) - count + rank;
     P.newCol[to] = __ldg(P.insTo + i);
     const long long last = __ldcg(S.lastIns + S.entrySlot[P.nDel + i]);
@@ -591,19 +615,21 @@ unsigned char *layout(unsigned char *p, long long n, long long m, long long nIns
   const long long B = nIns + nDel;
   S.slots = slotsFor(B);
   S.result = carve<FusedResult>(p, 1);
-  S.counts = carve<int>(p, 4);
+  S.counts = carve<int>(p, kCounts);
   S.key = carve<u64>(p, S.slots);
   for (int **x : {&S.cD, &S.cI, &S.firstIns, &S.lastIns, &S.occ, &S.first}) *x = carve<int>(p, S.slots);
   S.bits = carve<unsigned>(p, S.slots);
   S.filterBits = std::min(8 * S.slots, 1u << 20);
   S.filter = carve<unsigned>(p, S.filterBits / 32);
-  for (int **x : {&S.entrySlot, &S.rows, &S.nApp, &S.segApp, &S.curApp}) {
+  for (int **x : {&S.entrySlot, &S.rows, &S.nApp, &S.segApp, &S.curApp, &S.markOf}) {
     *x = carve<int>(p, B);
   }
   S.pieces = carve<u64>(p, m / kPiece + B);
   S.block = carve<Block>(p, (m + 31) / 32 + 1);
   S.moveSums = carve<long long>(p, kMaxCtas);
   S.app = carve<int>(p, nIns);
+  S.markWords = nIns > kMarkLeast ? static_cast<int>((nIns + 127) / 128 * 4) : 0;
+  S.marks = carve<unsigned>(p, static_cast<long long>(kMarkRows) * S.markWords);
   S.other = carve<int2>(p, nIns);
   S.rowSlot = carve<int>(p, n + 4);
   S.delta = carve<int>(p, n + 4);
