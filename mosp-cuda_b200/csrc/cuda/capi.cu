@@ -739,7 +739,6 @@ struct UpdateArgs {
   int *const *parent;
 };
 
-/// Build the parameters of a fused K-objective update.
 /// The full parent recovery's distances side by side, for `count`
 /// objectives; without room for them (false) it reads the objectives' own
 /// arrays.
@@ -778,6 +777,7 @@ int reserveRecovery(mosp_workspace *ws, long long m, int K) {
   return MOSP_OK;
 }
 
+/// Build the parameters of a fused K-objective update.
 int prepareUpdate(mosp_workspace *ws, const UpdateArgs &a, EngineParams &p, int *bitsOut) {
   if (a.n <= 0 || a.m < 0 || a.K < 1 || a.K > kMaxK || a.source < 0 || a.source >= a.n ||
       a.nHeads < 0 || (a.nHeads > 0 && a.heads == nullptr) || a.outRow == nullptr ||
