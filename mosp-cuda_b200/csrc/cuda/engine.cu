@@ -60,6 +60,11 @@ __device__ __forceinline__ void stRelease64(unsigned long long *p, unsigned long
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+/// Two adjacent words, each read on its own, past L1.
+__device__ __forceinline__ void ldPair(const unsigned *p, unsigned &a, unsigned &b) {
+  asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "l"(p) : "memory");
+}
+
 __device__ __forceinline__ void stRelaxed64(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -842,7 +847,7 @@ __device__ bool nearFarLoop(const EngineParams &P, const int *outRow,
 //     what improves back to it;
 //   * a CTA whose ring holds more than kDonate entries while others have run
 //     dry, or more than kRingSpill in any case, sends its pushes to a global
-//     spill queue, from which dry CTAs claim up to 256 entries at a time. A
+//     spill queue, from which dry CTAs claim up to 1,024 entries at a time. A
 //     push that finds its shard full goes to the far pile.
 //
 // Row records (one 32-byte sector with a vertex's first four edges) make the
@@ -878,9 +883,11 @@ constexpr unsigned kRingMask = kRing - 1;
 // a push finds the ring at most this full, plus 128 entries of each of the
 // other warps that passed the check at the same time, plus a claim
 constexpr unsigned kRingSpill = kRing / 4;
-constexpr unsigned kDonate = 512;    // ring entries above which a CTA feeds dry ones
+constexpr unsigned kDonate = 512;    // ring entries above which a CTA feeds dry ones,
+constexpr unsigned kDonateRows = 64;  // in graphs without row records
 constexpr unsigned kSliceFirst = 1024;  // ring entries above which the share waits
-constexpr int kClaim = 256;          // entries claimed from the spill queue at a time
+constexpr int kClaim = 1024;         // entries claimed from the spill queue at a time
+constexpr int kFetch = 256;          // of these read at a time
 constexpr int kOctBatch = 4;         // entries of a batch that is expanded by octets of lanes
 constexpr int kOctDeg = 32;          // longest row of such a batch
 constexpr int kQuadBatch = 8;        // the same with row records (four lanes each)
@@ -964,6 +971,7 @@ struct AsyncCta {
   int mail[kWarps];  // entries in a warp's mail
   u64 bar[kWarps];   // its mbarrier
   int K;
+  unsigned donateAt;  // ring entries above which the CTA feeds dry ones
   unsigned phase;
   unsigned long long deadline;
   AsyncObj obj[kMaxK];
@@ -1143,49 +1151,54 @@ __device__ __forceinline__ bool newInFar(const AsyncObj &O, u64 old, int x) {
   }
 }
 
-/// Near entries of the lanes with `want` to the spill queue: counted in
+/// Room for `count` near entries of the warp in the spill queue: counted in
 /// asyncPending before their slots can be claimed (the reservation releases
-/// the count). Past the shard's capacity a vertex goes to the far pile, once
-/// (by its flag), marked so that the split expands it. All lanes call it.
-__device__ __noinline__ void spillNear(const EngineParams &P, unsigned mask, u64 entry) {
+/// the count). The shard, and the first entry's position in it, which may lie
+/// past its capacity (spillWrite). All lanes call it.
+__device__ __noinline__ unsigned spillReserve(const EngineParams &P, int count, int &shard) {
   AsyncCta &C = asyncCta();
-  const LoopShared &L = C.L;
-  const int lane = static_cast<int>(laneId());
-  const int count = __popc(mask);
   // the shards take turns, a different one for each CTA
   const int s = static_cast<int>((blockIdx.x * 5u + (threadIdx.x >> 5) + (ldShared(&C.settled) >> 5)) %
                                  static_cast<unsigned>(P.aqShards));
   const int target = __shfl_sync(kFull, s, 0);
   unsigned base = 0;
-  if (lane == 0) {
+  if (laneId() == 0) {
     atomicAdd(&P.ctl->asyncPending[C.phase % 3], static_cast<unsigned>(count));
-    u64 old;
-    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
-                 : "=l"(old)
-                 : "l"(&P.aqCtr[C.phase % 3 * P.aqShards + target].claimed), "l"(static_cast<u64>(count) << 32)
-                 : "memory");
-    base = static_cast<unsigned>(old >> 32);
+    AsyncShard *A = P.aqCtr + C.phase % 3 * P.aqShards + target;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(base) : "l"(&A->reserved), "r"(count) : "memory");
     // the ones past the capacity are not queued
     const unsigned end = base + static_cast<unsigned>(count);
     if (end > P.aqShardCap) {
       atomicSub(&P.ctl->asyncPending[C.phase % 3], end - (base > P.aqShardCap ? base : P.aqShardCap));
     }
   }
-  base = __shfl_sync(kFull, base, 0);
-  if (!((mask >> lane) & 1u)) return;
-  const unsigned idx = base + __popc(mask & ((1u << lane) - 1u));
+  shard = target;
+  return __shfl_sync(kFull, base, 0);
+}
+
+/// A near entry to its reserved place. Past the shard's capacity its vertex
+/// goes to the far pile, once (by its flag), marked so that the split expands
+/// it.
+__device__ __forceinline__ void spillWrite(const EngineParams &P, int shard, unsigned idx, u64 entry) {
   if (idx < P.aqShardCap) {
     // release: an entry without a usable tag needs its word before it
-    stRelease64(P.aqSlots + static_cast<long long>(target) * P.aqShardCap + idx, entry);
+    stRelease64(P.aqSlots + static_cast<long long>(shard) * P.aqShardCap + idx, entry);
     return;
   }
   const int k = static_cast<int>(entry & 31u);
   const int v = static_cast<int>(static_cast<unsigned>(entry) >> 5);
   __threadfence();  // the word before the flag
   if (atomicExch(P.inFar + static_cast<long long>(k) * P.stride + v, 1) == 0) {
-    const Target t = listTarget(P, L, P.K + k, 0, nullptr, nullptr);
+    const Target t = listTarget(P, asyncCta().L, P.K + k, 0, nullptr, nullptr);
     t.v[atomicAdd(t.counter, 1)] = static_cast<int>(static_cast<unsigned>(v) | kOverflow);
   }
+}
+
+/// Near entries of the lanes in `mask` to the spill queue. All lanes call it.
+__device__ __noinline__ void spillNear(const EngineParams &P, unsigned mask, u64 entry) {
+  int shard;
+  const unsigned at = spillReserve(P, __popc(mask), shard);
+  if ((mask >> laneId()) & 1u) spillWrite(P, shard, at + __popc(mask & ((1u << laneId()) - 1u)), entry);
 }
 
 /// Write an entry to a reserved ring slot. The slot is empty unless the warp
@@ -1209,15 +1222,45 @@ __device__ __forceinline__ void ringWrite(const EngineParams &P, unsigned pos, u
 __device__ __forceinline__ bool ringReserve(bool donate, int count, unsigned &at) {
   AsyncCta &C = asyncCta();
   const unsigned held = ldShared(&C.tail) - ldShared(&C.head);
-  if (held > kRingSpill || (donate && held > kDonate)) return false;
+  if (held > kRingSpill || (donate && held > C.donateAt)) return false;
   at = atomicAdd(&C.tail, static_cast<unsigned>(count));
   __threadfence_block();  // the entries before the look at the idle warps
   if (ldShared(&C.idle) != 0) wakeIdle(1 + (count >> 3));
   return true;
 }
 
-/// Near entries of the lanes in `mask` to the CTA's ring, one reservation
-/// for the warp, or to the spill queue. All lanes call it.
+/// Near entries of N edges per lane (ballot[h]: the lanes whose edge h has one)
+/// to the CTA's ring or the spill queue, one reservation for the warp. All
+/// lanes call it.
+template <int N>
+__device__ __forceinline__ void nearPush(const EngineParams &P, const unsigned (&ballot)[N], bool donate,
+                                         const u64 (&entry)[N]) {
+  const unsigned lane = laneId();
+  int count = 0;
+#pragma unroll
+  for (int h = 0; h < N; ++h) count += __popc(ballot[h]);
+  if (count == 0) return;
+  unsigned at = 0;
+  int room = 0, shard = 0;
+  if (lane == 0) room = ringReserve(donate, count, at);
+  room = __shfl_sync(kFull, room, 0);
+  at = room ? __shfl_sync(kFull, at, 0) : spillReserve(P, count, shard);
+#pragma unroll
+  for (int h = 0; h < N; ++h) {
+    if ((ballot[h] >> lane) & 1u) {
+      const unsigned idx = at + __popc(ballot[h] & ((1u << lane) - 1u));
+      if (room) {
+        ringWrite(P, idx, entry[h]);
+      } else {
+        spillWrite(P, shard, idx, entry[h]);
+      }
+    }
+    at += __popc(ballot[h]);
+  }
+}
+
+/// The same for one edge per lane. (The way to the queue is a function of its
+/// own, which keeps the registers of this one few.)
 __device__ __noinline__ void ringPush(const EngineParams &P, unsigned mask, bool donate, u64 entry) {
   const unsigned lane = laneId();
   unsigned at = 0;
@@ -1308,10 +1351,10 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
   const int lane = static_cast<int>(laneId());
   const int S = P.aqShards;
   unsigned left = 1;
-  u64 q = 0;
+  unsigned head = 0, tail = 0;
   AsyncShard *shards = P.aqCtr + phase % 3 * S;
   // (relaxed polls: an acquire would empty L1 at every turn)
-  if (lane < S) q = *reinterpret_cast<volatile u64 *>(&shards[lane].claimed);
+  if (lane < S) ldPair(&shards[lane].claimed, head, tail);
   if (lane == 31) left = *reinterpret_cast<volatile unsigned *>(&c->asyncPending[phase % 3]);
   if (__shfl_sync(kFull, left, 31) == 0) {
     if (lane == 0) {
@@ -1324,7 +1367,6 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
     return;
   }
   const unsigned cap = P.aqShardCap;
-  unsigned head = static_cast<unsigned>(q), tail = static_cast<unsigned>(q >> 32);
   if (tail > cap) tail = cap;
   const unsigned have = __ballot_sync(kFull, lane < S && tail > head);
   if (have == 0) return;
@@ -1332,17 +1374,15 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
   const unsigned own = blockIdx.x % S;
   const unsigned later = have >> own << own;
   const int s = __ffs(later != 0 ? later : have) - 1;
-  q = __shfl_sync(kFull, q, s);
-  head = static_cast<unsigned>(q);
-  tail = static_cast<unsigned>(q >> 32);
-  if (tail > cap) tail = cap;
+  head = __shfl_sync(kFull, head, s);
+  tail = __shfl_sync(kFull, tail, s);
   const unsigned n = tail - head < kClaim ? tail - head : kClaim;
   unsigned r0 = 0;
   int got = 0;
   if (lane == 0 && atomicCAS(&C.lock, 0, 1) == 0) {
     __threadfence_block();
     if (ldShared(&C.tail) - ldShared(&C.head) <= kDonate &&
-        atomicCAS(&shards[s].claimed, q, q + n) == q) {
+        atomicCAS(&shards[s].claimed, head, head + n) == head) {
       __threadfence();  // acquire: the producers' counts and slots
       C.owed += n;
       C.taken += n;
@@ -1363,28 +1403,34 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
   if (__shfl_sync(kFull, got, 0) == 0) return;
   r0 = __shfl_sync(kFull, r0, 0);
   u64 *slots = P.aqSlots + static_cast<long long>(s) * cap + head;
-  u64 e[kClaim / 32];
+  for (unsigned j0 = 0; j0 < n; j0 += kFetch) {
+    u64 e[kFetch / 32];
 #pragma unroll
-  for (int i = 0; i < kClaim / 32; ++i) {
-    const unsigned j = static_cast<unsigned>(i * 32 + lane);
-    e[i] = j < n ? ldAcquire64(slots + j) : 0;
-  }
-#pragma unroll
-  for (int i = 0; i < kClaim / 32; ++i) {
-    const unsigned j = static_cast<unsigned>(i * 32 + lane);
-    if (j >= n) continue;
-    // the producer reserved the slot and is about to write it
-    for (unsigned spin = 0; e[i] == kEmptySlot; e[i] = ldAcquire64(slots + j)) {
-      if (++spin > (kSpinLimit >> 4) || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
-        asyncAbort(P);
-        break;
-      }
+    for (int i = 0; i < kFetch / 32; ++i) {
+      const unsigned j = j0 + static_cast<unsigned>(i * 32 + lane);
+      e[i] = j < n ? ldAcquire64(slots + j) : 0;
     }
-    stRelaxed64(slots + j, kEmptySlot);
-    ringWrite(P, r0 + j, e[i]);
+#pragma unroll
+    for (int i = 0; i < kFetch / 32; ++i) {
+      const unsigned j = j0 + static_cast<unsigned>(i * 32 + lane);
+      if (j >= n) continue;
+      // the producer reserved the slot and is about to write it
+      for (unsigned spin = 0; e[i] == kEmptySlot; e[i] = ldAcquire64(slots + j)) {
+        if (++spin > (kSpinLimit >> 4) || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
+          asyncAbort(P);
+          break;
+        }
+      }
+      stRelaxed64(slots + j, kEmptySlot);
+      ringWrite(P, r0 + j, e[i]);
+    }
   }
   __syncwarp();
-  if (lane == 0) wakeIdle(static_cast<int>(n >> 3));
+  if (n > 128) {
+    wakeAll();
+  } else if (lane == 0) {
+    wakeIdle(static_cast<int>(n >> 3));
+  }
 }
 
 /// Graph loads of the asynchronous loop. The combined mode's graph was
@@ -1691,36 +1737,18 @@ __device__ __noinline__ int expandRecords(const EngineParams &P, bool donate, in
     old[h] = 0;
     if (x[h] >= 0 && cw[h] <= most) old[h] = atomicMin(O.packed + x[h], cw[h]);
   }
-  unsigned near = 0, far = 0;  // bit h: this lane's edge h
+  unsigned far = 0;  // bit h: this lane's edge h
   unsigned ballot[4];
-  int count = 0;
+  u64 entry[4];
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     const bool imp = old[h] > (cw[h] | O.mask);
     const bool nr = imp && cw[h] < thrWord;
-    near |= static_cast<unsigned>(nr) << h;
     far |= static_cast<unsigned>(imp && !nr && newInFar<Mode>(O, old[h], x[h])) << h;
     ballot[h] = __ballot_sync(kFull, nr);
-    count += __popc(ballot[h]);
+    entry[h] = nearEntry(k, x[h], cw[h] >> O.bits);
   }
-  if (count > 0) {
-    unsigned at = 0;
-    int room = 0;
-    if (lane == 0) room = ringReserve(donate, count, at);
-    room = __shfl_sync(kFull, room, 0);
-    at = __shfl_sync(kFull, at, 0);
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      if (ballot[h] == 0) continue;
-      const u64 e = nearEntry(k, x[h], cw[h] >> O.bits);
-      if (!room) {
-        spillNear(P, ballot[h], e);
-      } else {
-        if ((near >> h) & 1u) ringWrite(P, at + __popc(ballot[h] & ((1u << lane) - 1u)), e);
-        at += __popc(ballot[h]);
-      }
-    }
-  }
+  nearPush<4>(P, ballot, donate, entry);
   if (__any_sync(kFull, far != 0)) {
 #pragma unroll
     for (int h = 0; h < 4; ++h) farAppend(P, farCount, (far >> h) & 1u, k, x[h], cw[h] >> O.bits);
@@ -1800,7 +1828,7 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
         if (atomicCAS(&C.head, h, h + n) != h) continue;
         at = h;
         what = (1u << 8) | n;
-        if (held > kDonate) what |= 1u << 16;
+        if (held > C.donateAt) what |= 1u << 16;
         break;
       }
     }
@@ -2032,6 +2060,7 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
     C.fed = 0;
     C.rounds = C.fedRounds = C.items = C.taken = 0;
     C.K = K;
+    C.donateAt = Kind == kCsrOnly ? kDonateRows : kDonate;
     C.deadline = sync.deadline;
   }
   for (int i = threadIdx.x; i < kRing; i += blockDim.x) asyncRing()[i] = kEmptySlot;
@@ -2070,8 +2099,12 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
         // network 2.90 -> 2.50 ms (1,500 entries per phase), combined graph
         // of 249,500 vertices 1.47 -> 1.29 ms, but the update of 2M vertices
         // with 1.2M entries per phase 1.20 -> 1.30 ms; four times: 2.71,
-        // 1.38 and 1.25 ms.
-        const u64 width = total <= static_cast<long long>(kThinShare) * gridDim.x ? 2 * delta : delta;
+        // 1.38 and 1.25 ms. Not so the first phase of a graph without
+        // records, where a root may reach most of a graph of small diameter
+        // (tree from scratch of 2M random vertices of degree 10: 10.2M
+        // entries in 2.64 ms, with the single width 4.6M in 1.36).
+        const bool thin = total <= static_cast<long long>(kThinShare) * gridDim.x && (phase > 0 || Kind != kCsrOnly);
+        const u64 width = thin ? 2 * delta : delta;
         const u64 lo = least > thr ? least : thr;
         thr = lo > kInfWord - width ? kInfWord - 1 : lo + width;
       }
@@ -2111,7 +2144,8 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
         }
       }
       if (blockIdx.x == 0 && static_cast<int>(lane) < P.aqShards) {
-        P.aqCtr[(phase + 1) % 3 * P.aqShards + lane].claimed = 0;
+        AsyncShard &A = P.aqCtr[(phase + 1) % 3 * P.aqShards + lane];
+        A.claimed = A.reserved = 0;
       }
       if (act && mode == kSplit) {
         if (blockIdx.x == 0) {
@@ -2671,7 +2705,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
   // share of the first phase (every mode passes a grid barrier before its
   // near-far loop)
   if ((P.flags & kFlagAsync) != 0 && P.aqCtr != nullptr) {
-    for (long long i = tid; i < P.aqShards; i += T) P.aqCtr[i].claimed = 0;
+    for (long long i = tid; i < P.aqShards; i += T) P.aqCtr[i].claimed = P.aqCtr[i].reserved = 0;
     if (tid == 0) c->asyncPending[0] = gridDim.x;
   }
   if constexpr (Mode == kModeUpdate) {

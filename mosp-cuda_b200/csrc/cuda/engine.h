@@ -142,10 +142,12 @@ enum : int {
 enum : unsigned char { kRecChanged = 1, kRecScan = 2 };
 
 /// Positions of one shard of the asynchronous loop's spill queue: entries
-/// reserved by producers (high half) and claimed by consumers (low half), in
-/// one word, so that one load sees both and one compare-and-swap claims.
+/// claimed by consumers and reserved by producers, side by side, so that one
+/// load sees both. Words of their own, as a claim is a compare-and-swap: in one
+/// word for both it failed whenever a producer came between (tree from scratch
+/// of 2M random vertices of degree 10: 6.2 ms so, 2.6 with two words).
 struct alignas(128) AsyncShard {
-  u64 claimed;  // reserved << 32 | claimed
+  unsigned claimed, reserved;
   unsigned pad[30];
 };
 constexpr int kAsyncShards = 16;  // shards of the spill queue
