@@ -50,14 +50,10 @@ namespace {
 // Small device helpers
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ unsigned long long ldAcquire64(const unsigned long long *p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+__device__ __forceinline__ u64 ldRelaxed64(const u64 *p) {
+  u64 v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
-}
-
-__device__ __forceinline__ void stRelease64(unsigned long long *p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 /// Two adjacent words, each read on its own, past L1.
@@ -883,11 +879,25 @@ constexpr unsigned kRingMask = kRing - 1;
 // a push finds the ring at most this full, plus 128 entries of each of the
 // other warps that passed the check at the same time, plus a claim
 constexpr unsigned kRingSpill = kRing / 4;
-constexpr unsigned kDonate = 512;    // ring entries above which a CTA feeds dry ones,
-constexpr unsigned kDonateRows = 64;  // in graphs without row records
+// Ring entries above which a CTA feeds dry ones: kDonate in updates with row
+// records, else kDonateLeast. Tree from scratch of random graphs, 500,000
+// vertices of degree 6, 300,000 of 18, 100,000 of 66, us: 455, 627, 1103 with
+// 512; 419, 522, 819 with 128; 441, 502, 638 with 64. Combined graph of 2M road
+// vertices 650 with 512, 601 with 64. But their update with long-range changes
+// is 3 % slower with 128 than with 512.
+constexpr unsigned kDonate = 512;
+constexpr unsigned kDonateLeast = 64;
 constexpr unsigned kSliceFirst = 1024;  // ring entries above which the share waits
-constexpr int kClaim = 1024;         // entries claimed from the spill queue at a time
-constexpr int kFetch = 256;          // of these read at a time
+// entries claimed from the spill queue at a time (256: tree from scratch of 2M
+// random vertices of degree 10 1.36 ms, 1,024 1.18), and read at a time
+constexpr int kClaim = 1024;
+constexpr int kFetch = 256;
+// A claim of so many entries says that the phase is wide. In a graph without
+// records the CTA's warps then take all they can carry and give each entry a
+// lane, which keeps the order breadth-first (combined graph of 2M random
+// vertices, 2.7 edges each: loop 661 -> 532 us; with records it makes road
+// networks slower, update of 2M vertices 1135 -> 1174).
+constexpr unsigned kBacklog = 64;
 constexpr int kOctBatch = 4;         // entries of a batch that is expanded by octets of lanes
 constexpr int kOctDeg = 32;          // longest row of such a batch
 constexpr int kQuadBatch = 8;        // the same with row records (four lanes each)
@@ -961,6 +971,7 @@ struct AsyncCta {
   int dry;
   int lock;
   int over;          // the phase is over
+  int full;          // the last claim found a backlog (kBacklog)
   int abort;         // the launch stops
   long long base;    // first far-pile index of the share
   // statistics: rounds, those of a phase from the CTA's first claim of spilled
@@ -1068,9 +1079,14 @@ __device__ __forceinline__ int takeIdle() {
 /// Sends up to `count` idle warps to the ring (lane 0).
 __device__ __noinline__ void wakeIdle(int count) {
   AsyncCta &C = asyncCta();
-  while (count-- > 0) {
-    const int w = takeIdle();
-    if (w < 0) return;
+  const unsigned idle = ldShared(&C.idle);
+  unsigned rest = idle;
+  for (; count > 0; --count) rest &= rest - 1u;
+  unsigned wake = idle ^ rest;
+  // (one that is no longer idle has been sent elsewhere and looks here next)
+  if (wake != 0) wake &= atomicAnd(&C.idle, ~wake);
+  for (; wake != 0; wake &= wake - 1u) {
+    const int w = __ffs(wake) - 1;
     C.mail[w] = 0;
     barArrive(&C.bar[w]);
   }
@@ -1181,8 +1197,8 @@ __device__ __noinline__ unsigned spillReserve(const EngineParams &P, int count, 
 /// it.
 __device__ __forceinline__ void spillWrite(const EngineParams &P, int shard, unsigned idx, u64 entry) {
   if (idx < P.aqShardCap) {
-    // release: an entry without a usable tag needs its word before it
-    stRelease64(P.aqSlots + static_cast<long long>(shard) * P.aqShardCap + idx, entry);
+    if (static_cast<unsigned>(entry >> 32) == kTagSat) __threadfence();  // the word before the entry
+    stRelaxed64(P.aqSlots + static_cast<long long>(shard) * P.aqShardCap + idx, entry);
     return;
   }
   const int k = static_cast<int>(entry & 31u);
@@ -1385,6 +1401,7 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
         atomicCAS(&shards[s].claimed, head, head + n) == head) {
       __threadfence();  // acquire: the producers' counts and slots
       C.owed += n;
+      C.full = n >= kBacklog;
       C.taken += n;
       if (C.fed == 0) {
         C.fed = 1;
@@ -1408,14 +1425,14 @@ __device__ __noinline__ void asyncFetch(const EngineParams &P, unsigned phase) {
 #pragma unroll
     for (int i = 0; i < kFetch / 32; ++i) {
       const unsigned j = j0 + static_cast<unsigned>(i * 32 + lane);
-      e[i] = j < n ? ldAcquire64(slots + j) : 0;
+      e[i] = j < n ? ldRelaxed64(slots + j) : 0;
     }
 #pragma unroll
     for (int i = 0; i < kFetch / 32; ++i) {
       const unsigned j = j0 + static_cast<unsigned>(i * 32 + lane);
       if (j >= n) continue;
       // the producer reserved the slot and is about to write it
-      for (unsigned spin = 0; e[i] == kEmptySlot; e[i] = ldAcquire64(slots + j)) {
+      for (unsigned spin = 0; e[i] == kEmptySlot; e[i] = ldRelaxed64(slots + j)) {
         if (++spin > (kSpinLimit >> 4) || ((spin & 1023u) == 0 && ldShared(&C.abort) != 0)) {
           asyncAbort(P);
           break;
@@ -1824,10 +1841,12 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
           break;
         }
         if (held == 0) break;
-        const unsigned n = held >= 128 ? 32u : (held + 3u) >> 2;
+        const bool full = !Rec && ldShared(&C.full) != 0;
+        const unsigned n = held >= 128 || (full && held >= 32) ? 32u : full ? held : (held + 3u) >> 2;
         if (atomicCAS(&C.head, h, h + n) != h) continue;
+        if (full) what = 1u << 17;
         at = h;
-        what = (1u << 8) | n;
+        what |= (1u << 8) | n;
         if (held > C.donateAt) what |= 1u << 16;
         break;
       }
@@ -1896,14 +1915,14 @@ __device__ __forceinline__ bool asyncConsume(const EngineParams &P, const int *o
     // other CTAs have run dry (read with the entries' loads)
     int hungry = 0;
     if (lane == 0) {
-      if ((what >> 16) != 0) hungry = ldVolatile(&c->asyncHungry[phase % 3]);
+      if (((what >> 16) & 1u) != 0) hungry = ldVolatile(&c->asyncHungry[phase % 3]);
       atomicAdd(&C.rounds, 1u);
       atomicAdd(&C.items, n);
     }
     owed += n;
     // few entries: a group of lanes each, expanded hop after hop
     constexpr unsigned kGroup = Rec ? 4 : 8;
-    const bool thin = n <= 32 / kGroup;
+    const bool thin = n <= 32 / kGroup && (what >> 17) == 0;
     const unsigned mine = thin ? lane / kGroup : lane;
     const bool lead = !thin || lane % kGroup == 0;
     const bool have = mine < n;
@@ -2060,7 +2079,7 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
     C.fed = 0;
     C.rounds = C.fedRounds = C.items = C.taken = 0;
     C.K = K;
-    C.donateAt = Kind == kCsrOnly ? kDonateRows : kDonate;
+    C.donateAt = Kind == kThinRecords ? kDonate : kDonateLeast;
     C.deadline = sync.deadline;
   }
   for (int i = threadIdx.x; i < kRing; i += blockDim.x) asyncRing()[i] = kEmptySlot;
@@ -2130,6 +2149,7 @@ __device__ __noinline__ bool asyncNearFar(const EngineParams &P, const int *outR
         C.owed = 1;
         C.dry = 0;
         C.over = 0;
+        C.full = 0;
         if (C.fed != 0) C.fedRounds += C.rounds - C.fedFrom;
         C.fed = 0;
         C.phase = phase;
