@@ -391,8 +391,8 @@ applyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedS
     const int occ = __ldcg(S.occ + s), cD = __ldcg(S.cD + s);
     if (occ <= cD && __ldcg(S.cI + s) > 0) {
       const int r = __ldcg(S.rowSlot + static_cast<int>(key >> 32)) - 1;
-      const int i = __ldcg(S.firstIns + s), bits = __ldcg(S.markOf + r);
-      S.app[__ldcg(S.segApp + r) + atomicAdd(S.curApp + r, 1)] = i;
+      const int i = __ldcg(S.firstIns + s), segment = __ldcg(S.segApp + r), bits = __ldcg(S.markOf + r);
+      S.app[segment + atomicAdd(S.curApp + r, 1)] = i;
       if (bits >= 0) atomicOr(S.marks + static_cast<long long>(bits) * S.markWords + (i >> 5), 1u << (i & 31));
     }
   }
@@ -559,9 +559,9 @@ copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedSc
     const int i = __ldcg(S.app + a);
     const int u = __ldg(P.insFrom + i);
     const int r = __ldcg(S.rowSlot + u) - 1;
-    const int count = __ldcg(S.nApp + r);
+    const int count = __ldcg(S.nApp + r), segment = __ldcg(S.segApp + r), bits = __ldcg(S.markOf + r);
     int rank = 0;
-    if (const int bits = __ldcg(S.markOf + r); bits >= 0) {
+    if (bits >= 0) {
       const unsigned *marks = S.marks + static_cast<long long>(bits) * S.markWords;
       for (int x = 0; x < i >> 7; ++x) {
         const uint4 b = __ldg(reinterpret_cast<const uint4 *>(marks) + x);
@@ -570,7 +570,7 @@ copyFused(const __grid_constant__ ApplyParams P, const __grid_constant__ FusedSc
       for (int x = i >> 7 << 2; x < i >> 5; ++x) rank += __popc(__ldg(marks + x));
       rank += __popc(__ldg(marks + (i >> 5)) & ((1u << (i & 31)) - 1u));
     } else {
-      const int *list = S.app + __ldcg(S.segApp + r);
+      const int *list = S.app + segment;
       for (int x = 0; x < count; ++x) rank += __ldcg(list + x) < i;
     }
     const int to = __ldcg(P.newRow + u + 1) - count + rank;
