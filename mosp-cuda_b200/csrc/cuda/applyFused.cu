@@ -33,7 +33,7 @@
 // the rows of 32 edges at a time instead, 1.4).
 //
 // Measured on a B200, sorted form and this one: 50,000 changes on a road
-// network of 5.56M edges, K = 3 (178 MB read and written): 578 -> 160 us;
+// network of 5.56M edges, K = 3 (178 MB read and written): 578 -> 145 us;
 // 24 changes on 4,200 edges: 307 -> 78 us; 20,000 on an R-MAT graph of 3.9M
 // edges, K = 4: 2112 -> 171 us; 60,000 on one of 65M, K = 5: 12.8 -> 1.2 ms.
 #include <cuda_runtime.h>

@@ -851,10 +851,12 @@ __device__ bool nearFarLoop(const EngineParams &P, const int *outRow,
 //
 // Measured on a B200 against one grid-wide sharded queue with a claim, a slot
 // and two counters per hop: a hop of a bare chain 0.59 us; tree from scratch
-// of a 497,700-vertex road network 10.05 -> 2.32 ms, update of a million
-// vertices with local detours (K = 3) 28.7 -> 7.8 ms, combined graph of
-// 249,500 vertices (K = 6) 5.26 -> 1.27 ms, update of 2M vertices with
-// long-range insertions (wide phases) 2.49 -> 2.30 ms.
+// of a 497,700-vertex road network 10.05 -> 2.33 ms, update of a million
+// vertices with local detours (K = 3) 28.7 -> 7.6 ms, combined graph of
+// 249,500 vertices (K = 6) 5.26 -> 1.25 ms, update of 2M vertices with
+// long-range insertions (wide phases) 2.49 -> 2.17 ms; tree from scratch of 2M
+// random vertices of degree 10 1.15 -> 1.05 ms, but the combined launch of such
+// a graph (K = 3) 0.51 -> 0.78 ms.
 //
 // A vertex enters the far pile when an atomicMin takes it from infinity (or,
 // in an update, from its tree distance) to a distance past the threshold;
