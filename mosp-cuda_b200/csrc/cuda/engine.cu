@@ -212,6 +212,15 @@ struct StageEntry {
   u64 d;
 };
 
+/// Whether a row of deg edges goes to the whole CTA. Rows above the hub
+/// threshold find the queue's second half free: a hub row left to one warp
+/// costs more than many shorter ones (tree from scratch of an R-MAT graph of 1M
+/// vertices 6.2 ms with any row in any place).
+__device__ __forceinline__ bool takesCta(const EngineParams &P, const StageHeader &H, int deg) {
+  if (deg <= ctaRowOf(P)) return false;
+  return deg > heavyDegOf(P) || *const_cast<const volatile int *>(&H.heavyCount) < kHeavyCap / 2;
+}
+
 constexpr size_t kStageHeaderBytes = (sizeof(StageHeader) + 15) / 16 * 16;
 constexpr size_t kStageBytes = kStageHeaderBytes + kStage * sizeof(StageEntry);
 
@@ -447,7 +456,7 @@ __device__ __forceinline__ void expandWarp(const EngineParams &P, const LoopShar
   if (__ballot_sync(kFull, deg > 0) == 0) return;
   // heavy rows go to the CTA's queue (expanded by the whole CTA after this
   // round of items) when the launch has any
-  if (heavyOn && deg > ctaRowOf(P)) {
+  if (heavyOn && takesCta(P, H, deg)) {
     const int slot = atomicAdd(&H.heavyCount, 1);
     if (slot < kHeavyCap) {
       H.heavyK[slot] = k;
@@ -2993,7 +3002,7 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
           end = __ldg(P.inRow + v + 1);
         }
         // heavy in-rows are reduced by the whole CTA after the tile
-        if (heavyOn && end - beg > ctaRowOf(P)) {
+        if (heavyOn && takesCta(P, H, end - beg)) {
           const int slot = atomicAdd(&H.heavyCount, 1);
           if (slot < kHeavyCap) {
             H.heavyK[slot] = k;
