@@ -2978,13 +2978,13 @@ __global__ void __launch_bounds__(kThreads, 1) sospEngine(const __grid_constant_
       // 22, K = 5, 270,959: 121, 120, 115; road networks: 64 of 20,020
       // vertices, 1.3M candidates: 61, 50, 83; 640,000 vertices, 413,402: 46,
       // 43, 54; 93,300 vertices, 83,544: 9.9, 9.4, 11.1.
-      const unsigned group = heavyOn ? 1 : 32;
+      const unsigned groupBits = heavyOn ? 0 : 5;
       const long long tileStride = static_cast<long long>(gridDim.x) * blockDim.x;
       for (long long tile = static_cast<long long>(blockIdx.x) * blockDim.x;
            tile - static_cast<long long>(blockIdx.x) * blockDim.x < total; tile += tileStride) {
         const long long j = tile - static_cast<long long>(blockIdx.x) * blockDim.x +
-                            (static_cast<long long>(threadIdx.x / group) * gridDim.x + blockIdx.x) * group +
-                            threadIdx.x % group;
+                            ((static_cast<long long>(threadIdx.x >> groupBits) * gridDim.x + blockIdx.x) << groupBits) +
+                            (threadIdx.x & ((1u << groupBits) - 1u));
         const bool valid = j < total;
         int k = 0;
         if (valid) {
